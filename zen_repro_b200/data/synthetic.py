@@ -29,7 +29,8 @@ class ZipfTokenStream:
         self._pool = [self._make(i) for i in range(pool)] if pool else None
 
     def _make(self, step: int) -> dict:
-        g = torch.Generator().manual_seed((self.seed * 1_000_003 + self.dp_rank) * 1_000_003 + step)
+        # modulo 2**64, all that a generator takes: the products above exceed it for seeds of some 18 million and more
+        g = torch.Generator().manual_seed(((self.seed * 1_000_003 + self.dp_rank) * 1_000_003 + step) % (1 << 64))
         u = torch.rand(self.batch * self.seq, generator=g, dtype=torch.float64)
         ids = torch.searchsorted(self.cdf, u).clamp_(max=self.vocab - 1).view(self.batch, self.seq)
         if self.pin:
