@@ -1,6 +1,8 @@
 """Edges of the fused passes around the vocabulary and the token positions: soft-capped cross-entropy (both CTA sizes), label shift and
 count, position gradients, column sums whose vectors do not divide the CTA, rotation split into head groups, gradients that the
 optimizer clears."""
+import math
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -25,6 +27,45 @@ def test_cross_entropy(rows, vocab, cap):
     loss, dl = E.cross_entropy(x.clone()[:, :vocab], labels, grad_scale=1.0, grad_scale_dev=inv, softcap=cap)
     torch.testing.assert_close(loss, want.detach(), atol=2e-2, rtol=2e-3)
     torch.testing.assert_close(dl.float(), g, atol=2e-3, rtol=2e-2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("masked", ["lowest", "-inf"])
+@pytest.mark.parametrize("rows,vocab", [(3, 1000), (2, 20_003), (2, 256_001)])
+def test_cross_entropy_of_masked_logits(rows, vocab, masked, dtype):
+    """Whole vectors, and all that one thread sees first, of the type's lowest value or of -inf."""
+    from zen_repro_b200.ops import elementwise as E
+
+    torch.manual_seed(vocab)
+    x = (torch.randn(rows, (vocab + 7) // 8 * 8, device="cuda") * 3).to(dtype)
+    x[:, : vocab - 70] = torch.finfo(dtype).min if masked == "lowest" else float("-inf")
+    x[0, 5] = 1.0
+    labels = torch.full((rows,), vocab - 3, device="cuda")
+    ref = x[:, :vocab].double().requires_grad_(True)
+    want = F.cross_entropy(ref, labels, reduction="none")
+    (g,) = torch.autograd.grad(want.sum(), ref)
+    loss, dl = E.cross_entropy(x.clone()[:, :vocab], labels, grad_scale=1.0)
+    torch.testing.assert_close(loss.double(), want.detach(), atol=1e-5, rtol=1e-6)
+    torch.testing.assert_close(dl.double(), g, atol=2e-6, rtol=1e-5 if dtype == torch.float32 else 2.0**-8)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1000.0])
+def test_cross_entropy_of_large_fp32_logits(scale):
+    """The loss to the rounding of a logit, the gradient to that rounding times its value: nothing is lost to log2(e)."""
+    from zen_repro_b200.ops import elementwise as E
+
+    torch.manual_seed(1)
+    x = torch.randn(64, 4096, device="cuda") + scale
+    labels = torch.randint(0, 4096, (64,), device="cuda")
+    ref = x.double().requires_grad_(True)
+    want = F.cross_entropy(ref, labels, reduction="none")
+    (g,) = torch.autograd.grad(want.sum(), ref)
+    loss, dl = E.cross_entropy(x.clone(), labels, grad_scale=1.0)
+    # the log-sum-exp (at most scale + 10) is rounded once; a gradient's exponent, 14 at most, in its difference, its product and
+    # log2(e), and the exponential is off by 2 units
+    lse = 2.0 ** (math.floor(math.log2(scale + 10.0)) - 24)
+    assert (loss - want).abs().max() <= lse + 2.0**-20
+    assert ((dl.double() - g).abs() <= (lse + 2.0**-24 * (2.5 * 14 + 8)) * torch.softmax(ref.detach(), -1) + 2.0**-24 * g.abs()).all()
 
 
 @pytest.mark.parametrize("bsz,seq,shift", [(1, 1, 1), (3, 77, 1), (2, 1500, 0)])

@@ -1036,15 +1036,17 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
           for (int i = 0; i < 8; ++i) mx = fmaxf(mx, x[u].at(i));
         if (CAP) mx = xent_cap<CAP>(mx, cap, k2, nullptr);  // monotonic
         const float nm = fmaxf(m, mx);
-        const float off = -nm * L2E;
+        // exponents are made of differences: with x * L2E - nm * L2E in one FMA a maximum of the type's lowest value (masked
+        // logits) overflows, and large logits lose the bits that cancel.  Nothing but -inf so far: exp(-inf - 0) = 0.
+        const float ref = nm == -INFINITY ? 0.f : nm;
         float add[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < XENT_U; ++u)
           if (v0 + u * XENT_THREADS < nv) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) add[i & 3] += ex2_fast(fmaf(xent_cap<CAP>(x[u].at(i), cap, k2, nullptr), L2E, off));
+            for (int i = 0; i < 8; ++i) add[i & 3] += ex2_fast((xent_cap<CAP>(x[u].at(i), cap, k2, nullptr) - ref) * L2E);
           }
-        s = s * ex2_fast(fmaf(m, L2E, off)) + ((add[0] + add[1]) + (add[2] + add[3]));
+        s = s * ex2_fast((m - ref) * L2E) + ((add[0] + add[1]) + (add[2] + add[3]));
         m = nm;
 #pragma unroll
         for (int u = 0; u < XENT_U; ++u) x[u] = y[u];
@@ -1052,8 +1054,8 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
     }
     for (int c = nv * 8 + threadIdx.x; c < vocab; c += XENT_THREADS) {
       const float x = xent_cap<CAP>(ZenVal<T>::to_f(lp[c]), cap, k2, nullptr);
-      const float nm = fmaxf(m, x);
-      s = s * __expf(m - nm) + __expf(x - nm);
+      const float nm = fmaxf(m, x), ref = nm == -INFINITY ? 0.f : nm;
+      s = s * __expf(m - ref) + __expf(x - ref);
       m = nm;
     }
     const float gm = block_max(m, sh);
@@ -1062,7 +1064,7 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
     const float lse = gm + logf(gs);
     if (threadIdx.x == 0) loss[row] = valid ? lse - at_label : 0.f;
     if (dp) {
-      const float sc = valid ? gscale : 0.f, off = -lse * L2E;
+      const float sc = valid ? gscale : 0.f;
       if ((int)threadIdx.x < nv) {
         Raw8v<T> x[XENT_U], y[XENT_U];
         fetch(x, threadIdx.x);
@@ -1075,7 +1077,7 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 float t = 0.f;
-                const float p = ex2_fast(fmaf(xent_cap<CAP>(x[u].at(i), cap, k2, &t), L2E, off));
+                const float p = ex2_fast((xent_cap<CAP>(x[u].at(i), cap, k2, &t) - lse) * L2E);
                 o[i] = CAP ? p * sc * (1.f - t * t) : p * sc;
               }
               Vec8<T>::store(dp + (size_t)(v0 + u * XENT_THREADS) * 8, o);
@@ -1091,7 +1093,7 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
       }
       __syncthreads();
       if (valid && threadIdx.x == 0) {                  // the label's own entry: softmax - 1
-        const float g = (ex2_fast(fmaf(at_label, L2E, off)) - 1.f) * sc;
+        const float g = (ex2_fast((at_label - lse) * L2E) - 1.f) * sc;
         dp[label] = ZenVal<T>::from_f(CAP ? g * (1.f - t_label * t_label) : g);
       }
     }
