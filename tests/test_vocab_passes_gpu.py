@@ -30,6 +30,36 @@ def test_cross_entropy(rows, vocab, cap):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,vocab,cap", [(5, 1003, 30.0), (9, 256_001, 30.0), (64, 4096, 5.0)])
+def test_soft_capped_cross_entropy_near_the_cap(rows, vocab, cap, dtype):
+    """Against 64 bits, with logits well into the flat part of the cap, where the gradient's factor 1 - tanh^2 cancels."""
+    from zen_repro_b200.ops import elementwise as E
+
+    torch.manual_seed(vocab)
+    ld = (vocab + 7) // 8 * 8
+    x = (torch.randn(rows, ld, device="cuda") * 2 * cap).to(dtype)
+    labels = torch.randint(0, vocab, (rows,), device="cuda")
+    ref = x[:, :vocab].double().requires_grad_(True)
+    z = cap * torch.tanh(ref / cap)
+    want = F.cross_entropy(z, labels, reduction="none")
+    (g,) = torch.autograd.grad(want.sum(), ref)
+    capped = E.softcap_logits(x[:, :vocab], cap)
+    loss, dl = E.cross_entropy(x.clone()[:, :vocab], labels, grad_scale=1.0, softcap=cap)
+    # fp32: a tanh within 2 units and the roundings of cap * t * log2(e) make some 8 units of the cap in an exponent
+    unit = 2.0**-24
+    assert (loss - want).abs().max() <= 16 * cap * unit + 8 * unit * want.abs().max()
+    assert (loss - F.cross_entropy(capped.double(), labels, reduction="none")).abs().max() <= 16 * cap * unit + 8 * unit * want.abs().max()
+    # p (1 - t^2), |p - 1| at the label: 1 - t^2 is off by 4 units of 1, p by the exponent's; then the rounding to the result's type
+    p = torch.softmax(z.detach(), -1)
+    p[torch.arange(rows), labels] -= 1.0
+    bound = p.abs() * 8 * unit + g.abs() * 32 * cap * unit + 2.0**-149
+    if dtype == torch.bfloat16:
+        bound = bound * (1 + 2.0**-8) + g.abs() * 2.0**-8
+    p_abs = 16 * cap * unit * torch.softmax(z.detach(), -1) * (1 - (z.detach() / cap) ** 2)     # p near 1 at the label
+    assert ((dl.double() - g).abs() <= bound + p_abs + 1e-37).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("masked", ["lowest", "-inf"])
 @pytest.mark.parametrize("rows,vocab", [(3, 1000), (2, 20_003), (2, 256_001)])
 def test_cross_entropy_of_masked_logits(rows, vocab, masked, dtype):
