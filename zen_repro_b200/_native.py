@@ -21,29 +21,16 @@ class NativeUnavailable(RuntimeError):
     pass
 
 
-# kernels launched by one call of each entry point (entries not listed launch one, helpers launch none)
-KERNELS_PER_CALL = {
-    "zen_gather_push": 1, "zen_densify": 1, "zen_sparse_allreduce": 4, "zen_sparse_allreduce_local": 4, "zen_sample_exchange": 2, "zen_sample_xchg_size": 0, "zen_mc_ar_ctx_size": 0, "zen_norm_bwd": 2, "zen_colsum": 2, "zen_embedding_bwd_rows": 4, "zen_embedding_flag_words": 0, "zen_block_fwd": 8, "zen_block_bwd": 16, "zen_block_size": 0, "zen_block_grads_size": 0, "zen_block_bytes": 0,
-    "zen_row_gather_push": 2, "zen_attn_bwd": 3, "zen_flash_bwd": 2, "zen_flash_error": 0, "zen_gemm_splitk_error": 0, "zen_attn_error": 0, "zen_attn_hsplit": 0, "zen_attn_bwd64_variant": 0, "zen_gemm2_force_bn": 0, "zen_gemm2_tail_split": 0, "zen_gemm_desc_size": 0, "zen_gemm_group_max": 0, "zen_act_bwd_colsum": 1, "zen_act_colsum_parts": 0, "zen_colsum_reduce": 1, "zen_colsum_partial": 1, "zen_colreduce_multi": 1, "zen_colreduce_job_size": 0, "zen_colreduce_max_jobs": 0, "zen_norm_bwd_parts_used": 0, "zen_norm_bwd_ex": 2, "zen_select_kth": 7, "zen_gemm2_error": 0, "zen_gemm_ar_ctx_size": 0, "zen_sparse_ctx_size": 0, "zen_row_ctx_size": 0, "zen_adam_tensor_size": 0,
-    "zen_norm_bwd_parts": 0, "zen_colsum_parts": 0, "zen_gemm_error": 0, "zen_sym_alloc": 0, "zen_sym_free": 0,
-    "zen_ipc_get_handle": 0, "zen_ipc_open": 0, "zen_ipc_close": 0, "zen_enable_peer": 0, "zen_ipc_handle_size": 0,
-}
-
-
 class _Library:
     """The library's functions as attributes, callable with ints (pointers included), floats, None and ctypes structures
-    (csrc/fastcall.c); kernel launches are counted on the way (read by the benchmark)."""
+    (csrc/fastcall.c)."""
 
     def __init__(self, path, fastcall):
         self._cdll, self._fast = ctypes.CDLL(str(path)), fastcall
 
-    @property
-    def launches(self) -> int:
-        return self._fast.launches()
-
     def __getattr__(self, name):
         addr = ctypes.cast(getattr(self._cdll, name), ctypes.c_void_p).value
-        fn = self._fast.function(addr, KERNELS_PER_CALL.get(name, 1))
+        fn = self._fast.function(addr)
         self.__dict__[name] = fn
         return fn
 
@@ -77,8 +64,12 @@ def lib() -> "_Library":
 
 
 def launch_count() -> int:
-    """Kernels of this library launched so far in this process."""
-    return _LIB.launches if _LIB is not None else 0
+    """Kernels of this library launched so far in this process, as the library counts them where it launches them."""
+    if _LIB is None:
+        return 0
+    n = ctypes.c_int64()
+    _LIB.zen_launch_count(ctypes.byref(n))
+    return n.value
 
 
 def available() -> bool:

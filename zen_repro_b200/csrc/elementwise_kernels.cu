@@ -1678,8 +1678,8 @@ int zen_colsum_noalloc(const void* a, void* out, int rows, int cols, int accumul
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   DISPATCH_T(dtype, {
-    colsum_partial_kernel<T><<<parts, 256, 0, st>>>((const T*)a, part, rows, cols, RPC);
-    colreduce_kernel<T><<<(cols + 31) / 32, 1024, 0, st>>>(part, (T*)out, parts, cols, accumulate);
+    zen_pdl::plain(colsum_partial_kernel<T>, parts, 256, 0, st, (const T*)a, part, rows, cols, RPC);
+    zen_pdl::plain(colreduce_kernel<T>, (cols + 31) / 32, 1024, 0, st, part, (T*)out, parts, cols, accumulate, (const float*)nullptr, (T*)nullptr);
   });
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return noalloc_fail((int)e, cudaGetErrorString(e));

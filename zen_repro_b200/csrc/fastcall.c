@@ -17,13 +17,10 @@
 #define MAX_INTS 28
 #define MAX_FLOATS 8
 
-static long long g_launches = 0;          /* kernels launched through these functions (read by benchmarks) */
-
 typedef struct {
   PyObject_HEAD
   vectorcallfunc vectorcall;
   void* fn;
-  long long kernels;
 } FastFn;
 
 typedef int (*any_fn)(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
@@ -82,7 +79,6 @@ static PyObject* fast_call(PyObject* self, PyObject* const* args, size_t nargsf,
     else if (a == Py_None) iv[ni++] = 0;
     else if (convert_other(a, iv, &ni, fv, &nf) != 0) return NULL;
   }
-  g_launches += f->kernels;
   Py_BEGIN_ALLOW_THREADS
   rc = ((any_fn)f->fn)(iv[0], iv[1], iv[2], iv[3], iv[4], iv[5], iv[6], iv[7], iv[8], iv[9], iv[10], iv[11], iv[12], iv[13], iv[14],
                        iv[15], iv[16], iv[17], iv[18], iv[19], iv[20], iv[21], iv[22], iv[23], iv[24], iv[25], iv[26], iv[27], fv[0],
@@ -98,23 +94,16 @@ static PyTypeObject* fast_type = NULL;
 
 static PyObject* make(PyObject* m, PyObject* args) {
   unsigned long long addr;
-  long long kernels;
   (void)m;
-  if (!PyArg_ParseTuple(args, "KL", &addr, &kernels)) return NULL;
+  if (!PyArg_ParseTuple(args, "K", &addr)) return NULL;
   FastFn* f = PyObject_New(FastFn, fast_type);
   if (!f) return NULL;
   f->vectorcall = fast_call;
   f->fn = (void*)(uintptr_t)addr;
-  f->kernels = kernels;
   return (PyObject*)f;
 }
-static PyObject* launches(PyObject* m, PyObject* a) {
-  (void)m; (void)a;
-  return PyLong_FromLongLong(g_launches);
-}
 
-static PyMethodDef methods[] = {{"function", make, METH_VARARGS, "function(address, kernels per call)"},
-                                {"launches", launches, METH_NOARGS, "kernels launched so far"}, {NULL, NULL, 0, NULL}};
+static PyMethodDef methods[] = {{"function", make, METH_VARARGS, "function(address)"}, {NULL, NULL, 0, NULL}};
 static struct PyModuleDef mod = {PyModuleDef_HEAD_INIT, "zen_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};
 
 PyMODINIT_FUNC PyInit_zen_fastcall(void) {

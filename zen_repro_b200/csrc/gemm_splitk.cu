@@ -222,7 +222,7 @@ int launch_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const SplitKPara
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, A_MN, B_MN>, ta, tb, p, S);
+  return zen_pdl::counted(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, A_MN, B_MN>, ta, tb, p, S));
 }
 
 }  // namespace

@@ -750,7 +750,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, 
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < sm_count_g() ? tiles : sm_count_g();
   if (p.npeers == 0 && p.coll_mode == 0) return zen_pdl::launch(gemm_bf16_kernel<BN, A_MN, B_MN>, grid, NUM_THREADS, C::SMEM_BYTES, st, ta, tb, tg, p);
-  gemm_bf16_kernel<BN, A_MN, B_MN><<<grid, NUM_THREADS, C::SMEM_BYTES, st>>>(ta, tb, tg, p);
+  zen_pdl::plain(gemm_bf16_kernel<BN, A_MN, B_MN>, grid, NUM_THREADS, C::SMEM_BYTES, st, ta, tb, tg, p);
   return (int)cudaGetLastError();
 }
 

@@ -16,7 +16,17 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 namespace zen_pdl {
+
+// Kernels launched by this library in this process (zen_launch_count; a captured launch counts when it is captured).  Every launch
+// of the library goes through this file, which is what makes the count one.
+inline std::atomic<long long> g_launched{0};
+inline int counted(cudaError_t e) {
+  if (e == cudaSuccess) g_launched.fetch_add(1, std::memory_order_relaxed);
+  return (int)e;
+}
 
 __device__ __forceinline__ void trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -39,11 +49,15 @@ inline int launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, si
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = early ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return counted(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 template <typename K, typename... A>
 inline int launch(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   return launch_if(true, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
+}
+template <typename K, typename... A>
+inline int plain(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_if(false, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 // Kernels that stream memory through a grid of several CTAs per SM start early only when they are small (at most two CTAs per
 // SM): waiting CTAs of a large grid settle unevenly over the SMs beside their predecessor's, which cost up to a third of a

@@ -11,6 +11,7 @@
 // The bucket must live in a multicast-mapped symmetric region (torch symmetric memory): `mc` is the
 // multicast alias of the region's base, `flags[r]` the flag block inside rank r's copy.
 // Reference counterpart: the dense bucket all-reduce of torch DDP (train.py:184-185, NCCL).
+#include "launch.cuh"
 #include "zen_common.cuh"
 
 struct ZenMcArCtx {
@@ -127,8 +128,8 @@ int zen_multimem_allreduce(const ZenMcArCtx* c, uint64_t byte_off, uint64_t nbyt
   if (nbytes == 0) return 0;
   if (ctas <= 0) ctas = 8;
   if (ctas > 148) ctas = 148;
-  if (dtype == ZEN_DTYPE_BF16) zen_multimem_allreduce_kernel<true><<<ctas, MCAR_THREADS, 0, (cudaStream_t)stream>>>(*c, byte_off, nbytes / 16, scale);
-  else zen_multimem_allreduce_kernel<false><<<ctas, MCAR_THREADS, 0, (cudaStream_t)stream>>>(*c, byte_off, nbytes / 16, scale);
+  if (dtype == ZEN_DTYPE_BF16) zen_pdl::plain(zen_multimem_allreduce_kernel<true>, ctas, MCAR_THREADS, 0, (cudaStream_t)stream, *c, byte_off, nbytes / 16, scale);
+  else zen_pdl::plain(zen_multimem_allreduce_kernel<false>, ctas, MCAR_THREADS, 0, (cudaStream_t)stream, *c, byte_off, nbytes / 16, scale);
   return (int)cudaGetLastError();
 }
 

@@ -5,7 +5,15 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "launch.cuh"
+
 extern "C" {
+
+// Kernels launched by this library in this process so far.
+int zen_launch_count(int64_t* out) {
+  *out = zen_pdl::g_launched.load(std::memory_order_relaxed);
+  return 0;
+}
 
 // Allocate `bytes` of device memory directly from the driver pool (not from a caching allocator, so
 // that the IPC handle covers exactly this allocation) and zero it.

@@ -1183,7 +1183,7 @@ static bool small_call(const ZenSparseCtx& c, int n) { return c.numel * (uint64_
 template <int NB, typename K, typename... A>
 static void start(bool small, K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
   if constexpr (NB > 1) zen_pdl::launch_if(small, kernel, grid, dim3(threads), smem, st, args...);
-  else kernel<<<grid, threads, smem, st>>>(args...);
+  else zen_pdl::plain(kernel, grid, threads, smem, st, args...);
 }
 // CTAs of one rank when `total` of them are wanted for the launch
 static int share_of(int total, int n) { return total / n > 0 ? total / n : 1; }
@@ -1309,7 +1309,7 @@ int zen_sparse_ctx_size() { return (int)sizeof(ZenSparseCtx); }
 
 // Advance a device-resident call counter by one (first launch of a call whose kernels read `epoch_dev`).
 int zen_sparse_epoch_bump(uint32_t* epoch_dev, void* stream) {
-  zen_sparse_epoch_bump_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(epoch_dev);
+  zen_pdl::plain(zen_sparse_epoch_bump_kernel, 1, 1, 0, (cudaStream_t)stream, epoch_dev);
   return (int)cudaGetLastError();
 }
 
@@ -1401,7 +1401,7 @@ int zen_sparse_allreduce_local(const ZenSparseCtx* c, int n, void* const* io, co
 
 int zen_owner_map(int32_t* out, uint64_t n, const ZenPerm* perm, int mode, uint32_t table, int parts, void* stream) {
   ZenPerm p = *perm;
-  zen_owner_map_kernel<<<grid_for(n, 256 * 8, sm_count() * 8), 256, 0, (cudaStream_t)stream>>>(out, n, p, mode, table, parts);
+  zen_pdl::plain(zen_owner_map_kernel, grid_for(n, 256 * 8, sm_count() * 8), 256, 0, (cudaStream_t)stream, out, n, p, mode, table, parts);
   return (int)cudaGetLastError();
 }
 
@@ -1410,7 +1410,7 @@ int zen_sparse_balance(const void* in, uint64_t n, int dtype, int32_t* table, ui
                        void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = grid_for(n, 256 * 4, sm_count() * 8);
-  DISPATCH_DTYPE(dtype, zen_sparse_balance_kernel<T><<<grid, 256, 0, st>>>((const T*)in, n, table, table_size, serial,
+  DISPATCH_DTYPE(dtype, zen_pdl::plain(zen_sparse_balance_kernel<T>, grid, 256, 0, st, (const T*)in, n, table, table_size, serial,
                                                                            serial_per_part, cursors, parts, rehash,
                                                                            status));
   return (int)cudaGetLastError();
@@ -1486,7 +1486,7 @@ extern "C" {
 int zen_sample_abs(const void* x, uint64_t n, float* out, uint32_t nsamples, uint32_t seed, int dtype, void* stream) {
   if (n == 0 || nsamples == 0) return -1;
   const int grid = grid_for(nsamples, 256, sm_count() * 4);
-  DISPATCH_DTYPE(dtype, zen_sample_abs_kernel<T><<<grid, 256, 0, (cudaStream_t)stream>>>((const T*)x, n, out, nsamples, seed));
+  DISPATCH_DTYPE(dtype, zen_pdl::plain(zen_sample_abs_kernel<T>, grid, 256, 0, (cudaStream_t)stream, (const T*)x, n, out, nsamples, seed));
   return (int)cudaGetLastError();
 }
 
@@ -1495,11 +1495,11 @@ int zen_sample_abs(const void* x, uint64_t n, float* out, uint32_t nsamples, uin
 int zen_select_kth(const float* v, uint32_t n, uint32_t k, uint32_t* hist, uint32_t* state, float* out, void* stream) {
   if (n == 0 || k == 0 || k > n) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  zen_select_init_kernel<<<1, 1, 0, st>>>(state, k);
+  zen_pdl::plain(zen_select_init_kernel, 1, 1, 0, st, state, k);
   const int grid = grid_for(n, 256 * 8, sm_count() * 2);
   for (int pass = 0; pass < 3; ++pass) {
-    zen_select_hist_kernel<<<grid, 256, 0, st>>>(v, n, hist, state, pass);
-    zen_select_pick_kernel<<<1, 1024, 0, st>>>(hist, state, out, pass);
+    zen_pdl::plain(zen_select_hist_kernel, grid, 256, 0, st, v, n, hist, state, pass);
+    zen_pdl::plain(zen_select_pick_kernel, 1, 1024, 0, st, hist, state, out, pass);
   }
   return (int)cudaGetLastError();
 }
@@ -1569,8 +1569,8 @@ int zen_sample_xchg_size() { return (int)sizeof(ZenSampleXchg); }
 int zen_sample_exchange(const ZenSampleXchg* c, const float* mine, float* out, void* stream) {
   if (!c || c->nranks < 1 || c->nranks > ZEN_MAX_RANKS || c->ns == 0) return -1;
   const int grid = grid_for(c->ns, 256 * 8, 16);
-  zen_sample_exchange_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(*c, mine);
-  zen_sample_collect_kernel<<<grid_for((uint64_t)c->nranks * c->ns, 256 * 4, sm_count()), 256, 0, (cudaStream_t)stream>>>(*c, out);
+  zen_pdl::plain(zen_sample_exchange_kernel, grid, 256, 0, (cudaStream_t)stream, *c, mine);
+  zen_pdl::plain(zen_sample_collect_kernel, grid_for((uint64_t)c->nranks * c->ns, 256 * 4, sm_count()), 256, 0, (cudaStream_t)stream, *c, out);
   return (int)cudaGetLastError();
 }
 

@@ -7,6 +7,7 @@
 // into its dense gradient.  Traffic and work are O(touched rows * d); the dense [V, d] gradient is
 // never scanned.  The reference has no row mode: it top-k sparsifies whole DDP buckets
 // (train.py:167-183).
+#include "launch.cuh"
 #include "zen_common.cuh"
 
 struct ZenRowCtx {
@@ -300,7 +301,7 @@ extern "C" {
 
 // Advance the device-side call counter (first launch of every call when the counter lives on the device).
 int zen_row_epoch_bump(uint32_t* epoch_dev, void* stream) {
-  row_epoch_bump_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(epoch_dev);
+  zen_pdl::plain(row_epoch_bump_kernel, 1, 1, 0, (cudaStream_t)stream, epoch_dev);
   return (int)cudaGetLastError();
 }
 
@@ -309,29 +310,29 @@ int zen_row_ctx_size() { return (int)sizeof(ZenRowCtx); }
 int zen_row_push(const ZenRowCtx* c, const int32_t* rows, const int32_t* count, const void* vals, int max_rows,
                  int dtype, void* stream) {
   if (c->d % 8) return -2;
-  DISPATCH_R(dtype, row_push_kernel<T><<<sm_count_r() * 2, 256, 0, (cudaStream_t)stream>>>(*c, rows, count, (const T*)vals, max_rows));
+  DISPATCH_R(dtype, zen_pdl::plain(row_push_kernel<T>, sm_count_r() * 2, 256, 0, (cudaStream_t)stream, *c, rows, count, (const T*)vals, max_rows));
   return (int)cudaGetLastError();
 }
 
 int zen_row_reduce(const ZenRowCtx* c, int dtype, int deterministic, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (deterministic) {
-    for (int s = 0; s < c->nranks; ++s) { DISPATCH_R(dtype, row_reduce_kernel<T><<<sm_count_r() * 2, 256, 0, st>>>(*c, s, s + 1)); }
+    for (int s = 0; s < c->nranks; ++s) { DISPATCH_R(dtype, zen_pdl::plain(row_reduce_kernel<T>, sm_count_r() * 2, 256, 0, st, *c, s, s + 1)); }
   } else {
-    DISPATCH_R(dtype, row_reduce_kernel<T><<<sm_count_r() * 2, 256, 0, st>>>(*c, 0, c->nranks));
+    DISPATCH_R(dtype, zen_pdl::plain(row_reduce_kernel<T>, sm_count_r() * 2, 256, 0, st, *c, 0, c->nranks));
   }
   return (int)cudaGetLastError();
 }
 
 int zen_row_gather_push(const ZenRowCtx* c, int dtype, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  row_list_kernel<<<1, 1024, 0, st>>>(*c);
-  DISPATCH_R(dtype, row_gather_push_kernel<T><<<sm_count_r() * 2, 256, 0, st>>>(*c));
+  zen_pdl::plain(row_list_kernel, 1, 1024, 0, st, *c);
+  DISPATCH_R(dtype, zen_pdl::plain(row_gather_push_kernel<T>, sm_count_r() * 2, 256, 0, st, *c));
   return (int)cudaGetLastError();
 }
 
 int zen_row_apply(const ZenRowCtx* c, void* grad, float scale, int overwrite, int dtype, void* stream) {
-  DISPATCH_R(dtype, row_apply_kernel<T><<<sm_count_r() * 2, 256, 0, (cudaStream_t)stream>>>(*c, (T*)grad, scale, overwrite));
+  DISPATCH_R(dtype, zen_pdl::plain(row_apply_kernel<T>, sm_count_r() * 2, 256, 0, (cudaStream_t)stream, *c, (T*)grad, scale, overwrite));
   return (int)cudaGetLastError();
 }
 
