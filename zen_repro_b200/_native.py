@@ -47,16 +47,18 @@ def _load_fastcall(path):
 
 
 def lib() -> "_Library":
-    """The loaded native library; builds it first if the ``.so`` is missing and nvcc exists."""
+    """The loaded native library; built first where the ``.so`` is missing (needs nvcc) or the CPython extension beside it is
+    missing or of another interpreter (needs a C compiler)."""
     global _LIB
     if _LIB is not None:
         return _LIB
     with _LOCK:
         if _LIB is None:
             path = _build.lib_path()
-            if not path.exists() or not _build.fastcall_path().exists():
+            if not path.exists() or not _build.fastcall_current():
                 try:
-                    path = _build.build()
+                    path = _build.build() if not path.exists() else path
+                    _build.build_fastcall()
                 except Exception as e:  # pragma: no cover - depends on toolchain
                     raise NativeUnavailable(f"native library missing and build failed: {e}") from e
             _LIB = _Library(path, _load_fastcall(_build.fastcall_path()))

@@ -67,19 +67,33 @@ def _compile_one(src: Path, verbose: bool) -> tuple[Path, str]:
     return obj, log
 
 
-def _build_fastcall() -> Path:
+def _fastcall_want() -> str:
+    """What ``fastcall.stamp`` says beside an extension that belongs to this source and this interpreter."""
+    return hashlib.sha256((CSRC / "fastcall.c").read_bytes()).hexdigest() + sys.version
+
+
+def fastcall_current() -> bool:
+    """Whether the CPython extension is there and was built from this source for this interpreter: one that another Python
+    built can be opened all the same, and then runs with the wrong object layouts."""
+    stamp = LIBDIR / "fastcall.stamp"
+    return (LIBDIR / CALLNAME).exists() and stamp.exists() and stamp.read_text() == _fastcall_want()
+
+
+def build_fastcall() -> Path:
     """The small CPython extension through which Python calls the library's functions."""
     src, out, stamp = CSRC / "fastcall.c", LIBDIR / CALLNAME, LIBDIR / "fastcall.stamp"
-    want = hashlib.sha256(src.read_bytes()).hexdigest() + sys.version
-    if not out.exists() or not stamp.exists() or stamp.read_text() != want:
+    if not fastcall_current():
+        LIBDIR.mkdir(exist_ok=True)
         cc = shutil.which("gcc") or shutil.which("cc")
         if cc is None:
             raise RuntimeError("no C compiler found")
-        cmd = [cc, "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out)]
+        tmp = out.with_suffix(f".{os.getpid()}.tmp")          # ranks that start together each replace the file as a whole
+        cmd = [cc, "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(tmp)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("fastcall build failed:\n" + r.stdout + r.stderr)
-        stamp.write_text(want)
+        os.replace(tmp, out)
+        stamp.write_text(_fastcall_want())
     return out
 
 
@@ -89,7 +103,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if force:
         for f in LIBDIR.glob("*.o"):
             f.unlink()
-    _build_fastcall()
+    build_fastcall()
     srcs = sources()
     with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs) or 1)) as ex:
         results = list(ex.map(lambda s: _compile_one(s, verbose), srcs))
