@@ -52,3 +52,25 @@ def test_matches_op_by_op(name, bsz, seq, buckets, monkeypatch):
     assert abs(float(loss - want_loss)) < 1e-3
     for n in want:
         assert (grads[n].float() - want[n].float()).norm() <= 1e-2 * want[n].float().norm() + 1e-7, n
+
+
+def test_parameters_given_other_storage_before_the_backward():
+    """The backward reads the weights where they are then, not where the forward found them."""
+    from zen_repro_b200.models import build_model
+
+    model = build_model("gpt2", device="cuda", num_layers=2, vocab_size=512, max_position=512, **CONFIGS["gpt2"])
+    model.reset_parameters(seed=1)
+    ids = torch.randint(0, 512, (2, 64), device="cuda")
+    model(ids, ids).backward()
+    want = {n: p.grad.clone() for n, p in model.named_parameters()}
+    model.zero_grad(set_to_none=True)
+    loss = model(ids, ids)
+    old = {}
+    for n, p in model.named_parameters():
+        old[n], p.data = p.data, p.data.clone()
+    for t in old.values():
+        t.fill_(float("nan"))                              # still allocated: whoever reads it finds no numbers
+    loss.backward()
+    for n, p in model.named_parameters():
+        if n.startswith("blocks."):
+            assert (p.grad.float() - want[n].float()).norm() <= 1e-2 * want[n].float().norm() + 1e-7, n

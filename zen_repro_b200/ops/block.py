@@ -106,11 +106,15 @@ def usable(blk, x: torch.Tensor, bsz: int, seq: int) -> bool:
 
 
 def _plan_for(blk, params, bsz, seq) -> _Plan:
-    key = (bsz, seq, *[p.data_ptr() for p in params if p is not None])
+    """The plan for the parameters as they are now: asked for in the forward and again in the backward, between which a
+    parameter may have been given other storage (``p.data = ...``, a move to another device and back)."""
+    present = [p for p in params if p is not None]
+    key = (bsz, seq, *[p.data_ptr() for p in present])
+    # not part of what is cached: another tensor may have come to lie at the same address
+    assert all(p.dtype is torch.bfloat16 and p.is_contiguous() for p in present), "block parameters must be contiguous bf16 tensors"
     cached = blk.__dict__.get("_native_plan")
     if cached is None or cached[0] != key:
-        for p in params:
-            assert p is None or (p.dtype == torch.bfloat16 and p.is_contiguous() and p.data_ptr() % 16 == 0)
+        assert all(p.data_ptr() % 16 == 0 for p in present), "block parameters must be 16-byte aligned"
         cached = blk.__dict__["_native_plan"] = (key, _Plan(blk, params, bsz, seq))
     return cached[1]
 
@@ -138,14 +142,15 @@ class BlockFn(torch.autograd.Function):
                 if p is not None:
                     p.zen_expected += 1
         ctx.save_for_backward(x, res, h2, saved, *[p for p in params if p is not None])
-        ctx.args = (blk, params, plan, bsz, seq, claimed, ctx.needs_input_grad[8:])
+        ctx.args = (blk, params, bsz, seq, claimed, ctx.needs_input_grad[8:])
         ctx.set_materialize_grads(False)
         return dn, h2
 
     @staticmethod
     def backward(ctx, d_dn, d_h2):
         x, res, h2, saved, *_ = ctx.saved_tensors          # also checks that no parameter was changed in place since
-        blk, params, plan, bsz, seq, claimed, needs = ctx.args
+        blk, params, bsz, seq, claimed, needs = ctx.args
+        plan = _plan_for(blk, params, bsz, seq)
         dev = x.device
         if d_dn is None:
             d_dn = torch.zeros_like(x)
