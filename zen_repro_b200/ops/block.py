@@ -84,7 +84,7 @@ class _Plan:
         q, h, u = (blk.hq + 2 * blk.hkv) * hd, blk.hq * hd, blk.inner * (2 if cfg.gated else 1)
         for i, (fin, fout) in enumerate(((d, q), (h, d), (d, u), (blk.inner, d))):
             z.fwd[i], z.dx[i] = _pick(G._plan(T, fout, fin, 0)), _pick(G._plan(T, fin, fout, 0))
-            z.fwd_only[i] = _pick(G.plan_in_order(T, fout, fin))
+            z.fwd_only[i] = _pick(G.plan_forward_only(T, fout, fin))
             z.dw[i] = _pick_weight(fin, fout, T) if z.w_in_out else _pick_weight(fout, fin, T)
         self.z, self.addr = z, ctypes.addressof(z)
         sizes = (ctypes.c_int64 * 4)()
