@@ -9,12 +9,13 @@ CONFIGS = {
     "gpt2": dict(hidden_size=128, num_heads=2, num_kv_heads=2, head_dim=64, intermediate_size=512),
     "facebook/opt-2.7b": dict(hidden_size=160, num_heads=2, num_kv_heads=2, head_dim=80, intermediate_size=640),
     "meta-llama/Llama-3.2-3B": dict(hidden_size=256, num_heads=4, num_kv_heads=2, head_dim=64, intermediate_size=320),
+    "gemma-2b": dict(hidden_size=136, num_heads=4, num_kv_heads=1, head_dim=256, intermediate_size=264),
     "google/gemma-2-2b": dict(hidden_size=128, num_heads=2, num_kv_heads=1, head_dim=256, intermediate_size=256),
 }
 
 
 @pytest.mark.parametrize("name,bsz,seq", [("gpt2", 2, 64), ("gpt2", 1, 7), ("facebook/opt-2.7b", 3, 100), ("meta-llama/Llama-3.2-3B", 1, 333),
-                                          ("google/gemma-2-2b", 2, 128)])
+                                          ("gemma-2b", 2, 77), ("google/gemma-2-2b", 2, 128)])
 @pytest.mark.parametrize("buckets", [False, True])
 def test_matches_op_by_op(name, bsz, seq, buckets, monkeypatch):
     from zen_repro_b200.models import build_model
