@@ -706,15 +706,6 @@ void launch_bwd(const CUtensorMap& t128, const CUtensorMap& t64, const CUtensorM
 
 extern "C" {
 
-// Selected one of several head_dim 64 backward kernels in earlier versions.  One is left (csrc/attention_flash.cu), so every
-// choice runs it; kept for callers of that switch.  Returns the previous choice.
-int zen_attn_bwd64_variant(int v) {
-  static int variant = 2;
-  const int old = variant;
-  if (v >= 0 && v <= 2) variant = v;
-  return old;
-}
-
 // CTA pairs that share the query heads of one KV head in the dK / dV kernels (a divisor of Hq / Hkv).  Few KV heads leave
 // pairs idle (4 x 2048, one KV head: 32 pairs of work for 74), more shares cost fp32 partials: the time of both kernels is
 // about 2.8 us per tile and pair, of the busiest pair the average load plus half of the longest share; a share's partials go

@@ -148,7 +148,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant
   if (!*abort_flag) {
     const int r0 = 128 * rank / S, r1 = 128 * (rank + 1) / S;
     constexpr int V = BN / 4;
-    const bool vec = p.out_fp32 ? p.ldc % 4 == 0 : p.ldc % 4 == 0;
+    const bool vec = p.ldc % 4 == 0;                  // four elements of either type
     for (int v = threadIdx.x; v < (r1 - r0) * V; v += 192) {
       const int r = r0 + v / V, c = (v % V) * 4;
       if (m0 + r >= p.M || n0 + c >= p.N) continue;

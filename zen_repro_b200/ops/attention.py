@@ -21,22 +21,19 @@ from .. import _native
 _MODE = os.environ.get("ZEN_ATTN", "auto")        # auto | own | lib
 
 
-def kernel_covers(seq, hq, hkv, hd, dtype, backward: bool = False) -> bool:
+def kernel_covers(seq, hq, hkv, hd, dtype) -> bool:
     """Shapes the tcgen05 attention kernels handle: head sizes up to 256 (multiples of 8) at any sequence length."""
     return dtype == torch.bfloat16 and hq % hkv == 0 and hd <= 256 and hd % 8 == 0
 
 
-def have_kernel(seq, hq, hkv, hd, dtype, softcap: float = 0.0) -> bool:
-    """True when forward AND backward run on the hand-written kernels for this shape."""
-    return _MODE != "lib" and HAVE_BWD and kernel_covers(seq, hq, hkv, hd, dtype, backward=True)
+def have_kernel(seq, hq, hkv, hd, dtype) -> bool:
+    """True when forward and backward run on the hand-written kernels for this shape, soft-capped or not."""
+    return _MODE != "lib" and kernel_covers(seq, hq, hkv, hd, dtype)
 
 
-HAVE_BWD = True
-
-
-def padded_shape(seq, hq, hkv, hd, dtype, softcap: float = 0.0):
+def padded_shape(seq, hq, hkv, hd, dtype):
     """(seq', hd') of the covered shape that (seq, hd) is zero-padded to, or None when padding cannot help."""
-    if _MODE == "lib" or dtype != torch.bfloat16 or hq % hkv or hd > 256 or not HAVE_BWD:
+    if _MODE == "lib" or dtype != torch.bfloat16 or hq % hkv or hd > 256:
         return None
     return seq, (hd + 7) // 8 * 8
 

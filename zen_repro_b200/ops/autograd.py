@@ -471,8 +471,8 @@ class PaddedAttentionFn(torch.autograd.Function):
 def attention(qkv, bsz, seq, hq, hkv, hd, scale=None, softcap: float = 0.0):
     """``softcap`` > 0: scores are soft-capped, cap * tanh(s * scale / cap), before the softmax (Gemma-2)."""
     scale = scale if scale is not None else 1.0 / math.sqrt(hd)
-    if qkv.is_cuda and not A.have_kernel(seq, hq, hkv, hd, qkv.dtype, softcap):
-        pad = A.padded_shape(seq, hq, hkv, hd, qkv.dtype, softcap)
+    if qkv.is_cuda and not A.have_kernel(seq, hq, hkv, hd, qkv.dtype):
+        pad = A.padded_shape(seq, hq, hkv, hd, qkv.dtype)
         if pad is not None:
             return PaddedAttentionFn.apply(qkv, bsz, seq, hq, hkv, hd, scale, softcap, *pad)
         if softcap > 0:

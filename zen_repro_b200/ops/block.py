@@ -100,7 +100,7 @@ def usable(blk, x: torch.Tensor, bsz: int, seq: int) -> bool:
         return False
     if not (G.native_defaults() and A._MODE != "lib" and O._FUSE_ACT_COLSUM):
         return False
-    if cfg.hidden_size % 8 or blk.inner % 8 or hd % 8 or not A.have_kernel(seq, blk.hq, blk.hkv, hd, x.dtype, cfg.attn_softcap):
+    if cfg.hidden_size % 8 or blk.inner % 8 or hd % 8 or not A.have_kernel(seq, blk.hq, blk.hkv, hd, x.dtype):
         return False
     return not (cfg.sliding_window and seq > cfg.sliding_window)
 
