@@ -86,6 +86,15 @@ __device__ __forceinline__ const ZenSparseCtx& zen_ctx(const ZenSparseBatch<NB>&
   }
 }
 
+// Orders this CTA's stores before its arrival at the counter whose last CTA publishes them.  All ranks on one device: GPU scope
+// (a system-scope fence in every CTA costs 4 to 5 us of a launch).  Peers on other devices: by the memory model GPU scope would do
+// here too, since the last CTA's system-scope release is cumulative over what it has seen, but that form has not run between GPUs.
+template <int NB>
+__device__ __forceinline__ void arrive_fence() {
+  if constexpr (NB > 1) __threadfence();
+  else __threadfence_system();
+}
+
 __device__ __forceinline__ uint32_t zen_epoch(const ZenSparseCtx& c) { return c.epoch_dev ? *c.epoch_dev : c.epoch; }
 __device__ __forceinline__ uint2* zen_rec_slots(const ZenSparseCtx& c, int at_rank, int src, uint32_t epoch) {
   return reinterpret_cast<uint2*>(c.sym[at_rank] + c.off_rec) + ((uint64_t)(epoch & 1u) * c.nranks + src) * c.cap_rec;
@@ -439,12 +448,10 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
   if (s_abort) local_status |= ZEN_TIMEOUT;
   if (local_status) atomicOr(c.status, local_status);
   // completion: the last CTA to arrive publishes counts and epochs to the consumers.  Every thread's stores are
-  // ordered before thread 0's system-scope fence by the barrier (the fence is cumulative).
+  // ordered before thread 0's fence by the barrier (the fence is cumulative).
   __syncthreads();
   if (tid == 0) {
-    // GPU scope is enough here: the last CTA's release below is cumulative over what it has seen (a system-scope fence in
-    // every CTA cost 4 to 5 us of a launch)
-    __threadfence();
+    arrive_fence<NB>();
     const uint32_t prev = atomicAdd(&c.cursors[ZEN_MAX_RANKS], 1u);
     s_last = (prev == gridDim.x - 1) ? 1u : 0u;
   }
@@ -804,7 +811,7 @@ zen_gather_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int ppw) {
   if (local_status) atomicOr(c.status, local_status);
   __syncthreads();
   if (tid == 0) {
-    __threadfence();
+    arrive_fence<NB>();
     const uint32_t prev = atomicAdd(&c.cursors[ZEN_MAX_RANKS + 1], 1u);
     s_last = (prev == gridDim.x - 1) ? 1u : 0u;
   }
