@@ -108,13 +108,17 @@ def usable(blk, x: torch.Tensor, bsz: int, seq: int) -> bool:
 def _plan_for(blk, params, bsz, seq) -> _Plan:
     """The plan for the parameters as they are now: asked for in the forward and again in the backward, between which a
     parameter may have been given other storage (``p.data = ...``, a move to another device and back)."""
-    present = [p for p in params if p is not None]
-    key = (bsz, seq, *[p.data_ptr() for p in present])
-    # not part of what is cached: another tensor may have come to lie at the same address
-    assert all(p.dtype is torch.bfloat16 and p.is_contiguous() for p in present), "block parameters must be contiguous bf16 tensors"
+    key = [bsz, seq]
+    for p in params:
+        if p is not None:
+            # not part of what is cached: another tensor may have come to lie at the same address
+            if p.dtype is not torch.bfloat16 or not p.is_contiguous():
+                raise ValueError("block parameters must be contiguous bf16 tensors")
+            key.append(p.data_ptr())
     cached = blk.__dict__.get("_native_plan")
     if cached is None or cached[0] != key:
-        assert all(p.data_ptr() % 16 == 0 for p in present), "block parameters must be 16-byte aligned"
+        if any(at % 16 for at in key[2:]):
+            raise ValueError("block parameters must be 16-byte aligned")
         cached = blk.__dict__["_native_plan"] = (key, _Plan(blk, params, bsz, seq))
     return cached[1]
 
