@@ -1028,7 +1028,7 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
   constexpr float L2E = 1.4426950408889634f;
   const float gscale = gscale_dev ? gscale_host * (*gscale_dev) : gscale_host;
   const float k2 = CAP ? 2.f * L2E / cap : 0.f;
-  const bool vec_ok = ld % 8 == 0;
+  const bool vec_ok = ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) % 16 == 0;
   const int nv = vec_ok ? vocab / 8 : 0;                // vector body; tail handled scalar
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* lp = logits + (size_t)row * ld;

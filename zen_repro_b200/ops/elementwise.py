@@ -39,6 +39,13 @@ def _c(t: torch.Tensor) -> torch.Tensor:
 
 
 # ----------------------------------------------------------------------------- norms
+def _index(t: torch.Tensor, beside: torch.Tensor) -> torch.Tensor:
+    """Token ids or labels as the kernels read them: flat, contiguous, 64-bit, on the device of ``beside``."""
+    if t.get_device() != beside.get_device():
+        raise ValueError(f"ids or labels on {t.device}, the data on {beside.device}")
+    return _c(t if t.dtype is torch.int64 else t.long()).view(-1)
+
+
 def norm_fwd(x, weight, bias=None, residual=None, *, eps=1e-5, layer=False, unit_offset=False, want_h=True):
     """h = x (+ residual); y = norm(h).  Returns (y, h, rstd, mean) -- h is x itself without a residual."""
     cols = x.shape[-1]
@@ -362,7 +369,9 @@ def rope_(x: torch.Tensor, seq: int, theta: float = 10000.0, inverse: bool = Fal
 def embedding_fwd(ids, wte, wpe=None, *, seq: int, pos_offset: int = 0, scale: float = 1.0):
     """out[t] = wte[ids[t]] * scale (+ wpe[pos_offset + t % seq]); ids int64 [tokens]."""
     tokens, d = ids.numel(), wte.shape[1]
-    ids1 = _c(ids).view(-1)
+    ids1 = _index(ids, wte)
+    if wpe is not None and pos_offset + min(seq, tokens) > wpe.shape[0]:
+        raise ValueError(f"sequence of {seq} tokens: the position table has {wpe.shape[0] - pos_offset}")
     if not wte.is_cuda:
         out = wte[ids1]
         if scale != 1.0:
@@ -397,7 +406,7 @@ def embedding_bwd_rows(ids, dy, vocab: int, scale: float = 1.0, scratch: RowSpar
     Only ``count`` leading rows are meaningful; nothing is synchronised with the host.
     """
     tokens, d = ids.numel(), dy.shape[-1]
-    ids1, dy2 = _c(ids).view(-1), _c(dy).view(-1, d)
+    ids1, dy2 = _index(ids, dy), _c(dy).view(-1, d)
     if not dy.is_cuda:
         uniq, inv = torch.unique(ids1, return_inverse=True)
         vals = torch.zeros(uniq.numel(), d, dtype=torch.float32)
@@ -430,7 +439,7 @@ def label_prep(labels: torch.Tensor, shift: int, ignore_index: int = -100, want_
         lab = torch.full_like(labels, ignore_index)
         lab.view(bsz, seq)[:, :seq - shift] = labels.view(bsz, seq)[:, shift:]
         return lab.reshape(-1), 1.0 / (lab != ignore_index).sum().clamp_(min=1).to(torch.float32).reshape(1)
-    labels = _c(labels)
+    labels = _c(labels.long())
     lab = torch.empty(bsz * seq, dtype=labels.dtype, device=labels.device) if want_labels else None
     inv = torch.empty(1, dtype=torch.float32, device=labels.device)
     _native.check(_native.lib().zen_label_prep(labels.data_ptr(), _native.ptr(lab), inv.data_ptr(), bsz, seq, shift, int(ignore_index),
@@ -481,7 +490,9 @@ def cross_entropy(logits, labels, *, grad_scale: float | None = None, ignore_ind
     vocab = logits.shape[-1]
     lg = logits.view(-1, vocab) if logits.dim() != 2 else logits
     rows = lg.shape[0]
-    lb = _c(labels).view(-1)
+    lb = _index(labels, logits)
+    if lb.numel() != rows:
+        raise ValueError(f"{lb.numel()} labels for {rows} rows of logits")
     if not logits.is_cuda:
         lf = lg.float()
         loss = F.cross_entropy(lf, lb, reduction="none", ignore_index=ignore_index)
