@@ -4,7 +4,7 @@
  * convention integer and pointer arguments fill the integer registers and then 8-byte stack slots in order, floats fill the
  * vector registers in order, whatever their order in the prototype; a callee ignores what it does not declare.  So one call
  * form (all integers, then all floats) reaches every function, and a call costs the conversion of its Python numbers: about
- * 0.4 us for 20 arguments, where ctypes took 4 to 5 us, which an eager training step pays about a hundred times.
+ * 0.2 us for 20 arguments, where ctypes took 4 to 5 us, which an eager training step pays about a hundred times.
  *
  * Arguments: int (also bool; pointers are ints), float, None (null pointer), and the ctypes objects that describe structures:
  * byref(x), arrays and structures are passed by address, simple values by value. */

@@ -10,7 +10,7 @@
 // What bounds it: a tile walks K at about 0.25 us per 64-wide block (the latency of loads from HBM over the stages in
 // flight), whatever the other SMs do, so the time is the length of that chain; S slices cut it by S and let S times as
 // many SMs pull the weights.  64 tokens, 50264 -> 768 (input gradient of an LM head, 77 MB of weights): 208 us on the 6 CTAs of
-// the plain kernel; see pick_split in this file for the measured rule.
+// the plain kernel.  When it is taken, with how many slices: cluster_split and _plan in ops/gemm.py, by a time model.
 #include "launch.cuh"
 #include "tc_common.cuh"
 #include "tmap_util.cuh"

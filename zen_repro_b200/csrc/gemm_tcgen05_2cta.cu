@@ -665,15 +665,13 @@ int fill_problem(GemmProblem& q, const void* A, const void* B, void* C, const vo
 int g_force_bn = 0;
 int g_tail_min_kb = 16;            // fewest 64-wide K blocks for which the tiles of the last wave are cut in two; 0 = never
 
-// 256-wide pair tiles.  The 128-wide variant exists for outputs whose 256-wide tiles fill the 74 CTA pairs unevenly
-// (96 tiles = 1.3 waves), but measured on 8192 x 768 outputs it lost (662 vs 858 TFLOP/s at K = 3072, 410 vs 472 at
-// K = 768): with half the columns per tile the A rows are fetched twice as often and the kernel is bound by that
-// traffic, not by the idle third of the second wave.  It is therefore only taken when forced.
-// 192-wide tiles (K-major B only: its half of 96 rows is one TMA box; an MN-major half would need one and a half
-// 64-column boxes) exist for the same 1.3-wave outputs: 8192 x 768 is 96 tiles of 256 = two waves of full tiles, but 128
-// tiles of 192 = two waves of three-quarter tiles.  Measured, they gain nothing either (857.9 TFLOP/s both at
-// 8192 x 768 x 3072): a 256 x 256 x 64 step takes 0.47 us here against 0.28 us of tensor-core time, i.e. the main loop
-// is bound by the operand traffic from L2, which per FLOP is higher for the narrower tile.  Taken only when forced.
+// 256-wide pair tiles.  The narrower ones exist for outputs whose 256-wide tiles fill the 74 CTA pairs unevenly: 8192 x 768 is
+// 96 tiles of 256, 1.3 rounds, or 128 tiles of 192 (K-major B only: its half of 96 rows is one TMA box; an MN-major half would
+// need one and a half 64-column boxes).  Back to back on a B200, us with tiles of 256 / 192 / 128 columns:
+//   8192 x 768 x 768    14.4 / 14.5 / 14.9      8192 x 768 x 3072   33.5 / 33.4 / 38.3
+//   8192 x 3072 x 768   32.2 / 32.7 / 40.2      4096 x 3072 x 8192   143 / 150 / 186
+// With half the columns the A rows are fetched twice as often.  192 columns gain nothing where they even out the rounds (with a
+// cold L2, 8192 x 768 x 768 takes 18.7 us instead of 20.5) and lose 2 to 5 % elsewhere.  Both are taken only when forced.
 int pick_pair_bn(int M, int N, int b_mn, int splits) {
   (void)M; (void)N;
   if (g_force_bn == 192) return (!b_mn && splits == 1) ? 192 : 256;

@@ -841,10 +841,11 @@ zen_gather_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int ppw) {
 // A warp works on three of its chunk pairs at a time: the bitmap words and the value offsets of the one after next are being
 // fetched, the values of the next one travel to shared memory with 16-byte asynchronous copies, and the current one is
 // assembled in shared memory (zeros, then the values at their slots) and written with full 16-byte vectors: the memory system
-// sees whole lines, however few or many values there are.  What bounds it is instruction issue: with one chunk at a time
-// (lane = 32 slots) a chunk took 383 instructions per warp, 312 us for eight ranks of 2^26 bf16 elements at 1 % (164 us of memory
-// time); with two, the prefix sum, the walk of the permutation and the bookkeeping are shared and every lane finds the
-// output place of its own block.
+// sees whole lines, however few or many values there are.  What bounds it now is where the lines go: for eight ranks of 2^26 bf16
+// elements at 1 % it takes 300 us (164 us of memory time), of which plain stores of 128-byte blocks in the same places take 235.
+// Before, instruction issue did: with one chunk at a time (lane = 32 slots) a chunk took 383 instructions per warp, 312 us; with
+// two, the prefix sum, the walk of the permutation and the bookkeeping are shared and every lane finds the output place of its
+// own block.
 #define K4_WARPS 8
 #define K4_VCAP 256                                       // values of a chunk that are staged; with more, the pair is read in place
 template <typename T>
