@@ -27,8 +27,16 @@ typedef int (*any_fn)(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int6
                       int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
                       int64_t, int64_t, int64_t, int64_t, float, float, float, float, float, float, float, float);
 
+/* The address of a ctypes object.  Anything else with a buffer is refused, as ctypes itself does: a NumPy integer has one too, and
+ * its address would pass for its value. */
 static int address_of(PyObject* o, int64_t* out) {
   Py_buffer view;
+  PyObject* owner = PyObject_GetAttrString(o, "_b_needsfree_");
+  if (!owner) {
+    PyErr_Format(PyExc_TypeError, "native call: cannot pass %.100s", Py_TYPE(o)->tp_name);
+    return -1;
+  }
+  Py_DECREF(owner);
   if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) return -1;
   *out = (int64_t)(intptr_t)view.buf;     /* the object outlives the call: the caller's argument list holds it */
   PyBuffer_Release(&view);
