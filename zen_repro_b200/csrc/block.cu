@@ -1,6 +1,6 @@
 // A whole decoder block, forward or backward, from one host call.
 //
-// A block is about 11 launches forward and 17 backward.  Launched op by op from Python, each paid for a tensor allocation, an
+// A block is 7 to 11 launches forward and 16 to 22 backward.  Launched op by op from Python, each paid for a tensor allocation, an
 // autograd node and the wrapper around the call, 15 to 40 us, against kernels of 3 to 10 us for few tokens: a 64-token step of
 // two GPT-2 layers took 3.0 ms of host time for 1.1 ms of kernels.  Here the host work per launch is the launch (about 2 us);
 // activations live in one buffer per block whose layout is computed in this file.
