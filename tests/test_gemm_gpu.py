@@ -261,3 +261,19 @@ def test_grouped_weight_gradients_in_one_launch(shapes):
         assert torch.equal(x, y)
         _check(x, want, K)
     assert G.gemm_error() == 0
+
+
+@pytest.mark.parametrize("N", [8, 64, 130, 257, 264, 520, 1001])
+@pytest.mark.parametrize("bn", [128, 256, 512])
+def test_bias_at_the_edges_of_the_boxes(N, bn):
+    """The bias reaches a row by shuffles from the lanes that hold its columns: widths that end inside a lane's pair, a 32-column
+    chunk, a 64-column box and a tile.  a = 0 leaves the bias alone, which comes through exactly."""
+    torch.manual_seed(21)
+    M, K = 300, 64
+    b = torch.randn(N, K, device="cuda").bfloat16()
+    bias = torch.randn(N, device="cuda").bfloat16()
+    zero = G.gemm_nt(torch.zeros(M, K, device="cuda").bfloat16(), b, bias=bias, bn=bn)
+    assert torch.equal(zero, bias.expand(M, N))
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    _check(G.gemm_nt(a, b, bias=bias, bn=bn), a.float() @ b.float().t() + bias.float(), K)
+    assert G.gemm_error() == 0

@@ -551,11 +551,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
         epilogue_barrier();
       }
+      // Bias: one column per lane, handed round by shuffles (every lane reading all 32 columns two bytes at a time made 3000 x 768 x
+      // 768 12.3 us instead of 8.5).  Sums over ranks take it last, as every rank must add it once.
+      const unsigned short* bias = reinterpret_cast<const unsigned short*>(p.bias);
+      const bool bias_last = p.npeers > 0 && !ag;
 #pragma unroll 1
       for (int ch = 0; ch < BN / 32; ++ch) {
         uint32_t r[32];
-        tmem_ld32(taddr0 + ch * 32, r);         // warp-wide, must not be skipped by single lanes
         const int col0 = n0 + ch * 32;
+        const uint32_t bcol = bias && !bias_last && col0 + lane < p.N ? (uint32_t)bias[col0 + lane] << 16 : 0u;
+        tmem_ld32(taddr0 + ch * 32, r);         // warp-wide, must not be skipped by single lanes
+        if (bias && !bias_last) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(__shfl_sync(0xffffffffu, bcol, i)));
+        }
         if (row < p.M && col0 < p.N) {
           float v[32];
 #pragma unroll
@@ -595,7 +604,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             }
           }
           const bool fullw = (col0 + 32 <= p.N);
-          if (p.bias) {
+          if (p.bias && bias_last) {
             const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0;
 #pragma unroll
             for (int i = 0; i < 32; ++i) if (fullw || col0 + i < p.N) v[i] += __bfloat162float(bp[i]);

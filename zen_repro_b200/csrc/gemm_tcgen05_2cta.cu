@@ -7,7 +7,7 @@
 // CTA's tensor memory receives its 128 accumulator rows.  Per SM that halves the shared-memory traffic of B, which
 // is what bounds the single-CTA kernel.  Roles per CTA: warp 0 TMA producer (both CTAs' loads complete on the
 // leader's "full" barrier), warp 1 MMA issuer (leader only; commits are multicast to both CTAs' barriers),
-// warps 2..5 epilogue.  Bounded waits everywhere; a CTA that gives up still joins the final cluster barrier.
+// the other warps (four or eight) epilogue.  Bounded waits everywhere; a CTA that gives up still joins the final cluster barrier.
 // Operands may be K-major or MN-major as in gemm_tcgen05.cu.
 #include "act_common.cuh"
 #include "launch.cuh"
@@ -28,8 +28,15 @@ template <int BN> struct PairCfg {
   static constexpr int TMEM_COLS = (2 * BN <= 256) ? 256 : 512;        // two accumulators; the allocation is a power of two
   static constexpr int STAGE_BYTES = 128 * 64 * 2 + BNH * 64 * 2;      // A rows of this CTA + its half of B
 };
-constexpr int MAX_SPLITS = 3;      // K slices per output tile at most (the last slice to arrive holds the others' partials in registers)
-constexpr int EPI_STAGE_BYTES = 4 * 2 * 4096;   // per epilogue warp two [32 rows][64 bf16] boxes for the TMA store
+constexpr int MAX_SPLITS = 3;      // K slices per output tile at most
+// Epilogue warps: one per 32 rows, or two of them (one for each half of the columns) where the epilogue has arithmetic to do
+// (bias, activation): a warp alone on its scheduler waits out the latency of everything it does, and with a K of 768 the
+// epilogue of a tile then takes longer than the products of the next one.  Without arithmetic the second warp costs more than it
+// hides.  us, one / two warps, passes of 64 MB between the launches:
+//   8192 x 3072 x 768   plain 37.8 / 39.9   with bias 46.0 / 41.9   with bias and activation 60.3 / 50.2
+//   8192 x 2304 x 768   plain 29.7 / 31.7   with bias 35.7 / 31.8   1024 x 768 x 3072 with bias 27.4 / 25.5
+// (with bias and activation 67.5 with the bias read as described at bias_pair).
+constexpr int EPI_STAGE_BYTES = 8 * 4096;          // boxes of [32 rows][64 bf16] for the TMA store: two per warp, or one
 template <int BN> constexpr int pair_smem_bytes() { return PairCfg<BN>::STAGES * PairCfg<BN>::STAGE_BYTES + EPI_STAGE_BYTES + 1024 + 256; }
 
 __device__ int g_gemm2_error = 0;
@@ -54,7 +61,7 @@ struct GemmGroup {
   GemmProblem pr[MAX_GROUP];
   int n, num_tiles;                 // products, tiles of all of them
   // split-K (one product only): a work unit is (output tile, K slice).  Every unit stores its fp32 partial tile in
-  // `ws`; per 32-row group a counter tells the last unit to arrive, which sums the slices in slice order and writes
+  // `ws`; per 32 rows and half of the columns a counter tells the last unit to arrive, which sums the slices in slice order and writes
   // the output; with two slices and a TMA-stored output the slices exchange half an accumulator each instead.
   int splits, kb_per_split;
   // tail split (splits == 1): the last `tail` tiles of the list, the ones of the launch's final, partly filled wave
@@ -63,7 +70,7 @@ struct GemmGroup {
   int tail;
   float* ws;                        // [slices * tiles][2 CTAs][8 column chunks][8 float4 of a row][128 rows] float4:
                                     // consecutive lanes (rows) are consecutive in memory, so a warp's store covers whole lines
-  int* counters;                    // [tiles][2 CTAs][4 row groups][2], zero between launches
+  int* counters;                    // [tiles][2 CTAs][4 row groups][2 column halves or slices], zero between launches
   // Activation in the epilogue (one product, whole tiles): act = 1 + its mode (act_common.cuh), 0 = none.  The activated tile goes
   // out through `tact`, the product itself only with keep_c.
   CUtensorMap tact;
@@ -141,63 +148,82 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Output of one tile with an activation: the tile itself (with keep_c) and the activated values, both as bf16 boxes of 64
-// columns through the warp's two staging buffers in turn.  The activation reads the rounded values, as a kernel of its own
-// would.  256 activations per thread take about 1.3 us (tanh at 16 per SM and cycle), less than the next tile's products;
-// product + activation of 8192 x 3072 x 768: 80 us as two kernels, 72 here, 62 without the product's own output.
-// (A gate and its factor in one tile, 128 columns of each, was slower than two kernels: 777 x 16 384 x 3072 80 -> 105 us, the
-// two halves of the weight lie a power of two apart and share memory channels.)
-__device__ __forceinline__ void epilogue_act(const GemmGroup& gg, const GemmProblem& p, unsigned char* stg, uint32_t taddr0, int tn, int row0, int lane) {
-  int buf = 0;
-  auto store = [&](const CUtensorMap* map, const uint32_t (&w)[32], int col) {
-    unsigned char* st = stg + buf * 4096;
-    buf ^= 1;
-    if (lane == 0) bulk_wait_read<1>();                // the store that read this buffer two boxes ago is done
-    __syncwarp();
+// Bias of a warp's boxes (64 columns each): lane l holds columns 2 l and 2 l + 1 of a box, fetched before the wait for the
+// products, and hands them round by shuffles.  (Every lane reading every column, 256 two-byte loads a tile, cost 3.3 us per
+// tile: 8192 x 2304 x 768 38 us with a bias against 25 without.)
+__device__ __forceinline__ uint32_t bias_pair(const GemmProblem& p, int col, int lane) {
+  const unsigned short* bp = reinterpret_cast<const unsigned short*>(p.bias);
+  const int c = col + 2 * lane;
+  if (!bp) return 0u;
+  return (c < p.N ? (uint32_t)bp[c] : 0u) | (c + 1 < p.N ? (uint32_t)bp[c + 1] << 16 : 0u);
+}
+__device__ __forceinline__ void add_bias(uint32_t (&ra)[32], uint32_t (&rb)[32], uint32_t pair) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(st + swz128(lane, q * 8)) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-    fence_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      if (col < p.N && row0 < p.M) tma_store_2d(map, st, col, row0);
-      bulk_commit();
-    }
-  };
-  auto load = [&](int at, int col, uint32_t (&w)[32]) {
-    uint32_t ra[32], rb[32];
-    tmem_ld32_nowait(taddr0 + at, ra);
-    tmem_ld32_nowait(taddr0 + at + 32, rb);
-    tmem_wait_ld();
-    if (p.bias) {
-      const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + col;
+  for (int i = 0; i < 16; ++i) {
+    const uint32_t wa = __shfl_sync(0xffffffffu, pair, i), wb = __shfl_sync(0xffffffffu, pair, 16 + i);
+    ra[2 * i] = __float_as_uint(__uint_as_float(ra[2 * i]) + __uint_as_float(wa << 16));
+    ra[2 * i + 1] = __float_as_uint(__uint_as_float(ra[2 * i + 1]) + __uint_as_float(wa & 0xffff0000u));
+    rb[2 * i] = __float_as_uint(__uint_as_float(rb[2 * i]) + __uint_as_float(wb << 16));
+    rb[2 * i + 1] = __float_as_uint(__uint_as_float(rb[2 * i + 1]) + __uint_as_float(wb & 0xffff0000u));
+  }
+}
+// One box of 32 rows and 64 columns: `w` = the lane's row, packed bf16, through the warp's staging buffer `st` to `map`.
+template <int EW>
+__device__ __forceinline__ void store_box(const CUtensorMap* map, unsigned char* st, uint32_t& buf, const uint32_t (&w)[32], int col, int row0, bool inside, int lane) {
+  st += buf;
+  if (EW == 4) buf ^= 4096;
+  if (lane == 0) bulk_wait_read<EW == 4 ? 1 : 0>();    // the store that read this buffer last is done
+  __syncwarp();
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (col + i < p.N) ra[i] = __float_as_uint(__uint_as_float(ra[i]) + __bfloat162float(bp[i]));
-        if (col + 32 + i < p.N) rb[i] = __float_as_uint(__uint_as_float(rb[i]) + __bfloat162float(bp[32 + i]));
-      }
-    }
+  for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(st + swz128(lane, q * 8)) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+  fence_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    if (inside) tma_store_2d(map, st, col, row0);
+    bulk_commit();
+  }
+}
+__device__ __forceinline__ void pack_box(const uint32_t (&ra)[32], const uint32_t (&rb)[32], uint32_t (&w)[32]) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      w[i] = pack_bf16(__uint_as_float(ra[2 * i]), __uint_as_float(ra[2 * i + 1]));
-      w[16 + i] = pack_bf16(__uint_as_float(rb[2 * i]), __uint_as_float(rb[2 * i + 1]));
-    }
-  };
-  const int mode = gg.act - 1;
-#pragma unroll 1
-  for (int cb = 0; cb < 4; ++cb) {
-    const int col = tn * 256 + cb * 64;
-    uint32_t x[32];
-    load(cb * 64, col, x);
-    if (gg.keep_c) store(&p.tc, x, col);
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      x[i] = pack_bf16(zen_act::value(mode, __uint_as_float(x[i] << 16), 0.f), zen_act::value(mode, __uint_as_float(x[i] & 0xffff0000u), 0.f));
-    store(&gg.tact, x, col);
+  for (int i = 0; i < 16; ++i) {
+    w[i] = pack_bf16(__uint_as_float(ra[2 * i]), __uint_as_float(ra[2 * i + 1]));
+    w[16 + i] = pack_bf16(__uint_as_float(rb[2 * i]), __uint_as_float(rb[2 * i + 1]));
   }
 }
 
-template <bool A_MN, bool B_MN, int BN2, bool ACT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// Output of boxes [cb_lo, cb_hi) of one tile with an activation: the product itself (with keep_c) and the activated values.  The
+// activation reads the rounded values, as a kernel of its own would.
+// (A gate and its factor in one tile, 128 columns of each, was slower than two kernels: 777 x 16 384 x 3072 80 -> 105 us, the
+// two halves of the weight lie a power of two apart and share memory channels.)
+template <int EW>
+__device__ __forceinline__ void epilogue_act(const GemmGroup& gg, const GemmProblem& p, unsigned char* stg, uint32_t& buf, uint32_t taddr0, int n0, int row0,
+                                             int cb_lo, int cb_hi, uint32_t bias, int lane) {
+  const int mode = gg.act - 1;
+#pragma unroll 1
+  for (int cb = cb_lo; cb < cb_hi; ++cb) {
+    const int col = n0 + cb * 64;
+    const bool inside = col < p.N && row0 < p.M;
+    const uint32_t next = bias_pair(p, col + 64, lane);
+    uint32_t x[32];
+    {
+      uint32_t ra[32], rb[32];
+      tmem_ld32_nowait(taddr0 + cb * 64, ra);
+      tmem_ld32_nowait(taddr0 + cb * 64 + 32, rb);
+      tmem_wait_ld();
+      if (p.bias) add_bias(ra, rb, bias);
+      bias = next;
+      pack_box(ra, rb, x);
+    }
+    if (gg.keep_c) store_box<EW>(&p.tc, stg, buf, x, col, row0, inside, lane);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      x[i] = pack_bf16(zen_act::value(mode, __uint_as_float(x[i] << 16), 0.f), zen_act::value(mode, __uint_as_float(x[i] & 0xffff0000u), 0.f));
+    store_box<EW>(&gg.tact, stg, buf, x, col, row0, inside, lane);
+  }
+}
+
+template <bool A_MN, bool B_MN, int BN2, int EW, bool ACT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + EW * 32, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
   constexpr int BNH = PairCfg<BN2>::BNH, STAGES2 = PairCfg<BN2>::STAGES, STAGE_BYTES2 = PairCfg<BN2>::STAGE_BYTES;
   extern __shared__ unsigned char smem_raw[];
@@ -207,7 +233,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
   uint64_t* full = bars;                       // [STAGES2]   used on the leader
   uint64_t* empty = bars + STAGES2;            // [STAGES2]   one copy per CTA
   uint64_t* tfull = bars + 2 * STAGES2;        // [2]         one copy per CTA
-  uint64_t* tempty = bars + 2 * STAGES2 + 2;   // [2]         used on the leader, 8 arrivals
+  uint64_t* tempty = bars + 2 * STAGES2 + 2;   // [2]         used on the leader, one arrival per epilogue warp of the pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES2 + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   constexpr uint32_t IDESC = make_idesc(256, BN2, A_MN, B_MN);
@@ -221,7 +247,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 2 * EW); }
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -304,8 +330,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       }
     }
   } else {
-    // -------------------------------------------------------------------- epilogue (warps 2..5, both CTAs)
-    const int grp = warp & 3;
+    // -------------------------------------------------------------------- epilogue (warps 2.., both CTAs)
+    constexpr int HALVES = EW / 4;
+    const int grp = warp & 3, half = HALVES == 2 ? (warp - 2) >> 2 : 0;        // 32 rows, and which half of the tile's 64-column boxes
+    constexpr int BOXES = BN2 / 64;
+    unsigned char* stg = epi_stage + (warp - 2) * (EPI_STAGE_BYTES / EW);
+    uint32_t buf = 0;
     uint32_t tcount = 0;
     bool ok = true;
     for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++tcount) {
@@ -316,24 +346,28 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       tile_coords(p, u.lt, tm, tn);
       const int m0 = tm * 256 + (int)cta * BM2, n0 = tn * BN2;
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
+      const bool split = BN2 == 256 && u.split;
+      // this warp's boxes: half of the tile's, or with two K slices half of what its slice finishes
+      int cb_lo = half ? (BOXES + 1) / 2 : 0, cb_hi = half || HALVES == 1 ? BOXES : (BOXES + 1) / 2;
+      if (split && p.tma_store) { cb_lo = ks * 2 + half; cb_hi = cb_lo + 2 / HALVES; }
+      uint32_t bias = bias_pair(p, n0 + cb_lo * 64, lane);
       if (!mbar_wait(&tfull[acc], aph, abort_flag, 4, &g_gemm2_error)) { ok = false; break; }
       fence_after();
       const int row = m0 + grp * 32 + lane;
       const uint32_t taddr0 = tmem_base + ((uint32_t)(grp * 32) << 16) + acc * BN2;
       if constexpr (ACT) {
-        epilogue_act(gg, p, epi_stage + grp * 8192, taddr0, tn, m0 + grp * 32, lane);
+        epilogue_act<EW>(gg, p, stg, buf, taddr0, n0, m0 + grp * 32, cb_lo, cb_hi, bias, lane);
         fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_leader(&tempty[acc]);
         continue;
       }
-      const bool split = u.split;
       if (split && !p.tma_store) {
         // store this K slice's partial tile and count in.  Every slice but the last to arrive for these 32 rows is
         // done then; the last one adds the others' partials to its own accumulator, in slice order, below.
         float4* wp = reinterpret_cast<float4*>(gg.ws + ((size_t)(ks * num_tiles + tile) * 2 + cta) * (BM2 * BN2)) + (grp * 32 + lane);
 #pragma unroll 1
-        for (int ch = 0; ch < BN2 / 32; ch += 2) {
+        for (int ch = half * (BN2 / 64); ch < (half + 1) * (BN2 / 32 / HALVES); ch += 2) {
           uint32_t r[32], r2[32];
           tmem_ld32_nowait(taddr0 + ch * 32, r);
           tmem_ld32_nowait(taddr0 + ch * 32 + 32, r2);
@@ -348,7 +382,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         }
         __threadfence();
         __syncwarp();
-        int* cnt = gg.counters + (tile * 2 + (int)cta) * 4 + grp;
+        int* cnt = gg.counters + ((tile * 2 + (int)cta) * 4 + grp) * 2 + half;
         int old = 0;
         if (lane == 0) {
           old = atomicAdd(cnt, 1);
@@ -368,20 +402,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         // tensor map) and one lane stores each box with TMA: whole lines, clipped at the matrix edge, no waiting.
         // With two K slices each slice finishes half of the columns: it hands the other half of its accumulator to
         // the peer through the workspace, waits (bounded) for the peer's half and adds it to its own.
-        unsigned char* stg = epi_stage + grp * 8192;
-        int cb_lo = 0, cb_hi = BN2 / 64;
         const float4* peer = nullptr;
         if (split) {
           const int other = 1 - ks;
           float4* wp = reinterpret_cast<float4*>(gg.ws + ((size_t)(ks * u.wtiles + u.wtile) * 2 + cta) * (BM2 * BN2)) + (grp * 32 + lane);
 #pragma unroll 1
-          for (int ch = other * (BN2 / 64); ch < (other + 1) * (BN2 / 64); ch += 2) {
+          for (int give = other * 2 + half; give < other * 2 + half + 2 / HALVES; ++give) {      // the boxes that the peer finishes
             uint32_t r[32], r2[32];
-            tmem_ld32_nowait(taddr0 + ch * 32, r);
-            tmem_ld32_nowait(taddr0 + ch * 32 + 32, r2);
+            tmem_ld32_nowait(taddr0 + give * 64, r);
+            tmem_ld32_nowait(taddr0 + give * 64 + 32, r2);
             tmem_wait_ld();
-            float4* dst = wp + (size_t)ch * (8 * BM2);
-            float4* dst2 = wp + (size_t)(ch + 1) * (8 * BM2);
+            float4* dst = wp + (size_t)(2 * give) * (8 * BM2);
+            float4* dst2 = wp + (size_t)(2 * give + 1) * (8 * BM2);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               dst[i * BM2] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
@@ -390,42 +422,37 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
           }
           __threadfence();
           __syncwarp();
-          // flags[..][ks] = 1: "slice ks has published its half"; the consumer clears it for the next launch
+          // flags[..][ks], bit `half`: "slice ks has published this warp's box"; the consumer clears it for the next launch
           int* flags = gg.counters + ((u.wtile * 2 + (int)cta) * 4 + grp) * 2;
           int got = 1;
           if (lane == 0) {
-            atomicExch(flags + ks, 1);
+            const int bit = 1 << half;
+            atomicOr(flags + ks, bit);
             const uint64_t t0 = gtimer();
-            while (atomicAdd(flags + other, 0) == 0) {
+            while ((atomicAdd(flags + other, 0) & bit) == 0) {
               if (*abort_flag || gtimer() - t0 > WAIT_NS) { got = 0; break; }
             }
-            if (got) atomicExch(flags + other, 0);
+            if (got) atomicAnd(flags + other, ~bit);
             else { *abort_flag = 5; atomicCAS(&g_gemm2_error, 0, 5); }
           }
           got = __shfl_sync(0xffffffffu, got, 0);
           if (!got) { ok = false; break; }
           __threadfence();
           peer = reinterpret_cast<const float4*>(gg.ws + ((size_t)(other * u.wtiles + u.wtile) * 2 + cta) * (BM2 * BN2)) + (grp * 32 + lane);
-          cb_lo = ks * (BN2 / 128);
-          cb_hi = cb_lo + BN2 / 128;
         }
 #pragma unroll 1
         for (int cb = cb_lo; cb < cb_hi; ++cb) {
-          unsigned char* st = stg + (cb & 1) * 4096;
           uint32_t ra[32], rb[32];
+          const uint32_t next = bias_pair(p, n0 + cb * 64 + 64, lane);
           tmem_ld32_nowait(taddr0 + cb * 64, ra);
           tmem_ld32_nowait(taddr0 + cb * 64 + 32, rb);
-          float4 oa[8], ob[8];
           if (split) {
+            float4 oa[8], ob[8];
             const float4* qa = peer + (size_t)(2 * cb) * (8 * BM2);
             const float4* qb = peer + (size_t)(2 * cb + 1) * (8 * BM2);
 #pragma unroll
             for (int i = 0; i < 8; ++i) { oa[i] = __ldcg(qa + i * BM2); ob[i] = __ldcg(qb + i * BM2); }
-          }
-          if (lane == 0) bulk_wait_read<1>();          // the store that read this buffer two boxes ago is done
-          __syncwarp();
-          tmem_wait_ld();
-          if (split) {
+            tmem_wait_ld();
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               ra[4 * i] = __float_as_uint(__uint_as_float(ra[4 * i]) + oa[i].x);
@@ -437,35 +464,15 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
               rb[4 * i + 2] = __float_as_uint(__uint_as_float(rb[4 * i + 2]) + ob[i].z);
               rb[4 * i + 3] = __float_as_uint(__uint_as_float(rb[4 * i + 3]) + ob[i].w);
             }
+          } else {
+            tmem_wait_ld();
           }
           const int col0 = n0 + cb * 64;
-          if (p.bias) {
-            const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (col0 + i < p.N) ra[i] = __float_as_uint(__uint_as_float(ra[i]) + __bfloat162float(bp[i]));
-              if (col0 + 32 + i < p.N) rb[i] = __float_as_uint(__uint_as_float(rb[i]) + __bfloat162float(bp[32 + i]));
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            *reinterpret_cast<uint4*>(st + swz128(lane, q * 8)) =
-                make_uint4(pack_bf16(__uint_as_float(ra[8 * q]), __uint_as_float(ra[8 * q + 1])),
-                           pack_bf16(__uint_as_float(ra[8 * q + 2]), __uint_as_float(ra[8 * q + 3])),
-                           pack_bf16(__uint_as_float(ra[8 * q + 4]), __uint_as_float(ra[8 * q + 5])),
-                           pack_bf16(__uint_as_float(ra[8 * q + 6]), __uint_as_float(ra[8 * q + 7])));
-            *reinterpret_cast<uint4*>(st + swz128(lane, 32 + q * 8)) =
-                make_uint4(pack_bf16(__uint_as_float(rb[8 * q]), __uint_as_float(rb[8 * q + 1])),
-                           pack_bf16(__uint_as_float(rb[8 * q + 2]), __uint_as_float(rb[8 * q + 3])),
-                           pack_bf16(__uint_as_float(rb[8 * q + 4]), __uint_as_float(rb[8 * q + 5])),
-                           pack_bf16(__uint_as_float(rb[8 * q + 6]), __uint_as_float(rb[8 * q + 7])));
-          }
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (col0 < p.N && m0 + grp * 32 < p.M) tma_store_2d(&p.tc, st, col0, m0 + grp * 32);
-            bulk_commit();
-          }
+          if (p.bias) add_bias(ra, rb, bias);
+          bias = next;
+          uint32_t w[32];
+          pack_box(ra, rb, w);
+          store_box<EW>(&p.tc, stg, buf, w, col0, m0 + grp * 32, col0 < p.N && m0 + grp * 32 < p.M, lane);
         }
         fence_before();
         __syncwarp();
@@ -473,36 +480,28 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         continue;
       }
 #pragma unroll 1
-      for (int ch = 0; ch < BN2 / 32; ++ch) {
+      for (int ch = half * (BN2 / 64); ch < (half + 1) * (BN2 / 32 / HALVES); ++ch) {
         uint32_t r[32];
         if (split) {
-          // the other slices' partials of this chunk first (independent loads, all in flight together), then the
-          // own accumulator; the sum runs over slice indices whichever slice arrived last
-          float4 buf[MAX_SPLITS][8];
+          // the sum runs over slice indices whichever slice arrived last; one slice's partials in flight at a time (all of
+          // them do not fit in the registers)
           const float4* src = reinterpret_cast<const float4*>(gg.ws + ((size_t)tile * 2 + cta) * (BM2 * BN2)) + (size_t)ch * (8 * BM2) + (grp * 32 + lane);
-#pragma unroll
-          for (int sidx = 0; sidx < MAX_SPLITS; ++sidx) {
-            if (sidx < gg.splits && sidx != ks) {
-              const float4* q = src + (size_t)sidx * num_tiles * 2 * (BM2 * BN2 / 4);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) buf[sidx][i] = __ldcg(q + i * BM2);
-            }
-          }
           tmem_ld32(taddr0 + ch * 32, r);
           float a[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) a[i] = 0.f;
+#pragma unroll 1
+          for (int sidx = 0; sidx < gg.splits; ++sidx) {
+            if (sidx == ks) {
 #pragma unroll
-          for (int sidx = 0; sidx < MAX_SPLITS; ++sidx) {
-            if (sidx < gg.splits) {
-              const bool own = (sidx == ks);
+              for (int i = 0; i < 32; ++i) a[i] += __uint_as_float(r[i]);
+            } else {
+              const float4* q = src + (size_t)sidx * num_tiles * 2 * (BM2 * BN2 / 4);
+              float4 buf[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                a[4 * i] += own ? __uint_as_float(r[4 * i]) : buf[sidx][i].x;
-                a[4 * i + 1] += own ? __uint_as_float(r[4 * i + 1]) : buf[sidx][i].y;
-                a[4 * i + 2] += own ? __uint_as_float(r[4 * i + 2]) : buf[sidx][i].z;
-                a[4 * i + 3] += own ? __uint_as_float(r[4 * i + 3]) : buf[sidx][i].w;
-              }
+              for (int i = 0; i < 8; ++i) buf[i] = __ldcg(q + i * BM2);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { a[4 * i] += buf[i].x; a[4 * i + 1] += buf[i].y; a[4 * i + 2] += buf[i].z; a[4 * i + 3] += buf[i].w; }
             }
           }
 #pragma unroll
@@ -583,19 +582,24 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
   }
 }
 
-template <bool A_MN, bool B_MN, int BN2, bool ACT = false>
-int launch2(const GemmGroup& g, cudaStream_t st) {
+template <bool A_MN, bool B_MN, int BN2, int EW, bool ACT = false>
+int launch2_as(const GemmGroup& g, cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_2cta_kernel<A_MN, B_MN, BN2, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes<BN2>());
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_2cta_kernel<A_MN, B_MN, BN2, EW, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes<BN2>());
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
   const int units = g.tail ? g.num_tiles + g.tail : g.num_tiles * g.splits;
   int clusters = zen_tmap::sm_count() / 2;
   if (units < clusters) clusters = units;
-  zen_pdl::launch(gemm_bf16_2cta_kernel<A_MN, B_MN, BN2, ACT>, clusters * 2, 192, pair_smem_bytes<BN2>(), st, g);
+  zen_pdl::launch(gemm_bf16_2cta_kernel<A_MN, B_MN, BN2, EW, ACT>, clusters * 2, 64 + EW * 32, pair_smem_bytes<BN2>(), st, g);
   return (int)cudaGetLastError();
+}
+
+template <bool A_MN, bool B_MN, int BN2>
+int launch2(const GemmGroup& g, cudaStream_t st) {
+  return g.pr[0].bias ? launch2_as<A_MN, B_MN, BN2, 8>(g, st) : launch2_as<A_MN, B_MN, BN2, 4>(g, st);   // a group has no bias
 }
 
 int launch2_layout(const GemmGroup& g, int a_mn, int b_mn, int bn, cudaStream_t st) {
@@ -763,7 +767,7 @@ int zen_gemm_bf16_2cta_act(const void* A, const void* B, void* C, const void* bi
   g.ws = nullptr; g.counters = nullptr;
   g.tail = 0;
   g.act = mode + 1; g.keep_c = keep_c;
-  return b_mn ? launch2<false, true, 256, true>(g, (cudaStream_t)stream) : launch2<false, false, 256, true>(g, (cudaStream_t)stream);
+  return b_mn ? launch2_as<false, true, 256, 8, true>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 8, true>(g, (cudaStream_t)stream);
 }
 
 // Several products with the same operand layouts in ONE launch (see GemmProblem): the tiles of all of them form one
