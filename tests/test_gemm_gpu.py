@@ -277,3 +277,36 @@ def test_bias_at_the_edges_of_the_boxes(N, bn):
     a = torch.randn(M, K, device="cuda").bfloat16()
     _check(G.gemm_nt(a, b, bias=bias, bn=bn), a.float() @ b.float().t() + bias.float(), K)
     assert G.gemm_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 264, 136), (512, 9520, 64), (8192, 776, 200), (2100, 2440, 72), (1000, 9344, 320)])
+def test_halved_tiles_equal_whole_ones(M, N, K):
+    """The tiles of a partly filled last wave run as two halves of 128 columns (all of them, some, ragged second halves): every
+    layout and output path, bit for bit what whole tiles give, since no element is summed in another order."""
+    from zen_repro_b200 import _native
+    lib = _native.lib()
+    torch.manual_seed(31)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = torch.randn(N, K, device="cuda").bfloat16()
+    bias = torch.randn(N, device="cuda").bfloat16()
+    at, bt = a.t().contiguous(), b.t().contiguous()
+
+    def everything():
+        acc, acc32 = torch.ones(M, N, device="cuda").bfloat16(), torch.ones(M, N, device="cuda")
+        G.gemm_nt(a, b, out=acc, accumulate=True, bn=512)
+        G.gemm_nn(a, bt, out=acc32, accumulate=True, bn=512)
+        outs = [G.gemm_nt(a, b, bn=512), G.gemm_nt(a, b, bias=bias, bn=512), G.gemm_nn(a, bt, bn=512), acc, acc32]
+        if M % 8 == 0:
+            outs.append(G.gemm_tn(at, bt, bn=512))
+        return outs
+
+    old = lib.zen_gemm2_tail_split(0)
+    try:
+        whole = everything()
+    finally:
+        lib.zen_gemm2_tail_split(old)
+    halves = everything()
+    for x, y in zip(halves, whole):
+        assert torch.equal(x, y)
+    _check(halves[0], a.float() @ b.float().t(), K)
+    assert G.gemm_error() == 0

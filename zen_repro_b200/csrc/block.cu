@@ -144,7 +144,7 @@ struct Call {
   void gemm(const GemmPick& k, const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, void* C, int ldc, const void* bias,
             int M, int N, int K, int acc) {
     if (rc) return;
-    if (k.kind == 1)                                       // p1: whole tiles, no workspace to cut the last round's with
+    if (k.kind == 1)                                       // p1: no workspace to cut the last round's K with
       rc = zen_gemm_bf16_2cta_splitk(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, 0, acc, k.p0, k.p1 ? nullptr : w.ws, k.p1 ? 0 : w.n_ws,
                                      k.p1 ? nullptr : w.cnt, k.p1 ? 0 : w.n_cnt, 0, st);
     else if (k.kind == 2 && reinterpret_cast<uintptr_t>(C) % 16 == 0)

@@ -48,6 +48,7 @@ __device__ int g_gemm2_error = 0;
 constexpr int MAX_GROUP = 6;
 struct GemmProblem {
   CUtensorMap ta, tb, tc;
+  CUtensorMap tb_half;              // K-major B in boxes of half as many rows, for units of half a tile
   void* C;
   const void* bias;
   int M, N, K, ldc;
@@ -61,13 +62,13 @@ struct GemmGroup {
   GemmProblem pr[MAX_GROUP];
   int n, num_tiles;                 // products, tiles of all of them
   // split-K (one product only): a work unit is (output tile, K slice).  Every unit stores its fp32 partial tile in
-  // `ws`; per 32 rows and half of the columns a counter tells the last unit to arrive, which sums the slices in slice order and writes
-  // the output; with two slices and a TMA-stored output the slices exchange half an accumulator each instead.
+  // `ws`; per 32 rows and epilogue warp a counter tells the last unit to arrive, which sums the slices in slice order and
+  // writes the output; with two slices and a TMA-stored output the slices exchange half an accumulator each instead.
   int splits, kb_per_split;
   // tail split (splits == 1): the last `tail` tiles of the list, the ones of the launch's final, partly filled wave
-  // of clusters, are cut into two K halves that run side by side in that wave and exchange half an accumulator
-  // each (the two-slice TMA-store path); 0 = every tile is one unit
-  int tail;
+  // of clusters, run as two units each, side by side in that wave: with tail_k two K halves that exchange half an
+  // accumulator each (the two-slice TMA-store path), else two halves of the columns; 0 = every tile is one unit
+  int tail, tail_k;
   float* ws;                        // [slices * tiles][2 CTAs][8 column chunks][8 float4 of a row][128 rows] float4:
                                     // consecutive lanes (rows) are consecutive in memory, so a warp's store covers whole lines
   int* counters;                    // [tiles][2 CTAs][4 row groups][2 column halves or slices], zero between launches
@@ -77,33 +78,31 @@ struct GemmGroup {
   int act, keep_c;
 };
 
-// One unit of work of a cluster: an output tile, or one K slice of it.
+// One unit of work of a cluster: an output tile, one K slice of it, or half of its columns.
 struct Unit {
   int pi, tile, lt, ks, kb0, kb1;   // product, tile in the launch's list, tile within the product, K slice and its blocks
-  int wtile, wtiles;                // index of the tile among the split ones and their number (workspace / flag addressing)
-  bool split;
+  int part;                         // columns: 0 all, 1 first half, 2 second half
+  int wtile, wtiles;                // index of the tile among those cut along K and their number (workspace / flag addressing)
+  bool split;                       // one of several K slices
 };
 __device__ __forceinline__ Unit decode_unit(const GemmGroup& g, int unit) {
   Unit u;
-  const int T = g.num_tiles;
-  if (g.tail == 0) {
-    u.tile = unit % T;
+  const int T = g.num_tiles, whole = T - g.tail;
+  u.ks = u.part = 0;
+  u.wtile = u.tile = unit;
+  u.wtiles = T;
+  u.split = g.splits > 1;
+  if (g.splits > 1) {
+    u.wtile = u.tile = unit % T;
     u.ks = unit / T;
-    u.split = g.splits > 1;
-    u.wtile = u.tile;
-    u.wtiles = T;
-  } else {
-    const int whole = T - g.tail;
+  } else if (unit >= whole) {
+    const int second = unit - whole >= g.tail ? 1 : 0;
+    u.wtile = unit - whole - second * g.tail;
     u.wtiles = g.tail;
-    if (unit < whole) {
-      u.tile = unit; u.ks = 0; u.split = false; u.wtile = 0;
-    } else {
-      const int j = unit - whole;
-      u.ks = j >= g.tail ? 1 : 0;
-      u.wtile = j - u.ks * g.tail;
-      u.tile = whole + u.wtile;
-      u.split = true;
-    }
+    u.tile = whole + u.wtile;
+    u.split = g.tail_k != 0;
+    if (g.tail_k) u.ks = second;
+    else u.part = 1 + second;
   }
   u.pi = 0;
 #pragma unroll
@@ -111,16 +110,9 @@ __device__ __forceinline__ Unit decode_unit(const GemmGroup& g, int unit) {
     if (i < g.n && u.tile >= g.pr[i].tile_start) u.pi = i;
   u.lt = u.tile - g.pr[u.pi].tile_start;
   const int nkb = (g.pr[u.pi].K + BK2 - 1) / BK2;
-  if (g.tail == 0) {
-    u.kb0 = u.ks * g.kb_per_split;
-    u.kb1 = min(nkb, u.kb0 + g.kb_per_split);
-  } else if (!u.split) {
-    u.kb0 = 0; u.kb1 = nkb;
-  } else {
-    const int half = (nkb + 1) / 2;
-    u.kb0 = u.ks ? half : 0;
-    u.kb1 = u.ks ? nkb : half;
-  }
+  const int per = u.split && g.splits == 1 ? (nkb + 1) / 2 : g.kb_per_split;
+  u.kb0 = u.ks * per;
+  u.kb1 = min(nkb, u.kb0 + per);
   return u;
 }
 
@@ -236,7 +228,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
   uint64_t* tempty = bars + 2 * STAGES2 + 2;   // [2]         used on the leader, one arrival per epilogue warp of the pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES2 + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  constexpr uint32_t IDESC = make_idesc(256, BN2, A_MN, B_MN);
+  constexpr uint32_t IDESC = make_idesc(256, BN2, A_MN, B_MN), IDESC_HALF = make_idesc(256, BN2 / 2, A_MN, B_MN);
   constexpr int A_BYTES = BM2 * BK2 * 2;
 
   const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -269,14 +261,16 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         const GemmProblem& p = gg.pr[u.pi];
         int tm, tn;
         tile_coords(p, u.lt, tm, tn);
-        const int m0 = tm * 256 + (int)cta * BM2, n0 = tn * BN2 + (int)cta * BNH;
+        const int nh = u.part ? BNH / 2 : BNH;               // rows of B that this CTA holds
+        const int m0 = tm * 256 + (int)cta * BM2, n0 = tn * BN2 + (u.part == 2 ? BNH : 0) + (int)cta * nh;
+        const uint32_t bytes = 2 * (A_BYTES + nh * (BK2 * 2));
         for (int kb = u.kb0; kb < u.kb1; ++kb, ++it) {
           const int s = it % STAGES2;
           const uint32_t ph = (it / STAGES2) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, 1, &g_gemm2_error)) { ok = false; break; }
           unsigned char* sa = smem + s * STAGE_BYTES2;
           unsigned char* sb = sa + A_BYTES;
-          if (cta == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES2);
+          if (cta == 0) mbar_expect_tx(&full[s], bytes);
           const int k0 = kb * BK2;
           if (!A_MN) {
             tma_load_2d_pair(sa, &p.ta, &full[s], k0, m0);
@@ -285,10 +279,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
             for (int j = 0; j < BM2 / 64; ++j) tma_load_2d_pair(sa + j * 8192, &p.ta, &full[s], m0 + 64 * j, k0);
           }
           if (!B_MN) {
-            tma_load_2d_pair(sb, &p.tb, &full[s], k0, n0);
+            tma_load_2d_pair(sb, u.part ? &p.tb_half : &p.tb, &full[s], k0, n0);
           } else {
 #pragma unroll
-            for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(sb + j * 8192, &p.tb, &full[s], n0 + 64 * j, k0);
+            for (int j = 0; j < BNH / 64; ++j)
+              if (64 * j < nh) tma_load_2d_pair(sb + j * 8192, &p.tb, &full[s], n0 + 64 * j, k0);
           }
         }
       }
@@ -307,6 +302,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         const uint32_t d_tmem = tmem_u + acc * BN2;
         const Unit u = decode_unit(gg, unit);
         const int kb0 = u.kb0, kb1 = u.kb1;
+        const uint32_t idesc = u.part ? IDESC_HALF : IDESC;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES2;
           const uint32_t ph = (it / STAGES2) & 1;
@@ -321,7 +317,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
             for (int j = 0; j < BK2 / 16; ++j) {
               const uint64_t astep = (uint64_t)((A_MN ? j * 2048 : j * 32) >> 4);
               const uint64_t bstep = (uint64_t)((B_MN ? j * 2048 : j * 32) >> 4);
-              umma_bf16_pair(d_tmem, adesc + astep, bdesc + bstep, IDESC, (kb != kb0 || j != 0) ? 1u : 0u);
+              umma_bf16_pair(d_tmem, adesc + astep, bdesc + bstep, idesc, (kb != kb0 || j != 0) ? 1u : 0u);
             }
             umma_commit_pair(&empty[s]);
           }
@@ -344,11 +340,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       const int tile = u.tile, ks = u.ks;
       int tm, tn;
       tile_coords(p, u.lt, tm, tn);
-      const int m0 = tm * 256 + (int)cta * BM2, n0 = tn * BN2;
+      const int m0 = tm * 256 + (int)cta * BM2, n0 = tn * BN2 + (u.part == 2 ? BNH : 0);
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
       const bool split = BN2 == 256 && u.split;
       // this warp's boxes: half of the tile's, or with two K slices half of what its slice finishes
-      int cb_lo = half ? (BOXES + 1) / 2 : 0, cb_hi = half || HALVES == 1 ? BOXES : (BOXES + 1) / 2;
+      const int boxes = u.part ? BOXES / 2 : BOXES;
+      int cb_lo = half ? (boxes + 1) / 2 : 0, cb_hi = half || HALVES == 1 ? boxes : (boxes + 1) / 2;
       if (split && p.tma_store) { cb_lo = ks * 2 + half; cb_hi = cb_lo + 2 / HALVES; }
       uint32_t bias = bias_pair(p, n0 + cb_lo * 64, lane);
       if (!mbar_wait(&tfull[acc], aph, abort_flag, 4, &g_gemm2_error)) { ok = false; break; }
@@ -479,8 +476,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
         if (lane == 0) mbar_arrive_leader(&tempty[acc]);
         continue;
       }
+      // 32-column chunks of this warp: as many as its boxes of 64 would be (192-wide tiles: three of six)
+      const int chunks = (u.part ? BN2 / 64 : BN2 / 32) / HALVES;
 #pragma unroll 1
-      for (int ch = half * (BN2 / 64); ch < (half + 1) * (BN2 / 32 / HALVES); ++ch) {
+      for (int ch = half * chunks; ch < (half + 1) * chunks; ++ch) {
         uint32_t r[32];
         if (split) {
           // the sum runs over slice indices whichever slice arrived last; one slice's partials in flight at a time (all of
@@ -645,6 +644,8 @@ int fill_problem(GemmProblem& q, const void* A, const void* B, void* C, const vo
   if (!b_mn) rc = zen_tmap::get(B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, (uint32_t)(bn / 2), &q.tb);
   else rc = zen_tmap::get(B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, 64, &q.tb);
   if (rc) return rc;
+  q.tb_half = q.tb;
+  if (!b_mn && bn == 256 && (rc = zen_tmap::get(B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, 64, &q.tb_half))) return rc;
   // Plain bf16 output with a TMA-compatible layout: store through shared memory.  The stored width must be a
   // multiple of 8 columns (16 bytes); a caller whose buffer has spare columns after N may allow them to be written
   // (with zeros) by passing n_store = N rounded up.
@@ -667,7 +668,30 @@ int fill_problem(GemmProblem& q, const void* A, const void* B, void* C, const vo
 }  // namespace
 
 int g_force_bn = 0;
-int g_tail_min_kb = 16;            // fewest 64-wide K blocks for which the tiles of the last wave are cut in two; 0 = never
+int g_tail_min_kb = 1;             // fewest 64-wide K blocks for which the tiles of the last wave are cut in two; 0 = never
+
+// The tiles of the last, partly filled wave of clusters run as two units each when both units of all of them fit in that wave.
+// Halves of 128 columns need nothing from each other and sum every element in the order of a whole tile, but each reads its
+// rows of A again, and what bounds a tile is what its SMs draw from L2: three quarters of a tile's time.  K halves take half
+// of it, and about 4 us to exchange half an accumulator each through memory; they pay from K = 4096 on (and need the TMA store and
+// a workspace).  us, K halves / column halves: the 108 tiles of a GPT-2 layer's weight gradients, K = 8192, 75 / 80;
+// 8192 x 768 x 3072 40.9 / 40.9; 8192 x 768 x 2304 34.7 / 32.7; 8192 x 3072 x 768 38.8 (whole) / 36.8; 700 x 2304 x 9216 without
+// a workspace 55.1 (whole) / 47.0.
+constexpr int TAIL_K_MIN_KB = 64;
+static void cut_tail(GemmGroup& g, int min_kb) {
+  const int clusters = zen_tmap::sm_count() / 2, rem = g.num_tiles % clusters;
+  g.tail = g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && 2 * rem <= clusters ? rem : 0;
+  g.tail_k = g.tail > 0 && min_kb >= TAIL_K_MIN_KB && g.ws && g.counters;
+  for (int i = 0; i < g.n && g.tail_k; ++i) {
+    const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
+    if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
+  }
+}
+// Whether a caller's workspace holds the halves of the tiles that a last wave may have: half of the clusters.
+static bool tail_workspace(const float* ws, uint64_t ws_floats, const int* counters, int n_counters) {
+  const int most = zen_tmap::sm_count() / 4;
+  return ws && counters && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && ws_floats >= (uint64_t)most * 2 * 2 * BM2 * 256 && n_counters >= most * 16;
+}
 
 // 256-wide pair tiles.  The narrower ones exist for outputs whose 256-wide tiles fill the 74 CTA pairs unevenly: 8192 x 768 is
 // 96 tiles of 256, 1.3 rounds, or 128 tiles of 192 (K-major B only: its half of 96 rows is one TMA box; an MN-major half would
@@ -689,8 +713,8 @@ extern "C" {
 // long K, the weight-gradient shape): `ws` must hold splits * tiles * 2 * 128 * 256 floats and `counters`
 // tiles * 16 ints that are zero on entry (the kernel leaves them zero); both are caller-owned and used in stream
 // order.  The slices are summed in slice order, so the result does not depend on timing.
-// With splits == 1 a caller may still pass `ws` and `counters` (same sizes as for two slices of one wave of clusters):
-// the launcher then cuts the tiles of the last, partly filled wave in two (see zen_gemm2_tail_split).
+// With splits == 1 a caller may still pass `ws` and `counters` (sizes as for two slices of one wave of clusters): the tiles of a
+// partly filled last wave may then be cut along K (cut_tail).
 // n_store: 0, or a width in [N, ldc] that the kernel may write (columns N.. receive zeros).
 int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                               int ldb, int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int splits, float* ws,
@@ -734,17 +758,10 @@ int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void*
   g.kb_per_split = kb_per;
   g.ws = ws;
   g.counters = counters;
-  // Tail split: the tiles of the last, partly filled wave of clusters run as two K slices each when both slices of
-  // all of them fit in that wave (so that the slices that wait for each other are resident together, as above) and K
-  // is long enough for half a tile to outweigh the exchange of half an accumulator.
-  g.tail = 0;
-  if (splits == 1 && bn == 256 && g.pr[0].tma_store && g_tail_min_kb > 0 && nkb >= g_tail_min_kb && ws && counters &&
-      (reinterpret_cast<uintptr_t>(ws) % 16) == 0) {
-    const int clusters = zen_tmap::sm_count() / 2;
-    const int rem = g.num_tiles % clusters;
-    if (g.num_tiles > clusters && rem > 0 && 2 * rem <= clusters && ws_floats >= (uint64_t)rem * 2 * 2 * BM2 * 256 &&
-        n_counters >= rem * 16)
-      g.tail = rem;
+  g.tail = g.tail_k = 0;
+  if (splits == 1 && bn == 256) {
+    if (!tail_workspace(ws, ws_floats, counters, n_counters)) g.ws = nullptr;
+    cut_tail(g, nkb);
   }
   return launch2_layout(g, a_mn, b_mn, bn, (cudaStream_t)stream);
 }
@@ -765,15 +782,15 @@ int zen_gemm_bf16_2cta_act(const void* A, const void* B, void* C, const void* bi
   g.splits = 1;
   g.kb_per_split = (K + BK2 - 1) / BK2;
   g.ws = nullptr; g.counters = nullptr;
-  g.tail = 0;
+  cut_tail(g, g.kb_per_split);
   g.act = mode + 1; g.keep_c = keep_c;
   return b_mn ? launch2_as<false, true, 256, 8, true>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 8, true>(g, (cudaStream_t)stream);
 }
 
 // Several products with the same operand layouts in ONE launch (see GemmProblem): the tiles of all of them form one
-// list that the persistent clusters walk, and the tiles of the last, partly filled wave are cut into two K halves when
-// their outputs take the TMA-store path.  `descs`: n records of ZenGemmDesc; every product follows the contract of
-// zen_gemm_bf16_2cta (no bias).  ws / counters as for zen_gemm_bf16_2cta_splitk (may be null: no tail split).
+// list that the persistent clusters walk, and the tiles of the last, partly filled wave are cut in two (cut_tail).  `descs`: n records of ZenGemmDesc; every product follows the contract of
+// zen_gemm_bf16_2cta (no bias).  ws / counters as for zen_gemm_bf16_2cta_splitk (may be null: K is
+// not cut).
 struct ZenGemmDesc {
   const void* A;
   const void* B;
@@ -806,18 +823,8 @@ int zen_gemm_bf16_2cta_group(const ZenGemmDesc* descs, int n, int a_mn, int b_mn
   g.kb_per_split = 1 << 30;
   g.ws = ws;
   g.counters = counters;
-  g.tail = 0;
-  const int clusters = zen_tmap::sm_count() / 2;
-  const int rem = tiles % clusters;
-  if (g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && ws && counters && (reinterpret_cast<uintptr_t>(ws) % 16) == 0 &&
-      rem > 0 && 2 * rem <= clusters && ws_floats >= (uint64_t)rem * 2 * 2 * BM2 * 256 && n_counters >= rem * 16) {
-    bool ok = true;                                           // every tile of the tail must take the two-slice store path
-    for (int i = 0; i < n; ++i) {
-      const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
-      if (end > tiles - rem && !g.pr[i].tma_store) ok = false;
-    }
-    if (ok) g.tail = rem;
-  }
+  if (!tail_workspace(ws, ws_floats, counters, n_counters)) g.ws = nullptr;
+  cut_tail(g, min_kb);
   return launch2_layout(g, a_mn, b_mn, 256, (cudaStream_t)stream);
 }
 
@@ -828,11 +835,11 @@ int zen_gemm2_force_bn(int bn) {
   return old;
 }
 
-// Fewest K blocks (of 64) from which the tiles of a launch's last, partly filled wave run as two K slices; 0 switches
-// the tail split off.  Returns the previous setting.
+// Fewest K blocks (of 64) from which the tiles of a launch's last, partly filled wave run as two units; 0 switches
+// that off.  Returns the previous setting.
 int zen_gemm2_tail_split(int min_kb) {
   const int old = g_tail_min_kb;
-  if (min_kb >= 0) g_tail_min_kb = (min_kb > 0 && min_kb < 2) ? 2 : min_kb;
+  if (min_kb >= 0) g_tail_min_kb = min_kb;
   return old;
 }
 

@@ -41,7 +41,7 @@ def _clusters() -> int:
 _T_ONE128 = (128, 128, 148, 11.6, 0.22, 1.0)
 _T_ONE256 = (128, 256, 148, 13.2, 0.38, 1.5)
 _T_PAIR = (256, 256, 74, 13.0, 0.306, 1.0)
-_TAIL_ROUND = 0.75                  # a last round that runs as two K halves
+_TAIL_ROUND = 0.75                  # a last round whose tiles run as two halves of their columns
 _SPLIT_EXCHANGE = 5.0               # two K slices of the pair kernel meeting through the workspace
 _CLUSTER_START = 13.0               # csrc/gemm_splitk.cu: launch, cluster barriers and the sum over shared memory
 # CTAs that clusters of up to 8 are sure to get side by side: with 132 and more, a second wave starts (18 -> 31 us measured
@@ -63,7 +63,7 @@ def _t_pair(M, N, nkb):
     bm, bn, _, start, step, store = _T_PAIR
     per = _clusters()
     full, rem = divmod(_tiles(M, N, bm, bn), per)
-    tail = 0.0 if rem == 0 else (_TAIL_ROUND if full and 2 * rem <= per and nkb >= 16 else 1.0)
+    tail = 0.0 if rem == 0 else (_TAIL_ROUND if 2 * rem <= per else 1.0)
     return start + (full + tail) * nkb * step + max(0, full - (rem == 0)) * store
 
 
@@ -178,10 +178,10 @@ def _plan(M: int, N: int, K: int, bn: int):
 
 @functools.lru_cache(maxsize=4096)
 def plan_forward_only(M: int, N: int, K: int):
-    """The plan for the products of a block that no backward will follow (scoring, validation).  K is cut into two at most, in two
-    places: by ``split_k_choice`` (from 256 rows, K from 4096, tiles for at most half of the CTA pairs), and in the last round of
-    an output of at least 512 rows whose tiles fill 60 % of the pairs' rounds.  Never among the clusters of csrc/gemm_splitk.cu,
-    nor in the last round of smaller outputs; a third element 1 asks for whole tiles.
+    """The plan for the products of a block that no backward will follow (scoring, validation).  K is cut into two at most, from
+    4096 on and in two places: by ``split_k_choice`` (from 256 rows, tiles for at most half of the CTA pairs), and in the last
+    round of an output of at least 512 rows whose tiles fill 60 % of the pairs' rounds.  Never among the clusters of
+    csrc/gemm_splitk.cu, nor in the last round of smaller outputs, which a third element 1 marks.
 
     So the order of summation is that of the products as they were before clusters shared K, but it is not the same at every
     token count: 3072 columns of depth 8192 take two slices at 256, 400 and 512 tokens and none at 300, 777 and 1024.  Another
@@ -223,8 +223,9 @@ def _launch(a, b, M, N, K, a_mn, b_mn, bias, out, accumulate, out_dtype, bn, pad
         kind, how = "one", (0,)
     if kind == "pair":
         n_store = min((N + 7) // 8 * 8, ldc) if pad_ok and how[0] == 1 else 0
-        # with one slice the workspace lets the launcher cut the tiles of a partly filled last wave of clusters into two
-        ws, n_ws, cnt, n_cnt = _workspace_args(a.device) if _TAIL_SPLIT or how[0] > 1 else (0, 0, 0, 0)
+        if not _TAIL_SPLIT:
+            lib.zen_gemm2_tail_split(0)
+        ws, n_ws, cnt, n_cnt = _workspace_args(a.device) if _TAIL_SPLIT or how[0] > 1 else (0, 0, 0, 0)       # where K slices meet
         rc = lib.zen_gemm_bf16_2cta_splitk(a2.data_ptr(), b2.data_ptr(), c, pbias, M, N, K, a2.stride(0), b2.stride(0), ldc, a_mn,
                                            b_mn, fp32, bool(accumulate), how[0], ws, n_ws, cnt, n_cnt, n_store, stream)
     elif kind == "cluster":
@@ -343,8 +344,9 @@ def flush_deferred() -> None:
         for i, (a2, b2, out, M, N, K, acc, _done) in enumerate(batch):
             descs[i] = _GemmDesc(a2.data_ptr(), b2.data_ptr(), out.data_ptr(), M, N, K, a2.stride(0), b2.stride(0),
                                  out.stride(0), int(out.dtype == torch.float32), int(acc))
-        dev = batch[0][0].device
-        ws, n_ws, cnt, n_cnt = _workspace_args(dev) if _TAIL_SPLIT else (0, 0, 0, 0)
+        if not _TAIL_SPLIT:
+            lib.zen_gemm2_tail_split(0)
+        ws, n_ws, cnt, n_cnt = _workspace_args(batch[0][0].device) if _TAIL_SPLIT else (0, 0, 0, 0)
         rc = lib.zen_gemm_bf16_2cta_group(descs, n, 1, 1, ws, n_ws, cnt, n_cnt, _native.stream_ptr())
         _native.check(rc, "zen_gemm_bf16_2cta_group")
         for item in batch:
