@@ -7,11 +7,13 @@
 // (train.py:149-157); nothing of them is in its tree.
 #include "act_common.cuh"
 #include "launch.cuh"
+#include "xent_common.cuh"
 #include "zen_common.cuh"
 
 namespace {
 
 using namespace zen_act;
+using namespace zen_xe;
 
 template <typename T> struct Vec8;   // 8 elements of T <-> 8 floats
 template <> struct Vec8<__nv_bfloat16> {
@@ -970,12 +972,6 @@ rows_add_kernel(T* __restrict__ grad, const int32_t* rows, const int32_t* count,
 // four loads in flight per thread, one rescaling of the running sum per 16 elements, no label test per element.
 constexpr int XENT_U = 2;
 
-__device__ __forceinline__ float ex2_fast(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // Eight elements as loaded; unpacked only where they are used (the loads in flight then take half the registers).
 template <typename T> struct Raw8v {
   uint4 q[sizeof(T) / 2];
@@ -990,34 +986,6 @@ template <typename T> struct Raw8v {
   }
 };
 
-// cap tanh(x / cap); *slope: its derivative 1 - tanh^2.  tanh.approx (relative error 2^-11) is no choice, whatever the type of the
-// logits: the slope cancels near the cap (tanh 0.999: half of it would be noise), and fp32 logits have 13 more bits than it gives.
-//  * fp32 logits: tanhf of the quotient, as in softcap_kernel: the loss is the loss of the logits that the model returns.
-//  * 16-bit logits: from e = exp(-2 |x| / cap), tanh = (1 - e) / (1 + e) and slope = 4 e / (1 + e)^2, without cancellation at the
-//    cap and within 3e-7 of tanh everywhere (2048 x 256 000 bf16 logits, both passes: 797 us; with tanhf 1 353, uncapped 503).
-template <typename T>
-__device__ __forceinline__ float xent_cap_value(float x, float cap, float k, float* slope) {
-  if constexpr (sizeof(T) == 4) {
-    const float t = tanhf(x / cap);
-    *slope = 1.f - t * t;
-    return cap * t;
-  } else {
-    const float e = ex2_fast(-fabsf(x) * k);
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-    *slope = 4.f * e * (r * r);
-    return copysignf(cap * ((1.f - e) * r), x);
-  }
-}
-template <typename T, bool CAP>
-__device__ __forceinline__ float xent_cap(float x, float cap, float k, float* slope = nullptr) {
-  if (!CAP) return x;
-  float d;
-  const float y = xent_cap_value<T>(x, cap, k, &d);
-  if (slope) *slope = d;
-  return y;
-}
-
 template <typename T, bool CAP, int XENT_THREADS>
 __global__ void __launch_bounds__(XENT_THREADS, XENT_THREADS == 512 ? 2 : 1)
 xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
@@ -1025,7 +993,6 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
             int64_t ignore_index, float cap) {
   zen_pdl::enter();
   __shared__ float sh[32];
-  constexpr float L2E = 1.4426950408889634f;
   const float gscale = gscale_dev ? gscale_host * (*gscale_dev) : gscale_host;
   const float k2 = CAP ? 2.f * L2E / cap : 0.f;
   const bool vec_ok = ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) % 16 == 0;
@@ -1117,6 +1084,104 @@ xent_kernel(const T* logits, const int64_t* labels, float* __restrict__ loss,
         dp[label] = ZenVal<T>::from_f(CAP ? g * slope_label : g);
       }
     }
+  }
+}
+
+// --------------------------------------------------------------------------------------------
+// Cross-entropy whose row statistics come out of the product that makes the logits (zen_gemm_bf16_2cta_loss):
+//   xent_finish_kernel : lse and loss of each row from the (maximum, sum of exponentials) of its 128-column pieces
+//   xent_grad_kernel   : dlogits = (exp(y - lse) - onehot) * gscale in place, one pass
+// xent_kernel makes the same out of the logits alone, but reads them twice and has two exponentials an element to do (three
+// times two special functions when soft-capped) between which nothing overlaps within a row.  us, xent_kernel / finish + grad:
+// 8192 x 50 257 397 / 11 + 296, 4096 x 128 256 539 / 23 + 360, 8192 x 256 000 2 210 / 47 + 1 493, 2048 x 256 000 soft-capped 972 / 39 + 558
+// (memory alone, read and write once: 251, 320, 1 280, 320).  Without a gradient the logits are not even written: 215 / 11.
+constexpr int XF_ROWS = 16, XF_G = 32;                  // rows of a CTA (128 bytes of a piece) and pieces side by side
+template <bool CAP>
+__global__ void __launch_bounds__(XF_ROWS * XF_G)
+xent_finish_kernel(const float2* part, int nparts, int part_ld, const float* target, const int64_t* labels, float* loss, float* lse_out,
+                   int rows, int vocab, int64_t ignore_index, float cap) {
+  zen_pdl::enter();
+  __shared__ float2 sh[XF_G][XF_ROWS];
+  const int r = threadIdx.x % XF_ROWS, g = threadIdx.x / XF_ROWS, row = blockIdx.x * XF_ROWS + r;
+  float m = -INFINITY, s = 0.f;
+  if (row < rows) {
+    for (int p0 = g; p0 < nparts; p0 += XF_G * 8) {
+      float2 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = p0 + u * XF_G < nparts ? part[(size_t)(p0 + u * XF_G) * part_ld + row] : make_float2(-INFINITY, 0.f);
+      float nm = m;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) nm = fmaxf(nm, x[u].x);
+      const float ref = nm == -INFINITY ? 0.f : nm;
+      s *= __expf(m - ref);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += x[u].y * __expf(x[u].x - ref);
+      m = nm;
+    }
+  }
+  sh[g][r] = make_float2(m, s);
+  __syncthreads();
+  if (g == 0 && row < rows) {
+#pragma unroll
+    for (int k = 0; k < XF_G; ++k) m = fmaxf(m, sh[k][r].x);
+    const float ref = m == -INFINITY ? 0.f : m;
+    s = 0.f;
+#pragma unroll
+    for (int k = 0; k < XF_G; ++k) s += sh[k][r].y * __expf(sh[k][r].x - ref);
+    const float lse = m + logf(s);
+    const int64_t label = labels[row];
+    const bool valid = label != ignore_index && label >= 0 && label < vocab;
+    lse_out[row] = lse;
+    loss[row] = valid ? lse - xent_cap<__nv_bfloat16, CAP>(target[row], cap, CAP ? 2.f * L2E / cap : 0.f) : 0.f;
+  }
+}
+
+constexpr int XG_U = 4;                                 // vectors of eight in flight per thread
+template <bool CAP>
+__global__ void __launch_bounds__(256)
+xent_grad_kernel(__nv_bfloat16* logits, const int64_t* labels, const float* lse_in, int rows, int vocab, int ld, float gscale_host,
+                 const float* gscale_dev, int64_t ignore_index, float cap) {
+  typedef __nv_bfloat16 T;
+  zen_pdl::enter();
+  const float gscale = gscale_dev ? gscale_host * (*gscale_dev) : gscale_host;
+  const float k2 = CAP ? 2.f * L2E / cap : 0.f;
+  const int nv = vocab / 8;                             // ld % 8 == 0 and the base on 16 bytes: checked by the launcher
+  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    T* lp = logits + (size_t)row * ld;
+    const int64_t label = labels[row];
+    const bool valid = label != ignore_index && label >= 0 && label < vocab;
+    const float lse = lse_in[row], sc = valid ? gscale : 0.f;
+    const int at = valid ? (int)label : -1;
+    auto grad = [&](float x, bool hit) -> float {
+      float slope = 1.f;
+      const float p = ex2_fast((xent_cap<T, CAP>(x, cap, k2, &slope) - lse) * L2E);
+      const float g = (hit ? p - 1.f : p) * sc;
+      return CAP ? g * slope : g;
+    };
+    for (int v0 = threadIdx.x; v0 < nv; v0 += 256 * XG_U) {
+      Raw8v<T> x[XG_U];
+#pragma unroll
+      for (int u = 0; u < XG_U; ++u)
+        if (v0 + u * 256 < nv) x[u].load(lp + (size_t)(v0 + u * 256) * 8);
+#pragma unroll
+      for (int u = 0; u < XG_U; ++u) {
+        const int v = v0 + u * 256;
+        if (v >= nv) continue;
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = grad(x[u].at(i), false);
+        if ((at >> 3) == v && at >= 0) {
+          float slope = 1.f;
+          const float y = xent_cap<T, CAP>(ZenVal<T>::to_f(lp[at]), cap, k2, &slope);
+          const float g = (ex2_fast((y - lse) * L2E) - 1.f) * sc;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if ((at & 7) == i) o[i] = CAP ? g * slope : g;
+        }
+        Vec8<T>::store(lp + (size_t)v * 8, o);
+      }
+    }
+    for (int c = nv * 8 + threadIdx.x; c < vocab; c += 256) lp[c] = ZenVal<T>::from_f(grad(ZenVal<T>::to_f(lp[c]), c == at));
   }
 }
 
@@ -1588,6 +1653,26 @@ int zen_xent(const void* logits, const int64_t* labels, float* loss, void* dlogi
     else { if (two) XENT(false, 512); else XENT(false, 1024); }
   });
 #undef XENT
+  return (int)cudaGetLastError();
+}
+
+// Loss and log-sum-exp of rows from their 128-column pieces; part: [nparts][part_ld] (maximum, sum of exponentials).
+int zen_xent_finish(const void* part, int nparts, int part_ld, const float* target, const int64_t* labels, float* loss, float* lse, int rows,
+                    int vocab, int64_t ignore_index, float softcap, void* stream) {
+  const int grid = (rows + XF_ROWS - 1) / XF_ROWS;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (softcap > 0.f) zen_pdl::launch_small(xent_finish_kernel<true>, grid, XF_ROWS * XF_G, 0, st, (const float2*)part, nparts, part_ld, target, labels, loss, lse, rows, vocab, ignore_index, softcap);
+  else zen_pdl::launch_small(xent_finish_kernel<false>, grid, XF_ROWS * XF_G, 0, st, (const float2*)part, nparts, part_ld, target, labels, loss, lse, rows, vocab, ignore_index, softcap);
+  return (int)cudaGetLastError();
+}
+// In place: bf16 logits <- (softmax - onehot) * gscale (* *gscale_dev), from each row's log-sum-exp.
+int zen_xent_grad(void* logits, const int64_t* labels, const float* lse, int rows, int vocab, int ld, float gscale, const float* gscale_dev,
+                  int64_t ignore_index, float softcap, void* stream) {
+  if (ld % 8 || reinterpret_cast<uintptr_t>(logits) % 16) return -2;
+  const int grid = cap_grid((size_t)rows, 8);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (softcap > 0.f) zen_pdl::launch_small(xent_grad_kernel<true>, grid, 256, 0, st, (__nv_bfloat16*)logits, labels, lse, rows, vocab, ld, gscale, gscale_dev, ignore_index, softcap);
+  else zen_pdl::launch_small(xent_grad_kernel<false>, grid, 256, 0, st, (__nv_bfloat16*)logits, labels, lse, rows, vocab, ld, gscale, gscale_dev, ignore_index, softcap);
   return (int)cudaGetLastError();
 }
 

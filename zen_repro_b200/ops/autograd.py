@@ -324,16 +324,23 @@ class LMHeadLossFn(torch.autograd.Function):
         in_kernel = h2.is_cuda                       # the cross-entropy kernel soft-caps by itself
         for s in range(0, T, chunk_tokens):
             e = min(T, s + chunk_tokens)
-            buf = torch.empty(e - s, vpad, dtype=h2.dtype, device=h2.device)
-            logits = buf[:, :V]
-            G.gemm_nt(h2[s:e], weight, out=logits, pad_ok=True)
-            th = None if in_kernel else _softcap_(logits, softcap)
-            loss, dl = E.cross_entropy(logits, lab[s:e], grad_scale=1.0 if train else None, grad_scale_dev=inv, ignore_index=ignore_index,
-                                       softcap=softcap if in_kernel else 0.0, loss_out=losses[s:e] if in_kernel else None)
-            if not in_kernel:
-                losses[s:e] = loss
-                if train:
-                    _softcap_grad_(dl, th)
+            hs, ls = h2[s:e], lab[s:e]
+            fused = in_kernel and G.makes_loss_statistics(hs, weight)
+            logits = torch.empty(e - s, vpad, dtype=h2.dtype, device=h2.device)[:, :V] if train or not fused else None
+            if fused:
+                ls = E._index(ls, hs)
+                part, target = G.gemm_nt_loss(hs, weight, ls, out=logits, softcap=softcap)
+                lse = E.xent_finish(part, target, ls, V, losses[s:e], ignore_index, softcap)
+                dl = E.xent_grad_(logits, ls, lse, inv, ignore_index=ignore_index, softcap=softcap) if train else None
+            else:
+                G.gemm_nt(hs, weight, out=logits, pad_ok=True)
+                th = None if in_kernel else _softcap_(logits, softcap)
+                loss, dl = E.cross_entropy(logits, ls, grad_scale=1.0 if train else None, grad_scale_dev=inv, ignore_index=ignore_index,
+                                           softcap=softcap if in_kernel else 0.0, loss_out=losses[s:e] if in_kernel else None)
+                if not in_kernel:
+                    losses[s:e] = loss
+                    if train:
+                        _softcap_grad_(dl, th)
             if want_h:
                 G.gemm_nn(dl, weight, out=dh[s:e])
             if want_w:

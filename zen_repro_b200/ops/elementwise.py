@@ -521,6 +521,29 @@ def cross_entropy(logits, labels, *, grad_scale: float | None = None, ignore_ind
     return loss, d
 
 
+def xent_finish(part, target, labels, vocab: int, loss_out, ignore_index: int = -100, softcap: float = 0.0):
+    """Losses (into ``loss_out``) and log-sum-exps of the rows from what :func:`gemm.gemm_nt_loss` left (CUDA)."""
+    rows = target.shape[0]
+    lb = _index(labels, target)
+    if lb.numel() != rows:
+        raise ValueError(f"{lb.numel()} labels for {rows} rows of logits")
+    lse = torch.empty_like(target)
+    _native.check(_native.lib().zen_xent_finish(part.data_ptr(), part.shape[0], part.shape[1], target.data_ptr(), lb.data_ptr(), loss_out.data_ptr(),
+                                                lse.data_ptr(), rows, vocab, int(ignore_index), float(softcap), _native.stream_ptr()),
+                  "zen_xent_finish")
+    return lse
+
+
+def xent_grad_(logits, labels, lse, grad_scale_dev=None, grad_scale: float = 1.0, ignore_index: int = -100, softcap: float = 0.0):
+    """In place: bf16 logits <- (softmax - onehot) * scale from each row's log-sum-exp (CUDA), back through the soft-capping."""
+    rows, vocab = logits.shape
+    lb = _index(labels, logits)
+    _native.check(_native.lib().zen_xent_grad(logits.data_ptr(), lb.data_ptr(), lse.data_ptr(), rows, vocab, logits.stride(0), float(grad_scale),
+                                              _native.ptr(grad_scale_dev), int(ignore_index), float(softcap), _native.stream_ptr()),
+                  "zen_xent_grad")
+    return logits
+
+
 # ----------------------------------------------------------------------------- vocabulary-parallel cross entropy
 def xent_partial(logits, labels, valid_cols: int, vocab_start: int, ignore_index: int = -100):
     """Per-row (max, sum-exp, target logit) over this rank's vocabulary shard ``logits[:, :valid_cols]``."""

@@ -250,6 +250,29 @@ def gemm_nt(a, b, bias=None, out=None, accumulate=False, out_dtype=None, bn=0, p
     return _launch(a, b, M, N, K, False, False, bias, out, accumulate, out_dtype, bn, pad_ok)
 
 
+def makes_loss_statistics(a, b) -> bool:
+    """Whether :func:`gemm_nt_loss` runs for these operands: the CTA-pair kernel with whole K, on operands that need no copy."""
+    if not _use_kernel(a, b) or a.dim() != 2 or b.dim() != 2 or _rowmajor(a) is not a or _rowmajor(b) is not b:
+        return False
+    kind, slices = _plan(a.shape[0], b.shape[0], a.shape[1], 0)[:2]
+    return kind == "pair" and slices == 1
+
+
+def gemm_nt_loss(a, b, labels, out=None, softcap: float = 0.0):
+    """The logits a[M,K] @ b[N,K]^T as bf16 into ``out`` (the first N columns of a buffer whose rows are a multiple of 8 wide; None:
+    nowhere) and what a cross-entropy against ``labels`` (int64) needs of them: ``(part, target)`` for ``elementwise.xent_finish``.
+    Operands as :func:`makes_loss_statistics` asks."""
+    (M, K), N = a.shape, b.shape[0]
+    part = torch.empty(2 * ((N + 255) // 256), (M + 31) // 32 * 32, 2, dtype=torch.float32, device=a.device)
+    target = torch.empty(M, dtype=torch.float32, device=a.device)
+    c, ldc = (0, 0) if out is None else (out.data_ptr(), out.stride(0))
+    rc = _native.lib().zen_gemm_bf16_2cta_loss(a.data_ptr(), b.data_ptr(), c, M, N, K, a.stride(0), b.stride(0), ldc,
+                                               min((N + 7) // 8 * 8, ldc), labels.data_ptr(), part.data_ptr(), part.shape[1],
+                                               target.data_ptr(), float(softcap), _native.stream_ptr())
+    _native.check(rc, "zen_gemm_bf16_2cta_loss")
+    return part, target
+
+
 def gemm_nn(a, b, bias=None, out=None, accumulate=False, out_dtype=None, bn=0):
     """a[M,K] @ b[K,N] (+ bias[N])."""
     K = a.shape[-1]
