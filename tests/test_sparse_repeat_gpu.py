@@ -1,0 +1,26 @@
+"""Many calls of a size whose stages are reused soon after they were read: every one exact (a stage that is overwritten while a lane still
+reads it showed in one call of fifty)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def test_repeated_calls_stay_exact():
+    from zen_repro_b200.sparse.engine import VirtualSparseAllReduce
+
+    n, P = 3_000_017, 8
+    eng = VirtualSparseAllReduce(n, P, max_density=0.065, methods=(3,), deterministic=True)
+    gen = torch.Generator("cuda").manual_seed(1)
+    xs = [torch.where(torch.rand(n, device="cuda", generator=gen) < 0.05, torch.randn(n, device="cuda", generator=gen),
+                      torch.zeros((), device="cuda")).bfloat16() for _ in range(P)]
+    want = torch.zeros(n, device="cuda")
+    for x in xs:
+        want += x.float()
+    want = want.bfloat16()
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(400):
+        outs = eng(xs, method=3)
+        wrong += (outs[i % P] != want).any()
+    assert eng.status() == [0] * P
+    assert int(wrong) == 0

@@ -401,8 +401,6 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
             }
           }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&empty[s]);                     // this warp is done with the stage
       } else {
 #pragma unroll
         for (int u = 0; u < VPL; ++u) {
@@ -411,12 +409,25 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
         }
       }
       const bool last_it = (it + gridDim.x >= nst);
+      bool hit[VPL];
+      uint32_t bals[VPL];
 #pragma unroll
       for (int u = 0; u < VPL; ++u) {
-        const bool has = plain ? v[u].any() : v[u].hit(tbits, t16);    // most vectors of a bucket stop here
-        const uint32_t bal = __ballot_sync(0xffffffffu, has);
+        hit[u] = plain ? v[u].any() : v[u].hit(tbits, t16);            // most vectors of a bucket stop here
+        bals[u] = __ballot_sync(0xffffffffu, hit[u]);
+      }
+      if (kRing) {
+        // This warp is done with the stage.  Not before the ballots, which need every word that was read: a load that has only
+        // been issued may still be queued when the arrival (of another unit) lets the next copy into the stage, and then returns
+        // the wrong stage's data (seen in one call of fifty at 8 x 3 M bf16: sixteen bytes of a lane's second vector).
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[s]);
+      }
+#pragma unroll
+      for (int u = 0; u < VPL; ++u) {
+        const uint32_t bal = bals[u];
         if (!bal) continue;
-        if (has) {
+        if (hit[u]) {
           const uint32_t idx = (wtail + __popc(bal & lt_mask)) & (K1_LIST - 1u);
           wel[warp][idx] = ebase + (uint32_t)u * (K1_CONSUMERS * VE);
           uint4* p4 = reinterpret_cast<uint4*>(&wdat[warp][idx]);
