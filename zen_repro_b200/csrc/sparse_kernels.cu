@@ -6,12 +6,12 @@
 //                         owners, stage (slot, value) records per owner in shared memory and push
 //                         them in large contiguous runs straight into the owner's receive region
 //                         over NVLink (P2P stores).
-//   zen_owner_reduce    : bounded wait on every source's mailbox at once, red.add the records
-//                         into this owner's fp32 slots, red.or the occupancy bitmap.
-//   zen_gather_push     : walk the occupancy bitmap, compact the touched slots chunk by chunk,
-//                         reserve room in the payload with one atomic per CTA step and push
-//                         bitmap|COO + values to every peer (P2P stores, or one multimem store
-//                         through the NVSwitch when a multicast alias of the region exists).
+//   zen_owner_reduce    : bounded wait on every source's mailbox at once; with many records, sort them by bucket of the
+//                         owner's slots (K2b).
+//   zen_gather_push     : add up a bucket's records in shared memory, compact the touched slots chunk by chunk, reserve
+//                         room in the payload with one atomic per bucket and push bitmap|COO + values to every peer
+//                         (P2P stores, or one multimem store through the NVSwitch when a multicast alias of the region
+//                         exists).  (K3b; owners of more than 2^25 slots keep sums and bitmap in global memory, K2 + K3.)
 //   zen_densify         : bounded wait on each owner's mailbox, one pass over the output that
 //                         writes zeros and values together.
 //
@@ -48,8 +48,8 @@ struct ZenSparseCtx {
   uint32_t nchunks;
   float* acc;               // [S] local
   uint32_t* bitmap;         // [nwords] local
-  uint32_t* chunk_off;      // unused by the kernels (kept for layout stability of the binding)
-  uint32_t* cursors;        // [P] record cursors, [MAX] done counter K1, [MAX+1] done counter K3, [MAX+2] payload cursor
+  uint32_t* seg;            // [buckets][P * tiles] runs of a bucket in the sorted record tiles (K2b)
+  uint32_t* cursors;        // [P] record cursors, [MAX] done counter K1, [MAX+1] done counter K3, [MAX+2] payload cursor, [MAX+3] what K2 / K2b tells the gather
   uint32_t* status;         // status word
   uint64_t numel;           // N
   uint32_t nslots;          // S = sb * G
@@ -93,6 +93,19 @@ template <int NB>
 __device__ __forceinline__ void arrive_fence() {
   if constexpr (NB > 1) __threadfence();
   else __threadfence_system();
+}
+// The last CTA's side of it: what the others arrived with is visible after the fence; `epoch` goes to the mail last.  All ranks on one
+// device: the consumer is a later kernel of the stream, so the stores need no release and the fence no system scope (each costs
+// the last CTA, and with it a small call, one to three microseconds: 50 000 elements on two ranks 27.1 -> 20.3 us).
+template <int NB>
+__device__ __forceinline__ void publish_fence() {
+  if constexpr (NB > 1) __threadfence();
+  else __threadfence_system();
+}
+template <int NB>
+__device__ __forceinline__ void publish_epoch(uint32_t* p, uint32_t v) {
+  if constexpr (NB > 1) *reinterpret_cast<volatile uint32_t*>(p) = v;
+  else zen_st_release_sys(p, v);
 }
 
 __device__ __forceinline__ uint32_t zen_epoch(const ZenSparseCtx& c) { return c.epoch_dev ? *c.epoch_dev : c.epoch; }
@@ -468,7 +481,7 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
   }
   __syncthreads();
   if (s_last) {
-    __threadfence_system();
+    publish_fence<NB>();
     if (tid < c.nranks) {
       const int p = tid;
       const uint32_t raw = atomicAdd(&c.cursors[kBroadcast ? 0 : p], 0u);
@@ -477,7 +490,7 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
       mail->count = min(raw, c.cap_rec);
       mail->info = ((raw > c.cap_rec) || (st & ZEN_REC_OVERFLOW)) ? 1u : 0u;
       mail->aux = 0;
-      zen_st_release_sys(&mail->epoch, epoch);
+      publish_epoch<NB>(&mail->epoch, epoch);
     }
     __syncthreads();
     if (tid < ZEN_MAX_RANKS + 1) c.cursors[tid] = 0;                  // ready for the next call
@@ -588,6 +601,34 @@ __device__ __forceinline__ void zen_multimem_st16(void* mc_addr, const uint4& v)
 }
 __device__ __forceinline__ void zen_multimem_st4(void* mc_addr, uint32_t v) {
   asm volatile("multimem.st.relaxed.sys.global.b32 [%0], %1;" ::"l"(mc_addr), "r"(v) : "memory");
+}
+
+// End of a gather: the last CTA of a rank publishes its payload to the consumers.
+template <int NB>
+__device__ __forceinline__ void publish_gather(const ZenSparseCtx& c, uint32_t fmt, uint32_t epoch, uint32_t& s_last) {
+  const int tid = threadIdx.x;
+  __syncthreads();
+  if (tid == 0) {
+    arrive_fence<NB>();
+    const uint32_t prev = atomicAdd(&c.cursors[ZEN_MAX_RANKS + 1], 1u);
+    s_last = (prev == gridDim.x - 1) ? 1u : 0u;
+  }
+  __syncthreads();
+  if (s_last) {
+    publish_fence<NB>();
+    if (tid < c.nranks) {
+      const uint32_t total = atomicAdd(&c.cursors[ZEN_MAX_RANKS + 2], 0u);
+      const uint32_t st = atomicOr(c.status, 0u);
+      const bool overflow = total > c.cap_g || (st & ZEN_GATHER_OVERFLOW);
+      ZenMail* mail = reinterpret_cast<ZenMail*>(c.sym[tid] + c.off_g_mail) + c.rank;
+      mail->count = overflow ? 0u : total;
+      mail->info = ((overflow || (st & (ZEN_REC_OVERFLOW | ZEN_PEER_OVERFLOW | ZEN_TIMEOUT))) ? 1u : 0u) | (fmt << 8);
+      mail->aux = 0;
+      publish_epoch<NB>(&mail->epoch, epoch);
+    }
+    __syncthreads();
+    if (tid == 0) { c.cursors[ZEN_MAX_RANKS + 1] = 0; c.cursors[ZEN_MAX_RANKS + 2] = 0; }
+  }
 }
 
 template <typename T, int NB>
@@ -820,28 +861,375 @@ zen_gather_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int ppw) {
   }
 
   if (local_status) atomicOr(c.status, local_status);
-  __syncthreads();
-  if (tid == 0) {
-    arrive_fence<NB>();
-    const uint32_t prev = atomicAdd(&c.cursors[ZEN_MAX_RANKS + 1], 1u);
-    s_last = (prev == gridDim.x - 1) ? 1u : 0u;
-  }
-  __syncthreads();
-  if (s_last) {
-    __threadfence_system();
-    if (tid < c.nranks) {
-      const uint32_t total = atomicAdd(&c.cursors[ZEN_MAX_RANKS + 2], 0u);
-      const uint32_t st = atomicOr(c.status, 0u);
-      const bool overflow = total > c.cap_g || (st & ZEN_GATHER_OVERFLOW);
-      ZenMail* mail = reinterpret_cast<ZenMail*>(c.sym[tid] + c.off_g_mail) + c.rank;
-      mail->count = overflow ? 0u : total;
-      mail->info = ((overflow || (st & (ZEN_REC_OVERFLOW | ZEN_PEER_OVERFLOW | ZEN_TIMEOUT))) ? 1u : 0u) | (fmt << 8);
-      mail->aux = 0;
-      zen_st_release_sys(&mail->epoch, epoch);
+  publish_gather<NB>(c, fmt, epoch, s_last);
+}
+
+// ---------------------------------------------------------------------------------------------
+// K2b + K3b: the owner's sums in shared memory.  The slot space of an owner is cut into buckets of 16 384 slots (32 768 from
+// 2^24 slots on); one CTA adds up all records of a bucket in shared memory and gathers and pushes from there, so neither sums nor
+// occupancy bitmap exist in global memory.  For that the records of a bucket have to be found:
+//   * few records: every CTA reads all of its owner's records and keeps its bucket's (no kernel before K3b at all);
+//   * else K2b sorts them by bucket first, tile by tile (4096 records of one source) and in place, and notes where the
+//     bucket's run of each tile begins and ends: seg[bucket][tile].
+//
+// What bounds K2 + K3, which this replaces: the scattered atomics of K2, two a record, 38 per clock over the whole GPU however
+// they are arranged, and in K3 the round trips from bitmap to slots to push.  Here a record costs one more trip through L2
+// (K2b) and one shared-memory atomic; what is left is the chain of a bucket (words, records, adds, count, reservation, push), about
+// 10 us with 24 warps to an SM, of which the stores to eight peers are a quarter.  us, K2 + K3 / K2b + K3b: 8 ranks of 2^26 bf16
+// elements at 1 % 170 + 121 / 34 + 100, 4 of 13 M 20 + 20 / 7 + 19, 2 of 50 000 (fp32) 4 + 11 / 0 + 8.
+// (Tried: one CTA per bucket, not persistent, 120 us for the first; the next bucket's runs fetched ahead 195, in spills and waits.)
+// K2 and K3 remain for owners of more than 2^25 slots, whose tiles would leave less than four records to a run.
+#define SB_TILE 4096
+#define SB_MAX_BUCKETS 1024
+#define SB_SORT_THREADS 512
+#define SB_WINDOW 512                                     // list entries per warp
+#define SB_FILTER_RECORDS 65536                           // most record slots of an owner that every CTA reads for itself
+
+struct SbShape { uint32_t lg, nbuckets, tiles, lg_lanes; bool on, sorted; };      // tiles: per source; lanes to a run
+__host__ __device__ __forceinline__ SbShape sb_shape(uint32_t nslots, uint32_t cap_rec, int nranks) {
+  SbShape s;
+  s.lg = nslots <= (SB_MAX_BUCKETS << 14) ? 14u : 15u;
+  s.nbuckets = (nslots + (1u << s.lg) - 1) >> s.lg;
+  s.tiles = (cap_rec + SB_TILE - 1) / SB_TILE;
+  s.lg_lanes = s.nbuckets > 384 ? 3u : s.nbuckets > 160 ? 4u : 5u;      // a full tile's runs: 4096 / buckets records
+  s.on = s.nbuckets <= SB_MAX_BUCKETS;
+  s.sorted = s.nbuckets > 1 && (uint64_t)cap_rec * nranks > SB_FILTER_RECORDS;
+  return s;
+}
+
+// Records received from each source, after a bounded wait for its mail; one thread per source.
+__device__ __forceinline__ void sb_wait(const ZenSparseCtx& c, uint32_t epoch, uint32_t* s_n, uint32_t* s_flag) {
+  if ((int)threadIdx.x < c.nranks) {
+    const ZenMail* mail = zen_rec_mail(c, c.rank, threadIdx.x, epoch);
+    uint32_t n = 0, fl = 0;
+    if (zen_wait_epoch(&mail->epoch, epoch, c.wait_ns)) {
+      // count and info were written before the epoch's release store: plain loads after the acquire above see them
+      n = min(*reinterpret_cast<const volatile uint32_t*>(&mail->count), c.cap_rec);
+      if (*reinterpret_cast<const volatile uint32_t*>(&mail->info) & 1u) fl = ZEN_PEER_OVERFLOW;
+    } else {
+      fl = ZEN_TIMEOUT;
     }
-    __syncthreads();
-    if (tid == 0) { c.cursors[ZEN_MAX_RANKS + 1] = 0; c.cursors[ZEN_MAX_RANKS + 2] = 0; }
+    s_n[threadIdx.x] = n;
+    s_flag[threadIdx.x] = fl;
   }
+  __syncthreads();
+}
+
+template <int NB>
+__global__ void __launch_bounds__(SB_SORT_THREADS, 2)
+zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int deterministic) {
+  zen_pdl::enter();
+  __shared__ ZenSparseCtx s_ctx;
+  const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS];
+  __shared__ uint32_t hist[SB_MAX_BUCKETS + 1], s_warp[SB_SORT_THREADS / 32];
+  __shared__ __align__(16) uint2 sorted[SB_TILE];
+  const uint32_t epoch = zen_epoch(c);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  sb_wait(c, epoch, s_n, s_flag);
+  uint32_t local_status = 0;
+  if (blockIdx.x == 0 && tid == 0) {
+    c.cursors[ZEN_MAX_RANKS + 3] = deterministic ? 2u : 0u;              // for a K3b that is launched without being told
+    for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
+  }
+  const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
+  if (sh.on && sh.sorted) {
+    const uint32_t nb = sh.nbuckets, stride = sh.tiles * c.nranks;
+    uint32_t* seg = c.seg;
+    for (uint32_t t = blockIdx.x; t < stride; t += gridDim.x) {
+      const uint32_t src = t / sh.tiles, first = (t - src * sh.tiles) * SB_TILE;
+      if (first >= s_n[src]) continue;
+      const uint32_t n = min((uint32_t)SB_TILE, s_n[src] - first);
+      uint2* rec = zen_rec_slots(c, c.rank, src, epoch) + first;
+      for (uint32_t b = tid; b <= nb; b += SB_SORT_THREADS) hist[b] = 0;
+      constexpr int PAIRS = SB_TILE / 2 / SB_SORT_THREADS;
+      uint4 r[PAIRS];
+#pragma unroll
+      for (int u = 0; u < PAIRS; ++u) {
+        const uint32_t i = (uint32_t)(u * SB_SORT_THREADS + tid) * 2;
+        r[u] = i + 1 < n ? reinterpret_cast<const uint4*>(rec)[i / 2] : make_uint4(0xffffffffu, 0u, 0xffffffffu, 0u);
+        if (i + 1 == n) { const uint2 x = rec[i]; r[u].x = x.x; r[u].y = x.y; }
+      }
+      __syncthreads();
+      // a slot that does not exist goes to the bucket after the last, which nobody reads
+      uint32_t at[2 * PAIRS];
+      auto bucket = [&](uint32_t slot) { return slot < c.nslots ? slot >> sh.lg : nb; };
+#pragma unroll
+      for (int u = 0; u < PAIRS; ++u) {
+        const uint32_t i = (uint32_t)(u * SB_SORT_THREADS + tid) * 2;
+        if (i < n) { at[2 * u] = atomicAdd(&hist[bucket(r[u].x)], 1u); if (r[u].x >= c.nslots) local_status |= ZEN_BAD_ARG; }
+        if (i + 1 < n) { at[2 * u + 1] = atomicAdd(&hist[bucket(r[u].z)], 1u); if (r[u].z >= c.nslots) local_status |= ZEN_BAD_ARG; }
+      }
+      __syncthreads();
+      // exclusive prefix sums over the buckets, two per thread
+      const uint32_t b0 = tid * 2, h0 = b0 < nb ? hist[b0] : 0u, h1 = b0 + 1 < nb ? hist[b0 + 1] : 0u;
+      uint32_t incl = h0 + h1;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += x;
+      }
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      uint32_t before = 0;
+#pragma unroll
+      for (int k = 0; k < SB_SORT_THREADS / 32; ++k) before += k < warp ? s_warp[k] : 0u;
+      const uint32_t e0 = before + incl - h0 - h1, e1 = e0 + h0;
+      if (b0 < nb) { hist[b0] = e0; seg[(size_t)b0 * stride + t] = e0 | h0 << 16; }
+      if (b0 + 1 < nb) { hist[b0 + 1] = e1; seg[(size_t)(b0 + 1) * stride + t] = e1 | h1 << 16; }
+      if (tid == SB_SORT_THREADS - 1) hist[nb] = e1 + h1;
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < PAIRS; ++u) {
+        const uint32_t i = (uint32_t)(u * SB_SORT_THREADS + tid) * 2;
+        if (i < n) sorted[hist[bucket(r[u].x)] + at[2 * u]] = make_uint2(r[u].x, r[u].y);
+        if (i + 1 < n) sorted[hist[bucket(r[u].z)] + at[2 * u + 1]] = make_uint2(r[u].z, r[u].w);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < PAIRS; ++u) {
+        const uint32_t i = (uint32_t)(u * SB_SORT_THREADS + tid) * 2;
+        if (i + 1 < n) reinterpret_cast<uint4*>(rec)[i / 2] = *reinterpret_cast<const uint4*>(&sorted[i]);
+        else if (i < n) rec[i] = sorted[i];
+      }
+      __syncthreads();                                     // hist and the tile are free
+    }
+  }
+  if (local_status) atomicOr(c.status, local_status);
+}
+
+template <int W> constexpr size_t sb_smem() { return (size_t)W * (2048 * 4 + 256 + SB_WINDOW * 2); }
+
+// det: 1 rank order, 0 any order, -1 as K2b left it
+template <typename T, int W, int NB>
+__global__ void __launch_bounds__(W * 32, W == 8 ? 3 : 1)
+zen_reduce_gather_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int det) {
+  zen_pdl::enter();
+  __shared__ ZenSparseCtx s_ctx;
+  const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  constexpr uint32_t BS = W * 2048;
+  float* acc = reinterpret_cast<float*>(smem_raw);                       // [BS]
+  uint32_t* bm = reinterpret_cast<uint32_t*>(acc + BS);                  // [BS / 32]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hl = lane & 15, hf = lane >> 4;
+  unsigned short* list = reinterpret_cast<unsigned short*>(bm + BS / 32) + warp * SB_WINDOW;    // pair-local slots
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS], s_last, s_fmt, s_base, s_tot[W];
+  const uint32_t epoch = zen_epoch(c);
+  const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
+  for (uint32_t i = tid; i < (BS + BS / 32) / 4; i += W * 32) reinterpret_cast<uint4*>(smem_raw)[i] = make_uint4(0u, 0u, 0u, 0u);
+  sb_wait(c, epoch, s_n, s_flag);
+  uint32_t local_status = 0;
+  uint64_t recs = 0;
+  for (int k = 0; k < c.nranks; ++k) recs += s_n[k];
+  // With many records the occupancy bitmap is not kept while they are added up: "touched" then means "sum is not zero" (a slot
+  // whose sum is exactly zero need not travel).
+  const bool dense_mode = recs * K2_DENSE > (uint64_t)c.nslots;
+  if (tid == 0) {
+    if (blockIdx.x == 0)
+      for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
+    // index format: bitmap when more than one slot in 32 is expected to be touched; the estimate is the number of records
+    // received (an upper bound of the union), which every CTA reads from the same mails
+    uint32_t fmt = c.fmt_mode;
+    if (fmt == 0) fmt = (recs * 32ull > (uint64_t)c.nslots) ? ZEN_FMT_BITMAP : ZEN_FMT_COO;
+    // a COO list (touched slots plus the padding between runs) must fit the index region
+    if (fmt == ZEN_FMT_COO && min(recs, (uint64_t)c.nslots) + K3_RUN_ALIGN * (uint64_t)c.nchunks > (uint64_t)c.g_idx_words) fmt = ZEN_FMT_BITMAP;
+    s_fmt = fmt;
+  }
+  const bool in_order = det < 0 ? c.cursors[ZEN_MAX_RANKS + 3] == 2u : det != 0;
+  __syncthreads();
+  auto apply = [&](uint32_t slot, uint32_t bits) {                       // a slot of this bucket
+    const uint32_t at = slot & (BS - 1);
+    atomicAdd(&acc[at], ZenVal<T>::unbits(bits));
+    if (!dense_mode) atomicOr(&bm[at >> 5], 1u << (at & 31));
+  };
+  const uint32_t fmt = s_fmt, nchunks = c.nchunks, nwords = c.nwords;
+  char* const mc = c.mc;
+  const int npeer = mc ? 1 : c.nranks;
+  constexpr uint32_t VPV = 16 / sizeof(T);                               // values per 16-byte vector
+  float* const pacc = acc + warp * 2048;                                 // gather: warp = one pair of chunks, lane = 64 of its slots
+  for (uint32_t bucket = blockIdx.x; bucket < sh.nbuckets; bucket += gridDim.x) {
+    for (int s_lo = 0; s_lo < c.nranks;) {
+      const int s_hi = in_order ? s_lo + 1 : c.nranks;
+      if (!sh.sorted) {
+        for (int s = s_lo; s < s_hi; ++s) {
+          const uint2* rec = zen_rec_slots(c, c.rank, s, epoch);
+          const uint32_t n = s_n[s], npair = (n + 1) >> 1;
+          for (uint32_t i = tid; i < npair; i += 4 * W * 32) {
+            uint4 r[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t j = i + u * W * 32;
+              r[u] = j < npair ? reinterpret_cast<const uint4*>(rec)[j] : make_uint4(0u, 0u, 0u, 0u);   // cap_rec is even
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t j = (i + u * W * 32) * 2;
+              if (j < n) {
+                if (r[u].x >= c.nslots) local_status |= ZEN_BAD_ARG;
+                else if ((r[u].x >> sh.lg) == bucket) apply(r[u].x, r[u].y);
+              }
+              if (j + 1 < n) {
+                if (r[u].z >= c.nslots) local_status |= ZEN_BAD_ARG;
+                else if ((r[u].z >> sh.lg) == bucket) apply(r[u].z, r[u].w);
+              }
+            }
+          }
+        }
+      } else {
+        // 8, 16 or 32 lanes to a run, at least half of what a full tile's runs hold; a group stays with one source and has U runs, two
+        // records of each per lane, under way together: words, then records, two trips to L2 for most buckets
+        constexpr int U = 6;
+        const uint32_t* seg = c.seg + (size_t)bucket * (sh.tiles * c.nranks);
+        const uint2* rec0 = zen_rec_slots(c, c.rank, 0, epoch);
+        const uint32_t lanes = 1u << sh.lg_lanes, l = lane & (lanes - 1u), group = tid >> sh.lg_lanes, ns = s_hi - s_lo;
+        const uint32_t per_src = ((W * 32u) >> sh.lg_lanes) / ns, k0 = group / ns, src = s_lo + group - k0 * ns;
+        const uint32_t rec_end = c.cap_rec * (uint32_t)c.nranks, ntiles = k0 < per_src ? (s_n[src] + SB_TILE - 1) / SB_TILE : 0u;
+        for (uint32_t k = k0; k < ntiles; k += U * per_src) {
+          uint32_t n[U], at[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t t = k + u * per_src;
+            n[u] = t < ntiles ? seg[src * sh.tiles + t] : 0u;
+            at[u] = src * c.cap_rec + t * SB_TILE;
+          }
+          uint2 x[U], y[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t first = n[u] & 0xffffu;
+            n[u] >>= 16;
+            at[u] += first;
+            // (K2b may have given up its wait for a source and left another call's runs: kept inside the tile and the region)
+            if (first + n[u] > SB_TILE || at[u] + n[u] > rec_end) n[u] = 0;
+            if (l < n[u]) x[u] = rec0[at[u] + l];
+            if (l + lanes < n[u]) y[u] = rec0[at[u] + l + lanes];
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (l < n[u]) apply(x[u].x, x[u].y);
+            if (l + lanes < n[u]) apply(y[u].x, y[u].y);
+            for (uint32_t i = l + 2 * lanes; i < n[u]; i += 4 * lanes) {   // long runs
+              uint2 z[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (i + q * lanes < n[u]) z[q] = rec0[at[u] + i + q * lanes];
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (i + q * lanes < n[u]) apply(z[q].x, z[q].y);
+            }
+          }
+        }
+      }
+      __syncthreads();                                                     // in order: the next source's adds come after these
+      s_lo = s_hi;
+    }
+
+    const uint32_t pair = bucket * W + warp;
+    uint2 word;
+    if (!dense_mode) {
+      uint2* at = reinterpret_cast<uint2*>(bm + warp * 64 + lane * 2);
+      word = *at;
+      *at = make_uint2(0u, 0u);
+    } else {
+      uint32_t w[2] = {0u, 0u};
+#pragma unroll 16
+      for (int i = 0; i < 64; ++i) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (__float_as_uint(pacc[i * 32 + lane]) & 0x7fffffffu) != 0u);
+        if (lane == (i >> 1)) w[i & 1] = m;
+      }
+      word = make_uint2(w[0], w[1]);
+    }
+    const uint32_t own = __popc(word.x) + __popc(word.y);
+    uint32_t incl = own;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d, 16);
+      if (hl >= d) incl += t;
+    }
+    const uint32_t n_mine = __shfl_sync(0xffffffffu, incl, 15, 16), n_pad = k3_pad(n_mine);
+    const uint32_t n0 = __shfl_sync(0xffffffffu, n_pad, 0), total = n0 + __shfl_sync(0xffffffffu, n_pad, 16);
+    const uint32_t run0 = hf ? n0 : 0u, first = run0 + incl - own;         // the half's first entry, and the lane's
+    if (lane == 0) s_tot[warp] = total;
+    __syncthreads();
+    uint32_t base = 0, cta_total = 0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) { const uint32_t x = s_tot[k]; base += k < warp ? x : 0u; cta_total += x; }
+    if (tid == 0) s_base = cta_total ? atomicAdd(&c.cursors[ZEN_MAX_RANKS + 2], cta_total) : 0u;
+    __syncthreads();
+    const uint32_t cta_base = s_base;
+    const bool fits = cta_base + cta_total <= c.cap_g && (fmt != ZEN_FMT_COO || cta_base + cta_total <= c.g_idx_words);
+    if (!fits) {
+      if (cta_total) local_status |= ZEN_GATHER_OVERFLOW;
+      for (int i = lane; i < 512; i += 32) reinterpret_cast<float4*>(pacc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    base += cta_base;
+    if (fits) {
+      for (uint32_t e0 = 0; e0 < total; e0 += SB_WINDOW) {                 // a window of the warp's entries at a time
+        const uint32_t n = min((uint32_t)SB_WINDOW, total - e0);
+        if (first < e0 + n && first + own > e0) {
+          uint32_t r = first - e0;                                         // wraps below the window: not stored
+          for (uint32_t w = word.x; w; w &= w - 1, ++r) if (r < n) list[r] = (unsigned short)(lane * 64 + __ffs(w) - 1);
+          for (uint32_t w = word.y; w; w &= w - 1, ++r) if (r < n) list[r] = (unsigned short)(lane * 64 + __ffs(w) + 31);
+        }
+        const uint32_t pad = run0 + n_mine + hl - e0;
+        if ((uint32_t)hl < n_pad - n_mine && pad < n) list[pad] = 0xffffu; // padding: skipped by the consumer
+        __syncwarp();
+        const uint64_t val_off = c.off_g_val + (uint64_t)c.rank * c.cap_g * 4ull + (uint64_t)(base + e0) * sizeof(T);
+        for (uint32_t i = lane; i < n / VPV; i += 32) {
+          uint32_t bits[VPV];
+#pragma unroll
+          for (int q = 0; q < (int)VPV; q += 4) {
+            const uint2 l4 = *reinterpret_cast<const uint2*>(list + i * VPV + q);
+            const uint32_t at[4] = {l4.x & 0xffffu, l4.x >> 16, l4.y & 0xffffu, l4.y >> 16};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              bits[q + k] = 0u;
+              if (at[k] == 0xffffu) continue;
+              bits[q + k] = ZenVal<T>::bits(ZenVal<T>::from_f(pacc[at[k]]));
+              pacc[at[k]] = 0.f;                                           // clean for the next bucket
+            }
+          }
+          uint4 v;
+          if constexpr (VPV == 4) v = make_uint4(bits[0], bits[1], bits[2], bits[3]);
+          else v = make_uint4(bits[0] | bits[1] << 16, bits[2] | bits[3] << 16, bits[VPV - 4] | bits[VPV - 3] << 16, bits[VPV - 2] | bits[VPV - 1] << 16);
+          if (mc) zen_multimem_st16(mc + val_off + (uint64_t)i * 16, v);   // one store, replicated by the switch
+          else
+            for (int p = 0; p < npeer; ++p) *reinterpret_cast<uint4*>(c.sym[p] + val_off + (uint64_t)i * 16) = v;
+        }
+        if (fmt == ZEN_FMT_COO) {
+          const uint64_t idx_off = c.off_g_idx + ((uint64_t)c.rank * c.g_idx_words + base + e0) * 4ull;
+          for (uint32_t i = lane; i < n / 4; i += 32) {
+            uint32_t sl[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { const uint32_t at = list[i * 4 + q]; sl[q] = at != 0xffffu ? pair * 2048 + at : 0xffffffffu; }
+            const uint4 v = make_uint4(sl[0], sl[1], sl[2], sl[3]);
+            if (mc) zen_multimem_st16(mc + idx_off + (uint64_t)i * 16, v);
+            else
+              for (int p = 0; p < npeer; ++p) *reinterpret_cast<uint4*>(c.sym[p] + idx_off + (uint64_t)i * 16) = v;
+          }
+        }
+        __syncwarp();                                                      // the list is free again
+      }
+      // bitmap words, and where each chunk's values begin
+      const uint32_t wi = pair * 64 + lane * 2, my_ch = pair * 2 + hf;
+      const uint32_t at = (fmt == ZEN_FMT_COO && n_mine == 0) ? K3_EMPTY : base + run0;
+      const uint64_t bmo = c.off_g_idx + ((uint64_t)c.rank * c.g_idx_words + wi) * 4ull;
+      const uint64_t ofo = c.off_g_off + ((uint64_t)c.rank * (nchunks + 1) + my_ch) * 4ull;
+      const bool words = fmt != ZEN_FMT_COO && wi < nwords, offset = hl == 0 && my_ch < nchunks;
+      if (mc) {
+        if (words) { zen_multimem_st4(mc + bmo, word.x); zen_multimem_st4(mc + bmo + 4, word.y); }
+        if (offset) zen_multimem_st4(mc + ofo, at);
+      } else {
+        for (int p = 0; p < npeer; ++p) {
+          if (words) *reinterpret_cast<uint2*>(c.sym[p] + bmo) = word;
+          if (offset) *reinterpret_cast<uint32_t*>(c.sym[p] + ofo) = at;
+        }
+      }
+    }
+    __syncthreads();                                                     // sums and bitmap are clean
+  }
+
+  if (local_status) atomicOr(c.status, local_status);
+  publish_gather<NB>(c, fmt, epoch, s_last);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1308,6 +1696,32 @@ static int launch_scatter(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
+// K2b; for owners whose CTAs read all records themselves it only waits and reports.
+template <int NB>
+static int launch_sort(const ZenSparseBatch<NB>& b, int n, int deterministic, cudaStream_t st) {
+  const ZenSparseCtx& c = b.c[0];
+  const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
+  const int grid = sh.sorted ? grid_for((uint64_t)sh.tiles * c.nranks, 1, share_of(sm_count() * 2, n)) : 1;
+  start<NB>(small_call(c, n), zen_record_sort_kernel<NB>, batch_grid<NB>(grid, n), SB_SORT_THREADS, 0, st, b, deterministic);
+  return (int)cudaGetLastError();
+}
+// K3b
+template <typename T, int W, int NB>
+static int launch_reduce_gather_as(const ZenSparseBatch<NB>& b, int n, uint32_t buckets, int det, cudaStream_t st) {
+  static int known[16][ZEN_MAX_RANKS + 1];
+  const int per_sm = resident(zen_reduce_gather_kernel<T, W, NB>, W * 32, sb_smem<W>(), sb_smem<W>(), known, 0);
+  if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
+  const int grid = grid_for(buckets, 1, share_of(sm_count() * per_sm, n));
+  start<NB>(small_call(b.c[0], n), zen_reduce_gather_kernel<T, W, NB>, batch_grid<NB>(grid, n), W * 32, sb_smem<W>(), st, b, det);
+  return (int)cudaGetLastError();
+}
+template <typename T, int NB>
+static int launch_reduce_gather(const ZenSparseBatch<NB>& b, int n, int det, cudaStream_t st) {
+  const SbShape sh = sb_shape(b.c[0].nslots, b.c[0].cap_rec, b.c[0].nranks);
+  return sh.lg == 14 ? launch_reduce_gather_as<T, 8, NB>(b, n, sh.nbuckets, det, st) : launch_reduce_gather_as<T, 16, NB>(b, n, sh.nbuckets, det, st);
+}
+static bool in_buckets(const ZenSparseCtx& c) { return sb_shape(c.nslots, c.cap_rec, c.nranks).on; }
+
 static ZenSparseBatch<1> one_rank(const ZenSparseCtx* c, const void* in, void* out) {
   ZenSparseBatch<1> b;
   b.c[0] = *c; b.in[0] = in; b.out[0] = out;
@@ -1339,16 +1753,30 @@ int zen_partition_push(const ZenSparseCtx* c, const void* g, const float* thr, i
   return rc;
 }
 
-// K2.  deterministic != 0: one launch per source, in rank order.
+// Buckets in shared memory where the owner's slots allow it (K2b + K3b), K2 + K3 otherwise: what `seg` has to hold, in words, and
+// whether `acc` and `bitmap` are used.
+int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, int64_t* out) {
+  const SbShape sh = sb_shape(nslots, cap_rec, nranks);
+  out[0] = sh.on && sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 1;
+  out[1] = sh.on ? 0 : 1;
+  return 0;
+}
+
+// K2 or K2b.  deterministic != 0: sums in rank order (K2: one launch per source).
 int zen_owner_reduce(const ZenSparseCtx* c, int dtype, int deterministic, void* stream) {
   int rc = 0;
+  if (in_buckets(*c)) return launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, (cudaStream_t)stream);
   DISPATCH_DTYPE(dtype, rc = (launch_reduce<T, 1>(one_rank(c, nullptr, nullptr), 1, deterministic, (cudaStream_t)stream)));
   return rc;
 }
 
-// K3 (compact + push in one launch).
+// K3 or K3b (compact + push in one launch).
 int zen_gather_push(const ZenSparseCtx* c, int dtype, void* stream) {
   int rc = 0;
+  if (in_buckets(*c)) {
+    DISPATCH_DTYPE(dtype, rc = (launch_reduce_gather<T, 1>(one_rank(c, nullptr, nullptr), 1, -1, (cudaStream_t)stream)));
+    return rc;
+  }
   DISPATCH_DTYPE(dtype, rc = (launch_gather<T, 1>(one_rank(c, nullptr, nullptr), 1, (cudaStream_t)stream)));
   return rc;
 }
@@ -1376,6 +1804,13 @@ int zen_sparse_allreduce(const ZenSparseCtx* c, const void* x, const float* thr,
   if (c->epoch_dev && (rc = zen_sparse_epoch_bump(const_cast<uint32_t*>(c->epoch_dev), stream))) return rc;
   if ((rc = zen_partition_push(c, x, thr, dtype, method1 ? 1 : 0, stream))) return rc;
   if (method1) return zen_scatter_sources(c, out, dtype, stream);
+  if (in_buckets(*c)) {
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, st))) return rc;
+    DISPATCH_DTYPE(dtype, rc = (launch_reduce_gather<T, 1>(one_rank(c, nullptr, nullptr), 1, deterministic ? 1 : 0, st)));
+    if (rc) return rc;
+    return zen_densify(c, out, dtype, stream);
+  }
   if ((rc = zen_owner_reduce(c, dtype, deterministic, stream))) return rc;
   if ((rc = zen_gather_push(c, dtype, stream))) return rc;
   return zen_densify(c, out, dtype, stream);
@@ -1399,6 +1834,11 @@ int zen_sparse_allreduce_local(const ZenSparseCtx* c, int n, void* const* io, co
   DISPATCH_DTYPE(dtype, {
     if ((rc = launch_partition<T, ZEN_MAX_RANKS>(b, n, thr, method1, st))) return rc;
     if (method1) return launch_scatter<T, ZEN_MAX_RANKS>(b, n, st);
+    if (in_buckets(*c)) {
+      if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<ZEN_MAX_RANKS>(b, n, deterministic, st))) return rc;
+      if ((rc = launch_reduce_gather<T, ZEN_MAX_RANKS>(b, n, deterministic ? 1 : 0, st))) return rc;
+      return launch_densify<T, ZEN_MAX_RANKS>(b, n, st);
+    }
     int group = (int)((80u << 20) / ((uint64_t)c->nslots * 4 + 1));
     if (group < 1) group = 1;
     if (group >= n) {

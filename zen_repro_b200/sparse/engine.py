@@ -47,7 +47,7 @@ class _Ctx(ctypes.Structure):
         ("off_g_idx", ctypes.c_uint64), ("off_g_off", ctypes.c_uint64), ("off_g_val", ctypes.c_uint64),
         ("cap_rec", ctypes.c_uint32), ("cap_g", ctypes.c_uint32), ("g_idx_words", ctypes.c_uint32),
         ("nchunks", ctypes.c_uint32),
-        ("acc", ctypes.c_void_p), ("bitmap", ctypes.c_void_p), ("chunk_off", ctypes.c_void_p),
+        ("acc", ctypes.c_void_p), ("bitmap", ctypes.c_void_p), ("seg", ctypes.c_void_p),
         ("cursors", ctypes.c_void_p), ("status", ctypes.c_void_p),
         ("numel", ctypes.c_uint64), ("nslots", ctypes.c_uint32), ("nwords", ctypes.c_uint32),
         ("perm", _Perm),
@@ -131,9 +131,12 @@ class SparseRank:
         self.lib = _native.lib()
         assert self.lib.zen_sparse_ctx_size() == ctypes.sizeof(_Ctx), "ctx layout mismatch"
         dev = torch.device(f"cuda:{torch.cuda.current_device()}")
-        self.acc = torch.zeros(plan.nslots, dtype=torch.float32, device=dev)
-        self.bitmap = torch.zeros(plan.nwords, dtype=torch.int32, device=dev)
-        self.chunk_off = torch.zeros(plan.nchunks + 1, dtype=torch.int32, device=dev)
+        # sums and bitmap live in shared memory unless the owner has too many slots for that
+        need = (ctypes.c_int64 * 2)()
+        self.lib.zen_sparse_scratch(plan.nslots, plan.cap_rec, plan.nranks, ctypes.addressof(need))
+        self.seg = torch.empty(int(need[0]), dtype=torch.int32, device=dev)
+        self.acc = torch.zeros(plan.nslots if need[1] else 1, dtype=torch.float32, device=dev)
+        self.bitmap = torch.zeros(plan.nwords if need[1] else 1, dtype=torch.int32, device=dev)
         self.cursors = torch.zeros(MAX_RANKS + 4, dtype=torch.int32, device=dev)
         self.status_t = torch.zeros(1, dtype=torch.int32, device=dev)
         c = _Ctx()
@@ -145,7 +148,7 @@ class SparseRank:
                      "cap_rec", "cap_g", "g_idx_words", "nchunks", "nwords"):
             setattr(c, name, getattr(plan, name))
         c.acc, c.bitmap = self.acc.data_ptr(), self.bitmap.data_ptr()
-        c.chunk_off, c.cursors, c.status = self.chunk_off.data_ptr(), self.cursors.data_ptr(), self.status_t.data_ptr()
+        c.seg, c.cursors, c.status = self.seg.data_ptr(), self.cursors.data_ptr(), self.status_t.data_ptr()
         c.numel, c.nslots = plan.numel, plan.nslots
         c.perm = perm_struct(plan.perm)
         c.k1_density_ppm = max(1, min(1_000_000, int(plan.max_density * 1e6)))
