@@ -16,7 +16,7 @@ def _shape(eng):
     import ctypes
     from zen_repro_b200 import _native
     out = (ctypes.c_int64 * 2)()
-    _native.lib().zen_sparse_scratch(eng.plan.nslots, eng.plan.cap_rec, eng.plan.nranks, ctypes.addressof(out))
+    _native.lib().zen_sparse_scratch(eng.plan.nslots, eng.plan.cap_rec, eng.plan.nranks, 0, ctypes.addressof(out))
     return ("sorted" if out[0] > 1 else "read") if not out[1] else "global"
 
 
@@ -94,3 +94,21 @@ def test_any_order(dtype, method):
     bound = sum(x.double().abs() for x in xs) * 3 * 2.0 ** -24 + want.abs() * unit + (2.0 ** -24 if dtype is torch.float16 else 0.0)
     for o in outs:
         assert ((o.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("n,P,density", [(1, 2, 1.0), (16_384, 3, 0.05), (16_385, 2, 0.5), (40_003, 8, 0.02), (524_288, 8, 0.05), (524_289, 2, 0.05)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_method_1_adds_source_after_source(n, P, density, dtype):
+    """The sum is rounded to the type after every source, in rank order: bit for bit, whatever the bucket shape."""
+    from zen_repro_b200.sparse.engine import VirtualSparseAllReduce
+
+    eng = VirtualSparseAllReduce(n, P, max_density=min(1.0, 1.3 * density), methods=(1,))
+    for call in range(3):
+        xs = _inputs(n, P, density * (1.0, 0.1, 0.9)[call], dtype, 3 * call + P)
+        want = torch.zeros(n, device="cuda", dtype=dtype)
+        for x in xs:
+            want = (want.float() + x.float()).to(dtype)
+        outs = eng(xs, method=1)
+        assert eng.status() == [0] * P
+        for o in outs:
+            assert torch.equal(o, want)

@@ -917,7 +917,7 @@ __device__ __forceinline__ void sb_wait(const ZenSparseCtx& c, uint32_t epoch, u
 
 template <int NB>
 __global__ void __launch_bounds__(SB_SORT_THREADS, 2)
-zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int deterministic) {
+zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int deterministic, int by_index) {
   zen_pdl::enter();
   __shared__ ZenSparseCtx s_ctx;
   const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
@@ -932,7 +932,8 @@ zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int determ
     c.cursors[ZEN_MAX_RANKS + 3] = deterministic ? 2u : 0u;              // for a K3b that is launched without being told
     for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
   }
-  const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
+  const uint32_t nslots = by_index ? (uint32_t)c.numel : c.nslots;       // method 1: records carry element indices
+  const SbShape sh = sb_shape(nslots, c.cap_rec, c.nranks);
   if (sh.on && sh.sorted) {
     const uint32_t nb = sh.nbuckets, stride = sh.tiles * c.nranks;
     uint32_t* seg = c.seg;
@@ -953,12 +954,12 @@ zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int determ
       __syncthreads();
       // a slot that does not exist goes to the bucket after the last, which nobody reads
       uint32_t at[2 * PAIRS];
-      auto bucket = [&](uint32_t slot) { return slot < c.nslots ? slot >> sh.lg : nb; };
+      auto bucket = [&](uint32_t slot) { return slot < nslots ? slot >> sh.lg : nb; };
 #pragma unroll
       for (int u = 0; u < PAIRS; ++u) {
         const uint32_t i = (uint32_t)(u * SB_SORT_THREADS + tid) * 2;
-        if (i < n) { at[2 * u] = atomicAdd(&hist[bucket(r[u].x)], 1u); if (r[u].x >= c.nslots) local_status |= ZEN_BAD_ARG; }
-        if (i + 1 < n) { at[2 * u + 1] = atomicAdd(&hist[bucket(r[u].z)], 1u); if (r[u].z >= c.nslots) local_status |= ZEN_BAD_ARG; }
+        if (i < n) { at[2 * u] = atomicAdd(&hist[bucket(r[u].x)], 1u); if (r[u].x >= nslots) local_status |= ZEN_BAD_ARG; }
+        if (i + 1 < n) { at[2 * u + 1] = atomicAdd(&hist[bucket(r[u].z)], 1u); if (r[u].z >= nslots) local_status |= ZEN_BAD_ARG; }
       }
       __syncthreads();
       // exclusive prefix sums over the buckets, two per thread
@@ -999,6 +1000,82 @@ zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int determ
 }
 
 template <int W> constexpr size_t sb_smem() { return (size_t)W * (2048 * 4 + 256 + SB_WINDOW * 2); }
+
+// The records of one bucket from sources [s_lo, s_hi), each handed to apply(slot, value bits).
+template <int W, typename Apply>
+__device__ __forceinline__ void sb_records(const ZenSparseCtx& c, const SbShape& sh, uint32_t nslots, uint32_t bucket, int s_lo, int s_hi,
+                                           const uint32_t* s_n, uint32_t epoch, uint32_t& status, Apply apply) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (!sh.sorted) {
+    for (int s = s_lo; s < s_hi; ++s) {
+      const uint2* rec = zen_rec_slots(c, c.rank, s, epoch);
+      const uint32_t n = s_n[s], npair = (n + 1) >> 1;
+      for (uint32_t i = tid; i < npair; i += 4 * W * 32) {
+        uint4 r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t j = i + u * W * 32;
+          r[u] = j < npair ? reinterpret_cast<const uint4*>(rec)[j] : make_uint4(0u, 0u, 0u, 0u);   // cap_rec is even
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t j = (i + u * W * 32) * 2;
+          if (j < n) {
+            if (r[u].x >= nslots) status |= ZEN_BAD_ARG;
+            else if ((r[u].x >> sh.lg) == bucket) apply(r[u].x, r[u].y);
+          }
+          if (j + 1 < n) {
+            if (r[u].z >= nslots) status |= ZEN_BAD_ARG;
+            else if ((r[u].z >> sh.lg) == bucket) apply(r[u].z, r[u].w);
+          }
+        }
+      }
+    }
+  } else {
+    // 8, 16 or 32 lanes to a run, at least half of what a full tile's runs hold; a group stays with one source and has U runs, two
+    // records of each per lane, under way together: words, then records, two trips to L2 for most buckets
+    constexpr int U = 6;
+    const uint32_t* seg = c.seg + (size_t)bucket * (sh.tiles * c.nranks);
+    const uint2* rec0 = zen_rec_slots(c, c.rank, 0, epoch);
+    const uint32_t lanes = 1u << sh.lg_lanes, l = lane & (lanes - 1u), group = tid >> sh.lg_lanes, ns = s_hi - s_lo;
+    const uint32_t per_src = ((W * 32u) >> sh.lg_lanes) / ns, k0 = group / ns, src = s_lo + group - k0 * ns;
+    const uint32_t rec_end = c.cap_rec * (uint32_t)c.nranks, ntiles = k0 < per_src ? (s_n[src] + SB_TILE - 1) / SB_TILE : 0u;
+    for (uint32_t k = k0; k < ntiles; k += U * per_src) {
+      uint32_t n[U], at[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t t = k + u * per_src;
+        n[u] = t < ntiles ? seg[src * sh.tiles + t] : 0u;
+        at[u] = src * c.cap_rec + t * SB_TILE;
+      }
+      uint2 x[U], y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t first = n[u] & 0xffffu;
+        n[u] >>= 16;
+        at[u] += first;
+        // (K2b may have given up its wait for a source and left another call's runs: kept inside the tile and the region)
+        if (first + n[u] > SB_TILE || at[u] + n[u] > rec_end) n[u] = 0;
+        if (l < n[u]) x[u] = rec0[at[u] + l];
+        if (l + lanes < n[u]) y[u] = rec0[at[u] + l + lanes];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (l < n[u]) apply(x[u].x, x[u].y);
+        if (l + lanes < n[u]) apply(y[u].x, y[u].y);
+        for (uint32_t i = l + 2 * lanes; i < n[u]; i += 4 * lanes) {   // long runs
+          uint2 z[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i + q * lanes < n[u]) z[q] = rec0[at[u] + i + q * lanes];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i + q * lanes < n[u]) apply(z[q].x, z[q].y);
+        }
+      }
+    }
+  }
+}
 
 // det: 1 rank order, 0 any order, -1 as K2b left it
 template <typename T, int W, int NB>
@@ -1050,75 +1127,7 @@ zen_reduce_gather_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int det)
   for (uint32_t bucket = blockIdx.x; bucket < sh.nbuckets; bucket += gridDim.x) {
     for (int s_lo = 0; s_lo < c.nranks;) {
       const int s_hi = in_order ? s_lo + 1 : c.nranks;
-      if (!sh.sorted) {
-        for (int s = s_lo; s < s_hi; ++s) {
-          const uint2* rec = zen_rec_slots(c, c.rank, s, epoch);
-          const uint32_t n = s_n[s], npair = (n + 1) >> 1;
-          for (uint32_t i = tid; i < npair; i += 4 * W * 32) {
-            uint4 r[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const uint32_t j = i + u * W * 32;
-              r[u] = j < npair ? reinterpret_cast<const uint4*>(rec)[j] : make_uint4(0u, 0u, 0u, 0u);   // cap_rec is even
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const uint32_t j = (i + u * W * 32) * 2;
-              if (j < n) {
-                if (r[u].x >= c.nslots) local_status |= ZEN_BAD_ARG;
-                else if ((r[u].x >> sh.lg) == bucket) apply(r[u].x, r[u].y);
-              }
-              if (j + 1 < n) {
-                if (r[u].z >= c.nslots) local_status |= ZEN_BAD_ARG;
-                else if ((r[u].z >> sh.lg) == bucket) apply(r[u].z, r[u].w);
-              }
-            }
-          }
-        }
-      } else {
-        // 8, 16 or 32 lanes to a run, at least half of what a full tile's runs hold; a group stays with one source and has U runs, two
-        // records of each per lane, under way together: words, then records, two trips to L2 for most buckets
-        constexpr int U = 6;
-        const uint32_t* seg = c.seg + (size_t)bucket * (sh.tiles * c.nranks);
-        const uint2* rec0 = zen_rec_slots(c, c.rank, 0, epoch);
-        const uint32_t lanes = 1u << sh.lg_lanes, l = lane & (lanes - 1u), group = tid >> sh.lg_lanes, ns = s_hi - s_lo;
-        const uint32_t per_src = ((W * 32u) >> sh.lg_lanes) / ns, k0 = group / ns, src = s_lo + group - k0 * ns;
-        const uint32_t rec_end = c.cap_rec * (uint32_t)c.nranks, ntiles = k0 < per_src ? (s_n[src] + SB_TILE - 1) / SB_TILE : 0u;
-        for (uint32_t k = k0; k < ntiles; k += U * per_src) {
-          uint32_t n[U], at[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint32_t t = k + u * per_src;
-            n[u] = t < ntiles ? seg[src * sh.tiles + t] : 0u;
-            at[u] = src * c.cap_rec + t * SB_TILE;
-          }
-          uint2 x[U], y[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint32_t first = n[u] & 0xffffu;
-            n[u] >>= 16;
-            at[u] += first;
-            // (K2b may have given up its wait for a source and left another call's runs: kept inside the tile and the region)
-            if (first + n[u] > SB_TILE || at[u] + n[u] > rec_end) n[u] = 0;
-            if (l < n[u]) x[u] = rec0[at[u] + l];
-            if (l + lanes < n[u]) y[u] = rec0[at[u] + l + lanes];
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (l < n[u]) apply(x[u].x, x[u].y);
-            if (l + lanes < n[u]) apply(y[u].x, y[u].y);
-            for (uint32_t i = l + 2 * lanes; i < n[u]; i += 4 * lanes) {   // long runs
-              uint2 z[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                if (i + q * lanes < n[u]) z[q] = rec0[at[u] + i + q * lanes];
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                if (i + q * lanes < n[u]) apply(z[q].x, z[q].y);
-            }
-          }
-        }
-      }
+      sb_records<W>(c, sh, c.nslots, bucket, s_lo, s_hi, s_n, epoch, local_status, apply);
       __syncthreads();                                                     // in order: the next source's adds come after these
       s_lo = s_hi;
     }
@@ -1498,6 +1507,67 @@ zen_scatter_source_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int src
   }
 }
 
+// Method 1 in buckets: the elements of the output are cut up as the slots of an owner are for K2b and K3b.  One CTA adds up a bucket's
+// elements in shared memory, source after source, rounding to T after each as the scatter above does, and writes them out, zeros
+// included: one or two launches instead of a clearing pass a rank and a launch a source.  That is what bounds small calls; from
+// IB_MAX elements on the scatter's traffic costs less than the sort's.  us, scatter / buckets: 2 x 20 000 bf16 at 2 % 47 / 34, 8 x
+// 200 000 fp32 at 10 % 140 / 80, 8 x 500 000 bf16 at 10 % 133 / 112; 8 x 1 M at 10 % 152 / 178, 2 x 2 M at 1 % 34 / 41.
+#define IB_MAX (1u << 19)
+template <typename T, int NB>
+__global__ void __launch_bounds__(256, 3)
+zen_index_buckets_kernel(const __grid_constant__ ZenSparseBatch<NB> bt) {
+  zen_pdl::enter();
+  __shared__ ZenSparseCtx s_ctx;
+  const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
+  T* __restrict__ out = reinterpret_cast<T*>(bt.out[NB > 1 ? blockIdx.y : 0]);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  constexpr int W = 8;
+  constexpr uint32_t BS = W * 2048, EPV = 16 / sizeof(T);
+  float* acc = reinterpret_cast<float*>(smem_raw);                       // [BS]
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS];
+  const uint32_t epoch = zen_epoch(c), tid = threadIdx.x;
+  for (uint32_t i = tid; i < BS / 4; i += W * 32) reinterpret_cast<float4*>(acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  sb_wait(c, epoch, s_n, s_flag);
+  uint32_t local_status = 0;
+  if (blockIdx.x == 0 && tid == 0)
+    for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
+  const uint32_t N = (uint32_t)c.numel;
+  const SbShape sh = sb_shape(N, c.cap_rec, c.nranks);
+  // an element occurs once in a source
+  auto apply = [&](uint32_t e, uint32_t bits) {
+    float* a = acc + (e & (BS - 1));
+    *a = ZenVal<T>::to_f(ZenVal<T>::from_f(*a + ZenVal<T>::unbits(bits)));
+  };
+  for (uint32_t bucket = blockIdx.x; bucket < sh.nbuckets; bucket += gridDim.x) {
+    for (int s = 0; s < c.nranks; ++s) {
+      sb_records<W>(c, sh, N, bucket, s, s + 1, s_n, epoch, local_status, apply);
+      __syncthreads();
+    }
+    const uint32_t e0 = bucket << sh.lg, n = min(BS, N - e0);
+    for (uint32_t i = tid * EPV; i < n; i += W * 32 * EPV) {
+      float v[EPV];
+#pragma unroll
+      for (uint32_t q = 0; q < EPV; q += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(acc + i + q);
+        *reinterpret_cast<float4*>(acc + i + q) = make_float4(0.f, 0.f, 0.f, 0.f);      // clean for the next bucket
+        v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
+      }
+      if (i + EPV <= n) {
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (uint32_t q = 0; q < EPV; ++q) w[q * sizeof(T) / 4] |= ZenVal<T>::bits(ZenVal<T>::from_f(v[q])) << (sizeof(T) == 2 ? (q & 1) * 16 : 0);
+        *reinterpret_cast<uint4*>(out + e0 + i) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+#pragma unroll
+        for (uint32_t q = 0; q < EPV; ++q)
+          if (i + q < n) out[e0 + i + q] = ZenVal<T>::from_f(v[q]);
+      }
+    }
+    __syncthreads();
+  }
+  if (local_status) atomicOr(c.status, local_status);
+}
+
 __global__ void zen_sparse_epoch_bump_kernel(uint32_t* e) { *e += 1u; }
 
 // ---------------------------------------------------------------------------------------------
@@ -1687,24 +1757,35 @@ static int launch_densify(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
+// K2b; for owners whose CTAs read all records themselves it only waits and reports.
+template <int NB>
+static int launch_sort(const ZenSparseBatch<NB>& b, int n, int deterministic, int by_index, cudaStream_t st) {
+  const ZenSparseCtx& c = b.c[0];
+  const SbShape sh = sb_shape(by_index ? (uint32_t)c.numel : c.nslots, c.cap_rec, c.nranks);
+  const int grid = sh.sorted ? grid_for((uint64_t)sh.tiles * c.nranks, 1, share_of(sm_count() * 2, n)) : 1;
+  start<NB>(small_call(c, n), zen_record_sort_kernel<NB>, batch_grid<NB>(grid, n), SB_SORT_THREADS, 0, st, b, deterministic, by_index);
+  return (int)cudaGetLastError();
+}
 template <typename T, int NB>
 static int launch_scatter(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   const ZenSparseCtx& c = b.c[0];
+  if (c.numel <= IB_MAX) {
+    const SbShape sh = sb_shape((uint32_t)c.numel, c.cap_rec, c.nranks);
+    int rc = 0;
+    if (sh.sorted && (rc = launch_sort<NB>(b, n, 0, 1, st))) return rc;
+    constexpr size_t smem = 8 * 2048 * 4;
+    static int known[16][ZEN_MAX_RANKS + 1];
+    const int per_sm = resident(zen_index_buckets_kernel<T, NB>, 256, smem, smem, known, 0);
+    if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
+    start<NB>(small_call(c, n), zen_index_buckets_kernel<T, NB>, batch_grid<NB>(grid_for(sh.nbuckets, 1, share_of(sm_count() * per_sm, n)), n), 256, smem, st, b);
+    return (int)cudaGetLastError();
+  }
   for (int i = 0; i < n; ++i) ZEN_CUDA_CHECK_RET(cudaMemsetAsync(b.out[i], 0, c.numel * sizeof(T), st));
   const int grid = grid_for(c.cap_rec, 256 * 4, share_of(sm_count() * 8, n));
   for (int s = 0; s < c.nranks; ++s) start<NB>(small_call(c, n), zen_scatter_source_kernel<T, NB>, batch_grid<NB>(grid, n), 256, 0, st, b, s);
   return (int)cudaGetLastError();
 }
 
-// K2b; for owners whose CTAs read all records themselves it only waits and reports.
-template <int NB>
-static int launch_sort(const ZenSparseBatch<NB>& b, int n, int deterministic, cudaStream_t st) {
-  const ZenSparseCtx& c = b.c[0];
-  const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
-  const int grid = sh.sorted ? grid_for((uint64_t)sh.tiles * c.nranks, 1, share_of(sm_count() * 2, n)) : 1;
-  start<NB>(small_call(c, n), zen_record_sort_kernel<NB>, batch_grid<NB>(grid, n), SB_SORT_THREADS, 0, st, b, deterministic);
-  return (int)cudaGetLastError();
-}
 // K3b
 template <typename T, int W, int NB>
 static int launch_reduce_gather_as(const ZenSparseBatch<NB>& b, int n, uint32_t buckets, int det, cudaStream_t st) {
@@ -1755,9 +1836,12 @@ int zen_partition_push(const ZenSparseCtx* c, const void* g, const float* thr, i
 
 // Buckets in shared memory where the owner's slots allow it (K2b + K3b), K2 + K3 otherwise: what `seg` has to hold, in words, and
 // whether `acc` and `bitmap` are used.
-int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, int64_t* out) {
-  const SbShape sh = sb_shape(nslots, cap_rec, nranks);
+// method1_numel: the elements of the output where method 1 is to be served, else 0.
+int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, uint32_t method1_numel, int64_t* out) {
+  const SbShape sh = sb_shape(nslots, cap_rec, nranks), s1 = sb_shape(method1_numel, cap_rec, nranks);
   out[0] = sh.on && sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 1;
+  const int64_t m1 = method1_numel <= IB_MAX && s1.sorted ? (int64_t)s1.nbuckets * s1.tiles * nranks : 1;
+  if (m1 > out[0]) out[0] = m1;
   out[1] = sh.on ? 0 : 1;
   return 0;
 }
@@ -1765,7 +1849,7 @@ int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, int64_t* o
 // K2 or K2b.  deterministic != 0: sums in rank order (K2: one launch per source).
 int zen_owner_reduce(const ZenSparseCtx* c, int dtype, int deterministic, void* stream) {
   int rc = 0;
-  if (in_buckets(*c)) return launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, (cudaStream_t)stream);
+  if (in_buckets(*c)) return launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, 0, (cudaStream_t)stream);
   DISPATCH_DTYPE(dtype, rc = (launch_reduce<T, 1>(one_rank(c, nullptr, nullptr), 1, deterministic, (cudaStream_t)stream)));
   return rc;
 }
@@ -1788,7 +1872,7 @@ int zen_densify(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
   return rc;
 }
 
-// Method 1 consumer: zero `out`, then add every source in rank order.
+// Method 1 consumer: every source added in rank order, in buckets or (above IB_MAX elements) into the cleared `out`.
 int zen_scatter_sources(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
   int rc = 0;
   DISPATCH_DTYPE(dtype, rc = (launch_scatter<T, 1>(one_rank(c, nullptr, out), 1, (cudaStream_t)stream)));
@@ -1806,7 +1890,7 @@ int zen_sparse_allreduce(const ZenSparseCtx* c, const void* x, const float* thr,
   if (method1) return zen_scatter_sources(c, out, dtype, stream);
   if (in_buckets(*c)) {
     const cudaStream_t st = (cudaStream_t)stream;
-    if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, st))) return rc;
+    if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<1>(one_rank(c, nullptr, nullptr), 1, deterministic, 0, st))) return rc;
     DISPATCH_DTYPE(dtype, rc = (launch_reduce_gather<T, 1>(one_rank(c, nullptr, nullptr), 1, deterministic ? 1 : 0, st)));
     if (rc) return rc;
     return zen_densify(c, out, dtype, stream);
@@ -1835,7 +1919,7 @@ int zen_sparse_allreduce_local(const ZenSparseCtx* c, int n, void* const* io, co
     if ((rc = launch_partition<T, ZEN_MAX_RANKS>(b, n, thr, method1, st))) return rc;
     if (method1) return launch_scatter<T, ZEN_MAX_RANKS>(b, n, st);
     if (in_buckets(*c)) {
-      if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<ZEN_MAX_RANKS>(b, n, deterministic, st))) return rc;
+      if (sb_shape(c->nslots, c->cap_rec, c->nranks).sorted && (rc = launch_sort<ZEN_MAX_RANKS>(b, n, deterministic, 0, st))) return rc;
       if ((rc = launch_reduce_gather<T, ZEN_MAX_RANKS>(b, n, deterministic ? 1 : 0, st))) return rc;
       return launch_densify<T, ZEN_MAX_RANKS>(b, n, st);
     }

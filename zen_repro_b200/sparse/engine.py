@@ -133,7 +133,7 @@ class SparseRank:
         dev = torch.device(f"cuda:{torch.cuda.current_device()}")
         # sums and bitmap live in shared memory unless the owner has too many slots for that
         need = (ctypes.c_int64 * 2)()
-        self.lib.zen_sparse_scratch(plan.nslots, plan.cap_rec, plan.nranks, ctypes.addressof(need))
+        self.lib.zen_sparse_scratch(plan.nslots, plan.cap_rec, plan.nranks, plan.numel if plan.method1 else 0, ctypes.addressof(need))
         self.seg = torch.empty(int(need[0]), dtype=torch.int32, device=dev)
         self.acc = torch.zeros(plan.nslots if need[1] else 1, dtype=torch.float32, device=dev)
         self.bitmap = torch.zeros(plan.nwords if need[1] else 1, dtype=torch.int32, device=dev)
