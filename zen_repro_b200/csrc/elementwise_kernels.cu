@@ -1265,6 +1265,18 @@ __device__ __forceinline__ void adam_update(float& p, float& m, float& v, float 
   p = fmaf(-lr, __fdividef(m * ibc1, den), p * decay);
 }
 
+// Eight floats in one access (32-byte aligned).  As two accesses of 16 bytes each lane's half-sectors are 32 bytes apart: the loads ask
+// for every sector twice, and the stores reach L2 as partial sectors.  AdamW over 58 M parameters 350 -> 320 us, over 50 M in fp32 276 ->
+// 269; over 700 M and more it stays at 6.0 TB/s, 92 % of a copy's rate, either way.
+__device__ __forceinline__ void load256(const float* p, float (&v)[8]) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+}
+__device__ __forceinline__ void store256(float* p, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 adamw_kernel(const AdamTensor* tab, int ntensors, const int32_t* chunk_tensor,
@@ -1285,6 +1297,7 @@ adamw_kernel(const AdamTensor* tab, int ntensors, const int32_t* chunk_tensor,
     T* g = reinterpret_cast<T*>(t.grad);
     const float zeros[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const float decay = 1.f - lr * t.wd;
+    const bool wide = ((reinterpret_cast<uintptr_t>(t.master) | reinterpret_cast<uintptr_t>(t.m) | reinterpret_cast<uintptr_t>(t.v)) & 31) == 0;
     // two 8-element vectors per thread and trip, all loads issued before the arithmetic
     for (uint64_t i0 = start + (uint64_t)threadIdx.x * 8; i0 < end; i0 += 2 * 256 * 8) {
       const uint64_t i1 = i0 + 256 * 8;
@@ -1293,19 +1306,32 @@ adamw_kernel(const AdamTensor* tab, int ntensors, const int32_t* chunk_tensor,
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint64_t i = u ? i1 : i0;
-          if (t.master) Vec8<float>::load(t.master + i, pv[u]); else Vec8<T>::load(p + i, pv[u]);
+          if (t.master && wide) load256(t.master + i, pv[u]);
+          else if (t.master) Vec8<float>::load(t.master + i, pv[u]);
+          else Vec8<T>::load(p + i, pv[u]);
           Vec8<T>::load(g + i, gv[u]);
-          Vec8<float>::load(t.m + i, mv[u]);
-          Vec8<float>::load(t.v + i, vv[u]);
+          if (wide) {
+            load256(t.m + i, mv[u]);
+            load256(t.v + i, vv[u]);
+          } else {
+            Vec8<float>::load(t.m + i, mv[u]);
+            Vec8<float>::load(t.v + i, vv[u]);
+          }
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint64_t i = u ? i1 : i0;
 #pragma unroll
           for (int k = 0; k < 8; ++k) adam_update(pv[u][k], mv[u][k], vv[u][k], gv[u][k] * gscale, b1, b2, eps, ibc1, isb2, decay, lr);
-          Vec8<float>::store(t.m + i, mv[u]);
-          Vec8<float>::store(t.v + i, vv[u]);
-          if (t.master) Vec8<float>::store(t.master + i, pv[u]);
+          if (wide) {
+            store256(t.m + i, mv[u]);
+            store256(t.v + i, vv[u]);
+            if (t.master) store256(t.master + i, pv[u]);
+          } else {
+            Vec8<float>::store(t.m + i, mv[u]);
+            Vec8<float>::store(t.v + i, vv[u]);
+            if (t.master) Vec8<float>::store(t.master + i, pv[u]);
+          }
           Vec8<T>::store(p + i, pv[u]);
           if (t.clear) Vec8<T>::store(g + i, zeros);
         }
