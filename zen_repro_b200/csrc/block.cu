@@ -13,8 +13,8 @@
 
 extern "C" {
 int zen_norm_fwd(const void*, const void*, const void*, const void*, void*, void*, float*, float*, int, int, float, int, int, int, void*);
-int zen_norm_bwd_ex(const void*, const void*, const void*, const float*, const float*, const void*, void*, float*, float*, void*, void*,
-                    int, int, int, int, int, int, int, void*);
+int zen_norm_bwd_sums(const void*, const void*, const void*, const float*, const float*, const void*, void*, float*, float*, float*, void*, void*,
+                      int, int, int, int, int, int, int, void*);
 int zen_norm_bwd_parts_used(int, int);
 int zen_colsum_partial(const void*, float*, int, int, int, void*);
 int zen_colsum_parts(int);
@@ -222,7 +222,7 @@ BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base) {
   if (z.w[QKV_B]) {
     const size_t cp = zen_colsum_parts(s.T);
     t.p_qkv = l.take<float>(cp * s.Q);
-    t.p_o = l.take<float>(cp * s.d);
+    t.p_o = l.take<float>(np);
     t.p_down = l.take<float>(cp * s.d);
     t.p_up = l.take<float>((size_t)(z.gated ? cp : zen_act_colsum_parts(s.T)) * s.U);
   }
@@ -297,10 +297,13 @@ int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* r
     if (g2) jobs[njobs++] = ReduceJob{p2, g2, nullptr, nullptr, nparts, cols, gr->acc[gi2], 0};
   };
   auto norm_back = [&](const void* dy, const void* h, int wi, int bi, const float* rstd, const float* mean, const void* dres, void* dh, float* pw,
-                       float* pb) {
-    if (!c.rc) c.rc = zen_norm_bwd_ex(dy, h, z.w[wi], rstd, L ? mean : nullptr, dres, dh, pw, L ? pb : nullptr, nullptr, nullptr, T, d, L,
-                                      z.unit_offset, 0, BF16, 1, stream);
-    reduce(pw, wi, pb, bi, zen_norm_bwd_parts_used(T, d), d);
+                       float* pb, int sum_gi = -1, float* psum = nullptr) {       // sum_gi: the bias whose gradient the column sums of dh are
+    const bool sum = sum_gi >= 0 && z.w[sum_gi] && gr->g[sum_gi];
+    const int parts = zen_norm_bwd_parts_used(T, d);
+    if (!c.rc) c.rc = zen_norm_bwd_sums(dy, h, z.w[wi], rstd, L ? mean : nullptr, dres, dh, pw, L ? pb : nullptr, sum ? psum : nullptr, nullptr, nullptr,
+                                        T, d, L, z.unit_offset, 0, BF16, 1, stream);
+    reduce(pw, wi, pb, bi, parts, d);
+    if (sum) reduce(psum, sum_gi, nullptr, -1, parts, d);
   };
   auto bias_back = [&](const void* dy, int cols, int gi, float* part) {
     if (!z.w[gi] || !gr->g[gi]) return;
@@ -328,7 +331,8 @@ int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* r
     }
   }
   c.project_back(UP, t.du, s.U, z.w[UP_W], t.dy, d, T);
-  norm_back(t.dy, h2, NORM2_W, NORM2_B, v.r2, v.m2, d_h2, t.dres, t.p_n2w, t.p_n2b);
+  // (its result goes to the output projection as it is, unless a norm lies between)
+  norm_back(t.dy, h2, NORM2_W, NORM2_B, v.r2, v.m2, d_h2, t.dres, t.p_n2w, t.p_n2b, s.post1 ? -1 : O_B, t.p_o);
   // weight gradients of the MLP before its scratch is needed no more (post2 and post1 share dpost)
   ZenGemmDesc group[4];
   int ngroup = 0;
@@ -349,11 +353,10 @@ int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* r
   const void* d_o = t.dres;
   if (s.post1) {
     if (s.post2) flush();                                  // the group may still read dpost
-    norm_back(t.dres, v.o, POST1_W, -1, v.rp1, nullptr, nullptr, t.dpost, t.p_p1, nullptr);
+    norm_back(t.dres, v.o, POST1_W, -1, v.rp1, nullptr, nullptr, t.dpost, t.p_p1, nullptr, O_B, t.p_o);
     d_o = t.dpost;
   }
   c.project_back(OUT, d_o, d, z.w[O_W], t.da, s.H, T);
-  bias_back(d_o, d, O_B, t.p_o);
   if (!c.rc) {
     if (!wide_attention(z))
       c.rc = zen_flash_bwd(v.qkv, v.a, t.da, v.lse, t.stat, t.dqkv, B, S, z.hq, z.hkv, z.hd, s.Q, s.H, s.Q, z.scale, stream);

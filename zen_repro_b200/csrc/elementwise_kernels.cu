@@ -7,6 +7,7 @@
 // (train.py:149-157); nothing of them is in its tree.
 #include "act_common.cuh"
 #include "launch.cuh"
+#include "tc_common.cuh"
 #include "xent_common.cuh"
 #include "zen_common.cuh"
 
@@ -445,6 +446,211 @@ norm_bwd_warp_kernel(const T* dy, const T* h, const T* wgt,
   for (int c = threadIdx.x; c < cols; c += blockDim.x) {
     part_dw[(size_t)blockIdx.x * cols + c] = sdw[c];
     if (kLayer && part_db) part_db[(size_t)blockIdx.x * cols + c] = sdb[c];
+  }
+}
+
+// Norm backward in one pass: dh, the partial sums of dw and db, and (part_dh) the column sums of dh itself, which are the bias
+// gradient of the layer before.  CTA b takes rows [b * chunk, (b + 1) * chunk), RS at a time: dy, h and dres arrive through a
+// ring of stages (bulk copies; rows lie end to end, so a stage is one copy an array), 8 / RS warps work out a row's sums and
+// its dh, then every thread adds its columns' share of the RS rows to sums that stay in registers until the chunk ends.
+//
+// What bounds it: memory, each operand once.  As separate kernels dh read dy, h and dres, the parameter sums dy and h again
+// and the bias sums dh, each at two thirds of the L2's rate and with a launch of its own.
+// us, two kernels / one (without the bias sums): 8192 x 768 18.8 / 13.4, 64 x 768 8.5 / 5.0, 4096 x 3072 37.2 / 24.3, 3000 x 2560
+// 24.9 / 19.1, 8192 x 2048 43.3 / 35.1, 2048 x 2304 without a residual gradient 15.0 / 11.1.
+constexpr int NF_STAGES = 3, NF_COLS = 3072;
+__device__ int g_norm_error = 0;                        // a copy that never arrived (zen_norm_error)
+template <typename T, bool kLayer, int RS>
+__global__ void __launch_bounds__(256, 2)
+norm_bwd_fused_kernel(const T* dy, const T* h, const T* wgt, const float* rstd_in, const float* mean_in, const T* dres, T* __restrict__ dh,
+                      float* __restrict__ part_dw, float* __restrict__ part_db, float* __restrict__ part_dh, int rows, int cols, int chunk,
+                      int unit_offset) {
+  constexpr int WPR = 8 / RS, NIT = 3, NVT = RS >= 4 ? 1 : 2;   // warps to a row; vectors of a lane; of a thread's columns
+  extern __shared__ __align__(128) unsigned char nf_smem[];
+  __shared__ __align__(8) uint64_t full[NF_STAGES];
+  __shared__ float red[8][2], srs[NF_STAGES][8], smu[NF_STAGES][8];
+  __shared__ volatile int s_abort;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nv = cols / 8;
+  const bool keep = part_dh != nullptr, third = dres != nullptr || keep;
+  const uint32_t row_bytes = (uint32_t)cols * sizeof(T), arr = RS * row_bytes, stage_bytes = arr * (third ? 3 : 2);
+  if (tid == 0) {
+    s_abort = 0;
+    for (int s = 0; s < NF_STAGES; ++s) tc::mbar_init(&full[s], 1);
+    tc::fence_barrier_init();
+  }
+  __syncthreads();
+  zen_pdl::enter();
+  const int row0 = blockIdx.x * chunk, nrows = min(chunk, rows - row0), nsb = (nrows + RS - 1) / RS;
+  auto issue = [&](int sb) {                            // thread 0
+    const int s = sb % NF_STAGES, n = min(RS, nrows - sb * RS);
+    const size_t at = (size_t)(row0 + sb * RS) * cols;
+    unsigned char* st = nf_smem + s * stage_bytes;
+    const uint32_t bytes = n * row_bytes;
+    tc::mbar_expect_tx(&full[s], bytes * (dres ? 3 : 2));
+    tc::bulk_load_1d(st, dy + at, bytes, &full[s]);
+    tc::bulk_load_1d(st + arr, h + at, bytes, &full[s]);
+    if (dres) tc::bulk_load_1d(st + 2 * arr, dres + at, bytes, &full[s]);
+  };
+  auto stats = [&](int sb) {                            // a thread per row of the stage
+    if (tid < RS && sb * RS + tid < nrows) {
+      const int r = row0 + sb * RS + tid;
+      srs[sb % NF_STAGES][tid] = rstd_in[r];
+      smu[sb % NF_STAGES][tid] = kLayer ? mean_in[r] : 0.f;
+    }
+  };
+  if (tid == 0)
+    for (int sb = 0; sb < min(nsb, NF_STAGES); ++sb) issue(sb);
+  for (int sb = 0; sb < min(nsb, NF_STAGES); ++sb) stats(sb);
+  const float woff = (!kLayer && unit_offset) ? 1.f : 0.f;
+  const int row = warp / WPR, wsub = warp % WPR;
+  typename Pack<T>::raw_t rw[NIT];
+#pragma unroll
+  for (int k = 0; k < NIT; ++k) {
+    const int v = wsub * 32 + lane + k * 32 * WPR;
+    if (v < nv) rw[k] = Pack<T>::load(wgt + (size_t)v * 8);
+  }
+  // column sums: threads in groups that walk interleaved rows where the columns do not take them all
+  const int groups = nv <= 128 ? min(256 / nv, RS) : 1, g = groups > 1 ? tid / nv : 0, c0 = groups > 1 ? tid % nv : tid;
+  float aw[NVT][8], ab[NVT][8], ah[NVT][8];
+#pragma unroll
+  for (int j = 0; j < NVT; ++j)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) aw[j][i] = ab[j][i] = ah[j][i] = 0.f;
+  __syncthreads();
+  for (int sb = 0; sb < nsb; ++sb) {
+    const int s = sb % NF_STAGES, n = min(RS, nrows - sb * RS);
+    unsigned char* st = nf_smem + s * stage_bytes;
+    T *sdy = reinterpret_cast<T*>(st), *shh = reinterpret_cast<T*>(st + arr), *sx = reinterpret_cast<T*>(st + 2 * arr);
+    if (!tc::mbar_test(&full[s], (sb / NF_STAGES) & 1)) {
+      const uint64_t t0 = tc::gtimer();
+      while (!tc::mbar_test(&full[s], (sb / NF_STAGES) & 1))
+        if (s_abort || tc::gtimer() - t0 > tc::WAIT_NS) { s_abort = 1; atomicCAS(&g_norm_error, 0, 1); break; }
+    }
+    const bool mine = row < n;
+    float s1 = 0.f, s2 = 0.f;
+    typename Pack<T>::raw_t rd[NIT], rh[NIT];
+    const float rstd = mine ? srs[s][row] : 0.f, mean = mine ? smu[s][row] : 0.f;
+    if (mine) {
+#pragma unroll
+      for (int k = 0; k < NIT; ++k) {
+        const int v = wsub * 32 + lane + k * 32 * WPR;
+        if (v < nv) {
+          rd[k] = Pack<T>::load(sdy + (size_t)row * cols + v * 8);
+          rh[k] = Pack<T>::load(shh + (size_t)row * cols + v * 8);
+          float d[8], x[8], w[8];
+          Pack<T>::unpack(rd[k], d);
+          Pack<T>::unpack(rh[k], x);
+          Pack<T>::unpack(rw[k], w);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float gr = d[i] * (w[i] + woff);
+            s1 += gr;
+            s2 += gr * ((x[i] - mean) * rstd);
+          }
+        }
+      }
+    }
+    s1 = kLayer ? warp_sum(s1) : 0.f;
+    s2 = warp_sum(s2);
+    if (WPR > 1) {
+      if (lane == 0) { red[warp][0] = s1; red[warp][1] = s2; }
+      __syncthreads();
+      s1 = s2 = 0.f;
+#pragma unroll
+      for (int k = 0; k < WPR; ++k) { s1 += red[row * WPR + k][0]; s2 += red[row * WPR + k][1]; }
+    }
+    s1 /= cols;
+    s2 /= cols;
+    if (mine) {
+      T* out = dh + (size_t)(row0 + sb * RS + row) * cols;
+#pragma unroll
+      for (int k = 0; k < NIT; ++k) {
+        const int v = wsub * 32 + lane + k * 32 * WPR;
+        if (v < nv) {
+          float d[8], x[8], w[8], o[8];
+          Pack<T>::unpack(rd[k], d);
+          Pack<T>::unpack(rh[k], x);
+          Pack<T>::unpack(rw[k], w);
+          if (dres) Vec8<T>::load(sx + (size_t)row * cols + v * 8, o);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float t = rstd * (d[i] * (w[i] + woff) - s1 - (x[i] - mean) * rstd * s2);
+            o[i] = dres ? o[i] + t : t;
+          }
+          Vec8<T>::store(out + v * 8, o);
+          if (keep) Vec8<T>::store(sx + (size_t)row * cols + v * 8, o);
+        }
+      }
+    }
+    if (keep) tc::fence_async_smem();                   // the next copy into this place comes after these stores
+    __syncthreads();
+    if (g < groups) {
+#pragma unroll
+      for (int j = 0; j < NVT; ++j) {
+        const int c = c0 + j * 256;
+        if (c >= nv) continue;
+        for (int r = g; r < n; r += groups) {
+          float d[8], x[8];
+          Vec8<T>::load(sdy + (size_t)r * cols + c * 8, d);
+          Vec8<T>::load(shh + (size_t)r * cols + c * 8, x);
+          const float rs = srs[s][r], mu = smu[s][r];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { aw[j][i] += d[i] * (x[i] - mu) * rs; if (kLayer) ab[j][i] += d[i]; }
+          if (keep) {
+            float o[8];
+            Vec8<T>::load(sx + (size_t)r * cols + c * 8, o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ah[j][i] += o[i];
+          }
+        }
+      }
+    }
+    // The stage of the step before this one is filled again: what was read from it has been added to sums that this step's sums
+    // continue, so none of those loads is still on its way (this step's may be).
+    const int next = sb - 1 + NF_STAGES;
+    if (sb >= 1 && next < nsb) {
+      if (tid == 0) issue(next);
+      stats(next);
+    }
+    __syncthreads();
+  }
+  if (s_abort) {                                        // copies in flight are given time to land
+    const uint64_t t0 = tc::gtimer();
+    while (tc::gtimer() - t0 < 200000ull) __nanosleep(1000);
+    return;
+  }
+  // groups fold into the first through shared memory, in group order
+  float* fold = reinterpret_cast<float*>(nf_smem);
+  for (int k = 1; k < groups; ++k) {
+    if (g == k && c0 < nv) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        fold[c0 * 8 + i] = aw[0][i];
+        if (kLayer) fold[cols + c0 * 8 + i] = ab[0][i];
+        if (keep) fold[2 * cols + c0 * 8 + i] = ah[0][i];
+      }
+    }
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        aw[0][i] += fold[c0 * 8 + i];
+        if (kLayer) ab[0][i] += fold[cols + c0 * 8 + i];
+        if (keep) ah[0][i] += fold[2 * cols + c0 * 8 + i];
+      }
+    }
+    __syncthreads();
+  }
+  if (g == 0) {
+#pragma unroll
+    for (int j = 0; j < NVT; ++j) {
+      const int c = c0 + j * 256;
+      if (c >= nv) continue;
+      const size_t at = (size_t)blockIdx.x * cols + c * 8;
+      Vec8<float>::store(part_dw + at, aw[j]);
+      if (kLayer && part_db) Vec8<float>::store(part_db + at, ab[j]);
+      if (keep) Vec8<float>::store(part_dh + at, ah[j]);
+    }
   }
 }
 
@@ -1458,16 +1664,76 @@ int zen_norm_bwd(const void* dy, const void* h, const void* w, const float* rstd
                          dtype, 0, stream);
 }
 
+int zen_colsum_partial(const void* x, float* part, int rows, int cols, int dtype, void* stream);
+int zen_norm_bwd_sums(const void* dy, const void* h, const void* w, const float* rstd, const float* mean, const void* dres,
+                      void* dh, float* part_dw, float* part_db, float* part_dh, void* dw, void* db, int rows, int cols, int layer,
+                      int unit_offset, int accumulate, int dtype, int skip_reduce, void* stream);
+
+int zen_norm_bwd_ex(const void* dy, const void* h, const void* w, const float* rstd, const float* mean, const void* dres,
+                    void* dh, float* part_dw, float* part_db, void* dw, void* db, int rows, int cols, int layer,
+                    int unit_offset, int accumulate, int dtype, int skip_reduce, void* stream) {
+  return zen_norm_bwd_sums(dy, h, w, rstd, mean, dres, dh, part_dw, part_db, nullptr, dw, db, rows, cols, layer, unit_offset, accumulate, dtype,
+                           skip_reduce, stream);
+}
+
+int zen_norm_error() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_norm_error, sizeof(int)) != cudaSuccess) return -1;
+  if (v) cudaMemcpyToSymbol(g_norm_error, &zero, sizeof(int));
+  return v;
+}
+
 // Partial rows that zen_norm_bwd_ex leaves in part_dw / part_db for a matrix of this shape.
 int zen_norm_bwd_parts_used(int rows, int cols) { (void)cols; const int rpc = colsum_rpc(rows); return (rows + rpc - 1) / rpc; }
 
 // skip_reduce != 0: leave the partial sums in part_dw / part_db (zen_norm_bwd_parts_used(rows, cols) rows of cols floats)
 // for a later zen_colreduce_multi; dw / db are not touched.
-int zen_norm_bwd_ex(const void* dy, const void* h, const void* w, const float* rstd, const float* mean, const void* dres,
-                    void* dh, float* part_dw, float* part_db, void* dw, void* db, int rows, int cols, int layer,
-                    int unit_offset, int accumulate, int dtype, int skip_reduce, void* stream) {
+// part_dh (may be null): column sums of dh, as many partial rows.
+int zen_norm_bwd_sums(const void* dy, const void* h, const void* w, const float* rstd, const float* mean, const void* dres,
+                      void* dh, float* part_dw, float* part_db, float* part_dh, void* dw, void* db, int rows, int cols, int layer,
+                      int unit_offset, int accumulate, int dtype, int skip_reduce, void* stream) {
   if (cols % 8 || cols > NORM_THREADS * NORM_MAXV * 8) return -2;
   cudaStream_t st = (cudaStream_t)stream;
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(dres) |
+                         reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(dh);
+  // One pass up to NF_COLS columns of a 16-bit type (wider rows leave the sums of a thread's columns no registers: 4096 x 5120 90 us as
+  // two kernels, 102 as one), where bulk copies and 16-byte accesses can reach.
+  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && ptrs % 16 == 0) {
+    const int chunk = colsum_rpc(rows), parts = (rows + chunk - 1) / chunk;
+    // rows to a stage: three stages in 108 KB, so that two CTAs fit an SM (8 x 1024 rows of 2048 columns take 56 us with one CTA to an SM,
+    // 46 with two), and three vectors of a row to a lane
+#define NORM_FUSED(L_, RS_)                                                                                                             \
+  do {                                                                                                                                  \
+    const size_t smem = (size_t)NF_STAGES * 3 * RS_ * cols * 2;                                                                         \
+    static const int rc = (int)cudaFuncSetAttribute(norm_bwd_fused_kernel<T, L_, RS_>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
+                                                    NF_STAGES * 3 * 2 * NF_COLS * 2);                                                          \
+    if (rc) return rc;                                                                                                                  \
+    zen_pdl::launch_small(norm_bwd_fused_kernel<T, L_, RS_>, parts, 256, smem, st, (const T*)dy, (const T*)h, (const T*)w, rstd, mean,  \
+                          (const T*)dres, (T*)dh, part_dw, part_db, part_dh, rows, cols, chunk, unit_offset);                           \
+  } while (0)
+#define NORM_FUSED_RS(L_)                                                                                        \
+  do {                                                                                                           \
+    if (cols <= 768) NORM_FUSED(L_, 8);                                                                          \
+    else if (cols <= 1536) NORM_FUSED(L_, 4);                                                                    \
+    else NORM_FUSED(L_, 2);                                                                                      \
+  } while (0)
+    const auto run = [&](auto zero) -> int {
+      typedef decltype(zero) T;
+      if (layer) NORM_FUSED_RS(true); else NORM_FUSED_RS(false);
+      if (skip_reduce) {}
+      else if (layer && db) zen_pdl::launch_small(colreduce_kernel<T>, dim3((cols + 31) / 32, 2), 1024, 0, st, part_dw, (T*)dw, parts, cols, accumulate, part_db, (T*)db);
+      else zen_pdl::launch_small(colreduce_kernel<T>, (cols + 31) / 32, 1024, 0, st, part_dw, (T*)dw, parts, cols, accumulate, (const float*)nullptr, (T*)nullptr);
+      return (int)cudaGetLastError();
+    };
+#undef NORM_FUSED_RS
+#undef NORM_FUSED
+    return dtype == ZEN_DTYPE_BF16 ? run(__nv_bfloat16()) : run(__half());
+  }
+  if (part_dh) {
+    const int rc = zen_norm_bwd_sums(dy, h, w, rstd, mean, dres, dh, part_dw, part_db, nullptr, dw, db, rows, cols, layer, unit_offset, accumulate, dtype,
+                                     skip_reduce, stream);
+    return rc ? rc : zen_colsum_partial(dh, part_dh, rows, cols, dtype, stream);
+  }
   const int grid = cap_grid((size_t)rows, 2);
   if (norm_warp_path(cols, dtype)) {
     // dh by warp-per-row (light on registers, many rows in flight), then dw / db by a column-sum pass
