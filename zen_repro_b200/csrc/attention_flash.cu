@@ -15,8 +15,11 @@
 //  * The products of one tile run while the softmax warps are busy with another: two query tiles per CTA take turns in
 //    the forward kernel; the next scores are issued ahead of the accumulating product in the backward kernels.
 //
-// Backward = dQ kernel (also computes D = rowsum(dO * O)), then dK / dV kernel; no atomics, results do not depend on the
-// schedule.  All mbarrier waits are bounded.
+// Backward, no atomics, results do not depend on the schedule:
+//  * with scratch for dS (zen_flash_ds_bytes): D = rowsum(dO * O), then the dK / dV kernel, which also leaves dS as bf16 tiles in the
+//    layout that the tensor core reads, then dQ as one product per tile over them;
+//  * else dQ kernel (also computes D), then dK / dV kernel: two products and the exponentials of every tile twice.
+//  All mbarrier waits are bounded.
 #include "attention_common.cuh"
 #include "launch.cuh"
 #include "tmap_util.cuh"
@@ -33,7 +36,8 @@ struct FlashParams {
   const __nv_bfloat16* o_in;     // backward: O and dO, row stride ld_o
   const __nv_bfloat16* dout;
   __nv_bfloat16* dqkv;           // backward: [B*S, (Hq + 2*Hkv)*hd], row stride ld_dqkv
-  float* stat;                   // backward: [2][B*Hq, Sp]: -lse2 and -D, left by the dQ kernel for the dK / dV kernel
+  float* stat;                   // backward: [2][B*Hq, Sp]: -lse2 and -D, made before the dK / dV kernel
+  unsigned char* ds;             // backward: dS tiles (see flash_bwd_dq_tiles_kernel), or null
   int B, S, Sp, Hq, Hkv, hd;
   int ld_o, ld_dqkv;
   float scale_log2, scale;
@@ -54,6 +58,12 @@ __device__ __forceinline__ void umma_tile_ts(uint32_t d, uint32_t ta, uint32_t b
   const uint64_t bd = make_desc(b, 16384, 1024);
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) umma_bf16_ts(d, ta + kk * 8, bd + (uint64_t)(kk * 128), idesc, (first && kk == 0) ? 0u : 1u);
+}
+// Byte offset of a dS tile: 128 queries x 128 keys as [16 pieces of 8 queries][128 keys][8 queries] (32 KB), the tiles of a query tile
+// in key order, query tiles of a head in order.
+constexpr int DS_TILE = 32768;
+__device__ __forceinline__ size_t ds_tile(size_t head, int qi, int kt, int nq) {
+  return (head * (size_t)(nq * (nq + 1) / 2) + (size_t)(qi * (qi + 1) / 2 + kt)) * DS_TILE;
 }
 __device__ __forceinline__ void leave(volatile int* abort_flag, bool owner, uint32_t tmem_base, uint32_t cols = 512) {
   fence_before();
@@ -628,7 +638,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
     const uint32_t tP = tDP + w * 64 + lane_addr;
     const uint64_t cs2 = pk2(p.scale_log2, p.scale_log2);
     bool ok = true;
-    int qi = kt;
+    int qi = kt, h = g * rep;
     for (int i = 0; i < n; ++i) {
       const int e = i % C::SB;
       const uint32_t tS = tm0 + (e ? C::S1 : 0) + w * 64 + lane_addr;
@@ -691,12 +701,17 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
           }
         }
         tmem_st32_nowait(tP, pk);
+        if (p.ds) {                                                  // 16 bytes = 8 queries of the key; a warp's stores are 512 in a row
+          uint4* dst = reinterpret_cast<uint4*>(p.ds + ds_tile((size_t)b * p.Hq + h, qi, kt, nq)) + w * 1024 + row;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) dst[c * 128] = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+        }
         tmem_wait_st();
       }
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_ready);
-      if (++qi == nq) qi = kt;
+      if (++qi == nq) { qi = kt; ++h; }
     }
     if (ok && mbar_wait(done, 0, abort_flag, 51, &g_flash_error)) {
       fence_after();
@@ -711,6 +726,124 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_consta
   leave(abort_flag, warp == 9, tm0);
 }
 
+// ============================================================================================ backward with dS kept: D, then dQ
+// stat = -lse2 and -D of every row (rows beyond S: -inf, 0).  CTA = 128 rows of a head; L lanes to a row (8 up to 64 columns, else 16),
+// L / 2 rows of a group under way.
+template <int L>
+__global__ void __launch_bounds__(256)
+flash_stat_kernel(const FlashParams p) {
+  zen_pdl::enter();
+  constexpr int R = L / 2;
+  const int l = threadIdx.x % L, h = blockIdx.y, b = blockIdx.z, s0 = blockIdx.x * 128 + threadIdx.x / L * R;
+  uint4 x[R], y[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const bool in = s0 + i < p.S && l * 8 < p.hd;
+    const size_t at = (size_t)(b * p.S + s0 + i) * p.ld_o + h * p.hd + l * 8;
+    x[i] = in ? *reinterpret_cast<const uint4*>(p.dout + at) : make_uint4(0u, 0u, 0u, 0u);
+    y[i] = in ? *reinterpret_cast<const uint4*>(p.o_in + at) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  const size_t at = ((size_t)b * p.Hq + h) * p.Sp + s0 + l;          // Sp is a multiple of 128
+  const float lse = l < R ? p.lse2[at] : 0.f;
+  float mine = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const uint32_t xw[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, yw[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+    float d = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      d += __uint_as_float(xw[k] << 16) * __uint_as_float(yw[k] << 16);
+      d += __uint_as_float(xw[k] & 0xffff0000u) * __uint_as_float(yw[k] & 0xffff0000u);
+    }
+#pragma unroll
+    for (int o = L / 2; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o, L);
+    if (l == i) mine = d;
+  }
+  if (l < R) {
+    p.stat[at] = -lse;
+    p.stat[(size_t)p.B * p.Hq * p.Sp + at] = -mine;
+  }
+}
+
+// dQ = dS K over the tiles that the dK / dV kernel left: a plain product, one CTA per (128-query tile, head, batch).  The tiles are the
+// A operand as they lie in memory (queries contiguous, 8 x 8 core matrices, no swizzle), one 32 KB bulk copy each.
+// What bounds it: reading dS (1 x 8192, 32 heads: 2.2 GB in 403 us, 5.4 TB/s; working the scores out again took 669 us).
+template <int ATOMS>
+struct DqtCfg {
+  static constexpr int KT = ATOMS * 16384, STAGE = DS_TILE + KT;
+  static constexpr int STAGES = ATOMS == 1 ? 2 : 3;               // up to 64 columns two CTAs fit an SM
+  static constexpr int SMEM = STAGES * STAGE + 128;
+};
+template <int ATOMS>
+__global__ void __launch_bounds__(192, ATOMS == 1 ? 2 : 1)
+flash_bwd_dq_tiles_kernel(const __grid_constant__ CUtensorMap tm, const FlashParams p) {
+  using C = DqtCfg<ATOMS>;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  if ((smem_u32(smem_raw) & 1023u) != 0u) {                        // uniform over the CTA: nothing has been allocated yet
+    if (threadIdx.x == 0) atomicCAS(&g_flash_error, 0, 97);
+    return;
+  }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::STAGES * C::STAGE);
+  uint64_t *full = bars, *empty = bars + 3, *done = bars + 6;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int qi = gridDim.z - 1 - blockIdx.z;                       // heavy query tiles first
+  const int h = blockIdx.x, b = blockIdx.y, g = h / (p.Hq / p.Hkv), n = qi + 1, nq = (p.S + 127) >> 7;
+  const int ksteps = (p.hd + 15) >> 4;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 128);
+  fence_before();
+  __syncthreads();
+  fence_after();
+  zen_pdl::enter();
+  const uint32_t tm0 = *tmem_slot;
+  if (warp == 0) {
+    if (lane == 0) {
+      const unsigned char* src = p.ds + ds_tile((size_t)b * p.Hq + h, qi, 0, nq);
+      for (int j = 0; j < n; ++j) {
+        const int st = j % C::STAGES;
+        if (!mbar_wait(&empty[st], ((j / C::STAGES) & 1) ^ 1, abort_flag, 61, &g_flash_error)) break;
+        unsigned char* dst = smem_raw + st * C::STAGE;
+        mbar_expect_tx(&full[st], C::STAGE);
+        bulk_load_1d(dst, src + (size_t)j * DS_TILE, DS_TILE, &full[st]);
+#pragma unroll
+        for (int a = 0; a < ATOMS; ++a) tma_load_4d(dst + DS_TILE + a * 16384, &tm, &full[st], a * 64, p.Hq + g, j * 128, b);
+      }
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    const uint32_t tmu = uniform(tm0), idesc = make_idesc(128, ksteps * 16, true, true);
+    bool ok = true;
+    for (int j = 0; j < n; ++j) {
+      const int st = j % C::STAGES;
+      ok = mbar_wait(&full[st], (j / C::STAGES) & 1, abort_flag, 62, &g_flash_error);
+      if (!ok) break;
+      fence_after();
+      if (leader) {
+        const uint32_t sa = smem_u32(smem_raw + st * C::STAGE);
+        // no swizzle, queries contiguous: core matrices 2048 bytes apart along the queries, 128 along the keys
+        const uint64_t ad = make_desc_plain(sa, 128, 2048), bd = make_desc(sa + DS_TILE, 16384, 1024);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) umma_bf16(tmu, ad + (uint64_t)(kk * 16), bd + (uint64_t)(kk * 128), idesc, (j > 0 || kk > 0) ? 1u : 0u);
+        if (j + C::STAGES < n) umma_commit(&empty[st]);            // only where a later load waits for it
+      }
+    }
+    if (ok && leader) umma_commit(done);
+  } else if (mbar_wait(done, 0, abort_flag, 63, &g_flash_error)) {
+    fence_after();
+    const int row = (warp & 3) * 32 + lane, qrow = qi * 128 + row;
+    store_rows(tm0 + ((uint32_t)((warp & 3) * 32) << 16), 0, ksteps * 16, p.hd, p.scale,
+               p.dqkv + (size_t)(b * p.S + qrow) * p.ld_dqkv + h * p.hd, qrow < p.S);
+  }
+  leave(abort_flag, warp == 1, tm0, 128);
+}
+
 template <typename F>
 int opt_in(F* f, int bytes) {
   return (int)cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -722,6 +855,7 @@ int flash_attrs() {
     int r = opt_in(flash_fwd_kernel<ATOMS>, FwdCfg<ATOMS>::SMEM);
     if (!r) r = opt_in(flash_bwd_dq_kernel<ATOMS>, DqCfg<ATOMS>::SMEM);
     if (!r) r = opt_in(flash_bwd_dkv_kernel<ATOMS>, DkvCfg<ATOMS>::SMEM);
+    if (!r) r = opt_in(flash_bwd_dq_tiles_kernel<ATOMS>, DqtCfg<ATOMS>::SMEM);
     return r;
   }();
   return rc;
@@ -760,12 +894,28 @@ int zen_flash_fwd(const void* qkv, void* out, float* lse2, int B, int S, int Hq,
   return (int)cudaGetLastError();
 }
 
+// Scratch for which the backward keeps dS between its kernels: 32 KB per pair of a query and a key tile at or below the diagonal.  0: not
+// kept, the scores are worked out twice.
+//  * Fewer than DS_MIN_TILES tiles: the third launch costs more than the scores (1 x 512, 12 heads of 64, 120 tiles: 20 us worked out
+//    twice, 23 kept; 8 x 256, 288 tiles: 25.3 / 24.0; 2 x 512, 24 heads of 128, 480 tiles: 51 / 45).
+//  * Head sizes up to 96 leave a tile in half the time that one of 128 takes, so that dS has to stay in L2 to pay: 8 x 1024, 12 heads of
+//    64 (113 MB) 116 / 110, 1 x 4096 (208 MB) 132 / 138; 3 x 1000, 32 heads of 80 (113 MB) 140 / 127, 1 x 8192 1444 / 1478.
+//  * Above that up to DS_MOST (1 x 4096, 24 heads of 128, 415 MB: 324 / 294; 1 x 8192, 32 heads, 2.2 GB: 1680 / 1575).
+int zen_flash_ds_bytes(int B, int S, int Hq, int Hkv, int hd, int64_t* bytes) {
+  constexpr int64_t DS_MIN_TILES = 256, DS_IN_L2 = (int64_t)128 << 20, DS_MOST = (int64_t)3 << 30;
+  (void)Hkv;
+  const int64_t nq = (S + 127) / 128, tiles = (int64_t)B * Hq * nq * (nq + 1) / 2;
+  *bytes = nq < 2 || tiles < DS_MIN_TILES || tiles * DS_TILE > (hd > 96 ? DS_MOST : DS_IN_L2) ? 0 : tiles * DS_TILE;
+  return 0;
+}
+
 // Backward of the above.  dout / out: bf16 [B*S, Hq*hd] (row stride ld_o); lse2 from the forward; stat: fp32 scratch
-// [2][B, Hq, Sp]; dqkv: bf16 [B*S, (Hq + 2*Hkv)*hd] (row stride ld_dqkv), fully overwritten.
+// [2][B, Hq, Sp]; dqkv: bf16 [B*S, (Hq + 2*Hkv)*hd] (row stride ld_dqkv), fully overwritten.  ds: null, or scratch of
+// zen_flash_ds_bytes (16-byte aligned) where that is not 0.
 int zen_flash_bwd(const void* qkv, const void* out, const void* dout, const float* lse2, float* stat, void* dqkv, int B, int S, int Hq,
-                  int Hkv, int hd, int ld_qkv, int ld_o, int ld_dqkv, float scale, void* stream) {
+                  int Hkv, int hd, int ld_qkv, int ld_o, int ld_dqkv, float scale, void* ds, void* stream) {
   if (!flash_shape_ok(qkv, out, S, Hq, Hkv, hd, ld_qkv, ld_o) || !flash_shape_ok(dout, dqkv, S, Hq, Hkv, hd, ld_o, ld_dqkv)) return -2;
-  if (reinterpret_cast<uintptr_t>(stat) % 16) return -3;
+  if (reinterpret_cast<uintptr_t>(stat) % 16 || reinterpret_cast<uintptr_t>(ds) % 16) return -3;
   CUtensorMap tm, tm_do;
   int rc = zen_tmap::get_heads(qkv, hd, Hq + 2 * Hkv, S, B, ld_qkv, &tm);
   if (!rc) rc = zen_tmap::get_heads(dout, hd, Hq, S, B, ld_o, &tm_do);
@@ -773,19 +923,23 @@ int zen_flash_bwd(const void* qkv, const void* out, const void* dout, const floa
   const int nq = (S + 127) / 128;
   FlashParams p{};
   p.lse2 = const_cast<float*>(lse2); p.o_in = (const __nv_bfloat16*)out; p.dout = (const __nv_bfloat16*)dout;
-  p.dqkv = (__nv_bfloat16*)dqkv; p.stat = stat;
+  p.dqkv = (__nv_bfloat16*)dqkv; p.stat = stat; p.ds = (unsigned char*)ds;
   p.B = B; p.S = S; p.Sp = nq * 128; p.Hq = Hq; p.Hkv = Hkv; p.hd = hd; p.ld_o = ld_o; p.ld_dqkv = ld_dqkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   const dim3 gq(Hq, B, nq), gk(Hkv, B, nq);
   cudaStream_t st = (cudaStream_t)stream;
   if (hd <= 64) {
     if ((rc = flash_attrs<1>())) return rc;
-    zen_pdl::launch(flash_bwd_dq_kernel<1>, gq, 320, DqCfg<1>::SMEM, st, tm, tm_do, p);
+    if (ds) zen_pdl::launch(flash_stat_kernel<8>, dim3(nq, Hq, B), 256, 0, st, p);
+    else zen_pdl::launch(flash_bwd_dq_kernel<1>, gq, 320, DqCfg<1>::SMEM, st, tm, tm_do, p);
     zen_pdl::launch(flash_bwd_dkv_kernel<1>, gk, 320, DkvCfg<1>::SMEM, st, tm, tm_do, p);
+    if (ds) zen_pdl::launch(flash_bwd_dq_tiles_kernel<1>, gq, 192, DqtCfg<1>::SMEM, st, tm, p);
   } else {
     if ((rc = flash_attrs<2>())) return rc;
-    zen_pdl::launch(flash_bwd_dq_kernel<2>, gq, 320, DqCfg<2>::SMEM, st, tm, tm_do, p);
+    if (ds) zen_pdl::launch(flash_stat_kernel<16>, dim3(nq, Hq, B), 256, 0, st, p);
+    else zen_pdl::launch(flash_bwd_dq_kernel<2>, gq, 320, DqCfg<2>::SMEM, st, tm, tm_do, p);
     zen_pdl::launch(flash_bwd_dkv_kernel<2>, gk, 320, DkvCfg<2>::SMEM, st, tm, tm_do, p);
+    if (ds) zen_pdl::launch(flash_bwd_dq_tiles_kernel<2>, gq, 192, DqtCfg<2>::SMEM, st, tm, p);
   }
   return (int)cudaGetLastError();
 }

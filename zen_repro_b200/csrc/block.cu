@@ -25,7 +25,8 @@ int zen_act_colsum_parts(int);
 int zen_rope(void*, int, int, int, int, int, int, float, int, int, void*);
 int zen_colreduce_multi(const void*, int, int, void*);
 int zen_flash_fwd(const void*, void*, float*, int, int, int, int, int, int, int, float, void*);
-int zen_flash_bwd(const void*, const void*, const void*, const float*, float*, void*, int, int, int, int, int, int, int, int, float, void*);
+int zen_flash_bwd(const void*, const void*, const void*, const float*, float*, void*, int, int, int, int, int, int, int, int, float, void*, void*);
+int zen_flash_ds_bytes(int, int, int, int, int, int64_t*);
 int zen_attn_fwd(const void*, void*, float*, int, int, int, int, int, int, int, float, float, void*);
 int zen_attn_bwd(const void*, const void*, const void*, const float*, float*, void*, int, int, int, int, int, int, int, int, float, float,
                  float*, int, void*);
@@ -192,6 +193,7 @@ struct ReduceJob {
 struct BwdTemp {
   void *dm, *du, *dy, *dres, *da, *dqkv, *dpost;
   float *stat, *part256;
+  void* ds;
   float *p_n1w, *p_n1b, *p_n2w, *p_n2b, *p_p1, *p_p2, *p_qkv, *p_o, *p_up, *p_down;
   size_t bytes;
 };
@@ -210,7 +212,11 @@ BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base) {
   t.dqkv = l.take<bf>((size_t)s.T * s.Q);
   if (s.post1 || s.post2) t.dpost = l.take<bf>(td);
   t.stat = l.take<float>(2 * lse_floats(z, s));
-  if (wide_attention(z)) {
+  if (!wide_attention(z)) {
+    int64_t need = 0;
+    zen_flash_ds_bytes(s.B, s.S, z.hq, z.hkv, z.hd, &need);
+    if (need) t.ds = l.take<char>((size_t)need);
+  } else {
     const int hs = zen_attn_hsplit(s.B, s.S, z.hq, z.hkv, z.hd);
     if (hs > 1) t.part256 = l.take<float>((size_t)2 * hs * s.T * z.hkv * z.hd);
   }
@@ -359,7 +365,7 @@ int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* r
   c.project_back(OUT, d_o, d, z.w[O_W], t.da, s.H, T);
   if (!c.rc) {
     if (!wide_attention(z))
-      c.rc = zen_flash_bwd(v.qkv, v.a, t.da, v.lse, t.stat, t.dqkv, B, S, z.hq, z.hkv, z.hd, s.Q, s.H, s.Q, z.scale, stream);
+      c.rc = zen_flash_bwd(v.qkv, v.a, t.da, v.lse, t.stat, t.dqkv, B, S, z.hq, z.hkv, z.hd, s.Q, s.H, s.Q, z.scale, t.ds, stream);
     else
       c.rc = zen_attn_bwd(v.qkv, v.a, t.da, v.lse, t.stat, t.dqkv, B, S, z.hq, z.hkv, z.hd, s.Q, s.H, s.Q, z.scale, z.softcap, t.part256,
                           zen_attn_hsplit(B, S, z.hq, z.hkv, z.hd), stream);

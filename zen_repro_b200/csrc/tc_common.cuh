@@ -165,6 +165,12 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   d |= (uint64_t)2 << 61;
   return d;
 }
+// The same without swizzle, MN-major operand: core matrices of 8 K rows by 16 bytes of M/N (128 contiguous bytes), `lbo` bytes apart
+// along K and `sbo` along M/N.
+__device__ __forceinline__ uint64_t make_desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16 | (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32 |
+         (uint64_t)1 << 46;
+}
 // Instruction descriptor: bf16 x bf16 -> fp32, M x N tile, operand majors (0 = K-major, 1 = MN-major).
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N, bool a_mn, bool b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |

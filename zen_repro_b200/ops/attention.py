@@ -9,12 +9,11 @@ oracle for tests.  The library attention is reached only for other dtypes or whe
 """
 from __future__ import annotations
 
-import torch
-import torch.nn.functional as F
-
-
 import ctypes
 import os
+
+import torch
+import torch.nn.functional as F
 
 from .. import _native
 
@@ -67,15 +66,24 @@ def attention_fwd_kernel(qkv, bsz, seq, hq, hkv, hd, scale, softcap: float = 0.0
     return out, lse2
 
 
+def _flash_ds_bytes(bsz, seq, hq, hkv, hd) -> int:
+    """Bytes of scratch for which the backward keeps dS between its kernels, or 0."""
+    out = ctypes.c_int64()
+    _native.lib().zen_flash_ds_bytes(bsz, seq, hq, hkv, hd, ctypes.addressof(out))
+    return out.value
+
+
 def attention_bwd_kernel(dout, qkv, out, lse2, bsz, seq, hq, hkv, hd, scale, softcap: float = 0.0):
-    """tcgen05 backward: gradient of the fused qkv buffer (dQ kernel + dK/dV kernel, no atomics)."""
+    """tcgen05 backward: gradient of the fused qkv buffer (no atomics)."""
     dout = dout if (dout.is_contiguous() and dout.data_ptr() % 16 == 0) else dout.contiguous()
     dqkv = torch.empty_like(qkv)
     stat = torch.empty(2, *lse2.shape, dtype=torch.float32, device=qkv.device)
     if hd <= 128 and softcap <= 0:
+        need = _flash_ds_bytes(bsz, seq, hq, hkv, hd)
+        ds = torch.empty(need, dtype=torch.uint8, device=qkv.device) if need else None
         rc = _native.lib().zen_flash_bwd(_native.ptr(qkv), _native.ptr(out), _native.ptr(dout), _native.ptr(lse2), _native.ptr(stat),
                                          _native.ptr(dqkv), bsz, seq, hq, hkv, hd, qkv.stride(0), out.stride(0), dqkv.stride(0),
-                                         float(scale), _native.stream_ptr())
+                                         float(scale), _native.ptr(ds), _native.stream_ptr())
         _native.check(rc, "zen_flash_bwd")
         return dqkv
     # few KV heads (MQA / GQA): the query heads of a group are shared out over several CTA pairs
