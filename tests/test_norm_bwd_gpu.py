@@ -41,3 +41,28 @@ def test_against_64_bits(rows, cols, layer):
             assert ((pb.double().sum(0) - dy.double().sum(0)).abs() <= tol).all()
         if sums:
             assert ((ph.double().sum(0) - dh.double().sum(0)).abs() <= tol * (1 + float(dh.abs().max()))).all()
+
+
+@pytest.mark.parametrize("layer", [True, False])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (64, 768), (301, 768), (5000, 1024), (2500, 1032), (900, 2304), (777, 3072), (600, 3080), (9999, 256), (500, 776),
+                                       (300, 1544)])
+def test_forward_against_64_bits(rows, cols, layer):
+    from zen_repro_b200.ops import elementwise as E
+
+    torch.manual_seed(rows * 3 + cols)
+    x, res = (torch.randn(rows, cols, device="cuda").bfloat16() for _ in range(2))
+    w = (torch.randn(cols, device="cuda") * 0.2 + 1.0).bfloat16()
+    b = torch.randn(cols, device="cuda").bfloat16() if layer else None
+    for r in (res, None):
+        y, h, rstd, mean = E.norm_fwd(x, w, b, r, eps=1e-5, layer=layer)
+        want_h = (x.float() + r.float()).bfloat16() if r is not None else x
+        assert torch.equal(h, want_h)
+        hd = want_h.double()
+        mu = hd.mean(1, keepdim=True) if layer else 0.0
+        rs = ((hd - mu).pow(2).mean(1, keepdim=True) + 1e-5).rsqrt()
+        want = (hd - mu) * rs * w.double() + (b.double() if layer else 0.0)
+        # one rounding to bf16 of a result whose terms (the value and the bias) carry a few units of fp32
+        assert ((y.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+        assert ((rstd.double() - rs[:, 0]).abs() <= 1e-5 * rs[:, 0]).all()
+        if layer:
+            assert ((mean.double() - mu[:, 0]).abs() <= 1e-6).all()

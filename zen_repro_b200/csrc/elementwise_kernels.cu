@@ -654,6 +654,140 @@ norm_bwd_fused_kernel(const T* dy, const T* h, const T* wgt, const float* rstd_i
   }
 }
 
+// Norm forward through the same ring of stages: x and the residual arrive while earlier rows are worked on, and few enough CTAs
+// start under their predecessor.  What bounds the kernels above, which it replaces up to NF_COLS columns of a 16-bit type: one
+// row per warp or CTA, read, summed and written in turn, and (a CTA per row) h read back from where it had just been stored.
+// us, before / now, with a residual: 8192 x 768 10.5 / 8.8, 20 000 x 768 28.8 / 20.5, 4096 x 3072 18.2 / 13.9, 8192 x 2048 25.2 / 21.0,
+// 777 x 3072 6.2 / 4.5, 64 x 768 5.0 / 4.8.
+template <typename T, bool kLayer, int RS>
+__global__ void __launch_bounds__(256, 2)
+norm_fwd_staged_kernel(const T* x, const T* res, const T* wgt, const T* bias, T* __restrict__ y, T* __restrict__ hout, float* __restrict__ rstd_out,
+                       float* __restrict__ mean_out, int rows, int cols, int chunk, float eps, int unit_offset) {
+  constexpr int WPR = 8 / RS, NIT = 3;
+  extern __shared__ __align__(128) unsigned char nf_smem[];
+  __shared__ __align__(8) uint64_t full[NF_STAGES];
+  __shared__ float red[2][8];
+  __shared__ volatile int s_abort;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nv = cols / 8;
+  const uint32_t row_bytes = (uint32_t)cols * sizeof(T), arr = RS * row_bytes, stage_bytes = arr * (res ? 2 : 1);
+  if (tid == 0) {
+    s_abort = 0;
+    for (int s = 0; s < NF_STAGES; ++s) tc::mbar_init(&full[s], 1);
+    tc::fence_barrier_init();
+  }
+  __syncthreads();
+  zen_pdl::enter();
+  const int row0 = blockIdx.x * chunk, nrows = min(chunk, rows - row0), nsb = (nrows + RS - 1) / RS;
+  auto issue = [&](int sb) {                            // thread 0
+    const int s = sb % NF_STAGES, n = min(RS, nrows - sb * RS);
+    const size_t at = (size_t)(row0 + sb * RS) * cols;
+    unsigned char* st = nf_smem + s * stage_bytes;
+    const uint32_t bytes = n * row_bytes;
+    tc::mbar_expect_tx(&full[s], bytes * (res ? 2 : 1));
+    tc::bulk_load_1d(st, x + at, bytes, &full[s]);
+    if (res) tc::bulk_load_1d(st + arr, res + at, bytes, &full[s]);
+  };
+  if (tid == 0)
+    for (int sb = 0; sb < min(nsb, NF_STAGES); ++sb) issue(sb);
+  const int row = warp / WPR, wsub = warp % WPR;
+  typename Pack<T>::raw_t rw[NIT], rb[kLayer ? NIT : 1];
+#pragma unroll
+  for (int k = 0; k < NIT; ++k) {
+    const int v = wsub * 32 + lane + k * 32 * WPR;
+    if (v < nv) {
+      rw[k] = Pack<T>::load(wgt + (size_t)v * 8);
+      if (kLayer && bias) rb[k] = Pack<T>::load(bias + (size_t)v * 8);
+    }
+  }
+  // sum over a row's warps; `slot` alternates so that one barrier a sum is enough
+  auto row_sum = [&](float v, int slot) {
+    v = warp_sum(v);
+    if (WPR == 1) return v;
+    if (lane == 0) red[slot][warp] = v;
+    __syncthreads();
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < WPR; ++k) t += red[slot][row * WPR + k];
+    return t;
+  };
+  for (int sb = 0; sb < nsb; ++sb) {
+    const int s = sb % NF_STAGES, n = min(RS, nrows - sb * RS);
+    const T* sx = reinterpret_cast<const T*>(nf_smem + s * stage_bytes);
+    const T* sr = reinterpret_cast<const T*>(nf_smem + s * stage_bytes + arr);
+    if (!tc::mbar_test(&full[s], (sb / NF_STAGES) & 1)) {
+      const uint64_t t0 = tc::gtimer();
+      while (!tc::mbar_test(&full[s], (sb / NF_STAGES) & 1))
+        if (s_abort || tc::gtimer() - t0 > tc::WAIT_NS) { s_abort = 1; atomicCAS(&g_norm_error, 0, 2); break; }
+    }
+    const bool mine = row < n;
+    const size_t base = (size_t)(row0 + sb * RS + row) * cols;
+    float h[NIT][8], sum = 0.f;
+    if (mine) {
+#pragma unroll
+      for (int k = 0; k < NIT; ++k) {
+        const int v = wsub * 32 + lane + k * 32 * WPR;
+        if (v < nv) {
+          Vec8<T>::load(sx + (size_t)row * cols + v * 8, h[k]);
+          if (res) {
+            float r[8];
+            Vec8<T>::load(sr + (size_t)row * cols + v * 8, r);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) h[k][i] += r[i];
+          }
+          if (hout) {                                   // continue with exactly what is stored
+            Vec8<T>::store(hout + base + v * 8, h[k]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) h[k][i] = ZenVal<T>::to_f(ZenVal<T>::from_f(h[k][i]));
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sum += kLayer ? h[k][i] : h[k][i] * h[k][i];
+        }
+      }
+    }
+    float mean = 0.f, var = row_sum(sum, 0) / cols;
+    if (kLayer) {
+      mean = var;
+      float d2 = 0.f;
+      if (mine) {
+#pragma unroll
+        for (int k = 0; k < NIT; ++k)
+          if (wsub * 32 + lane + k * 32 * WPR < nv) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { const float d = h[k][i] - mean; d2 += d * d; }
+          }
+      }
+      var = row_sum(d2, 1) / cols;
+    }
+    const float rstd = rsqrtf(var + eps);
+    if (mine) {
+      if (wsub == 0 && lane == 0) {
+        rstd_out[row0 + sb * RS + row] = rstd;
+        if (kLayer) mean_out[row0 + sb * RS + row] = mean;
+      }
+#pragma unroll
+      for (int k = 0; k < NIT; ++k) {
+        const int v = wsub * 32 + lane + k * 32 * WPR;
+        if (v < nv) {
+          float w[8], b[8], o[8];
+          Pack<T>::unpack(rw[k], w);
+          if (kLayer && bias) Pack<T>::unpack(rb[k], b);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            o[i] = kLayer ? (h[k][i] - mean) * rstd * w[i] + (bias ? b[i] : 0.f) : h[k][i] * rstd * (unit_offset ? 1.f + w[i] : w[i]);
+          Vec8<T>::store(y + base + v * 8, o);
+        }
+      }
+    }
+    __syncthreads();
+    // this step's rows have been summed, so none of its loads is still on its way: sums went through shuffles before the barrier
+    if (tid == 0 && sb + NF_STAGES < nsb) issue(sb + NF_STAGES);
+  }
+  if (s_abort) {                                        // copies in flight are given time to land
+    const uint64_t t0 = tc::gtimer();
+    while (tc::gtimer() - t0 < 200000ull) __nanosleep(1000);
+  }
+}
+
 // Parameter gradients of a norm, column-sum style: CTA b covers rows [32 b, 32 b + 32) and every column (a thread
 // owns 8 columns, loads are coalesced along the row): part_dw[b][c] = sum_r dy * xhat, part_db[b][c] = sum_r dy.
 template <typename T, bool kLayer>
@@ -1671,6 +1805,34 @@ int zen_norm_fwd(const void* x, const void* res, const void* w, const void* b, v
                  float* mean, int rows, int cols, float eps, int layer, int unit_offset, int dtype, void* stream) {
   if (cols % 8 || cols > NORM_THREADS * NORM_MAXV * 8) return -2;
   cudaStream_t st = (cudaStream_t)stream;
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(w) |
+                         reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(hout);
+  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && rows > 0 && ptrs % 16 == 0) {
+    const int chunk = (rows + 2 * sm_count_e() - 1) / (2 * sm_count_e()), grid = (rows + chunk - 1) / chunk;
+#define NORM_STAGED(L_, RS_)                                                                                                            \
+  do {                                                                                                                                  \
+    const size_t smem = (size_t)NF_STAGES * (res ? 2 : 1) * RS_ * cols * 2;                                                             \
+    static const int rc = (int)cudaFuncSetAttribute(norm_fwd_staged_kernel<T, L_, RS_>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+                                                    NF_STAGES * 2 * 2 * NF_COLS * 2);                                                   \
+    if (rc) return rc;                                                                                                                  \
+    zen_pdl::launch_small(norm_fwd_staged_kernel<T, L_, RS_>, grid, 256, smem, st, (const T*)x, (const T*)res, (const T*)w, (const T*)b,  \
+                          (T*)y, (T*)hout, rstd, mean, rows, cols, chunk, eps, unit_offset);                                            \
+  } while (0)
+#define NORM_STAGED_RS(L_)                                   \
+  do {                                                       \
+    if (cols <= 768) NORM_STAGED(L_, 8);                     \
+    else if (cols <= 1536) NORM_STAGED(L_, 4);               \
+    else NORM_STAGED(L_, 2);                                 \
+  } while (0)
+    const auto run = [&](auto zero) -> int {
+      typedef decltype(zero) T;
+      if (layer) NORM_STAGED_RS(true); else NORM_STAGED_RS(false);
+      return (int)cudaGetLastError();
+    };
+#undef NORM_STAGED_RS
+#undef NORM_STAGED
+    return dtype == ZEN_DTYPE_BF16 ? run(__nv_bfloat16()) : run(__half());
+  }
   if (norm_warp_path(cols, dtype)) {
     const int grid = cap_grid((size_t)(rows + NORMW_WARPS - 1) / NORMW_WARPS, 8);
     DISPATCH_T(dtype, {
