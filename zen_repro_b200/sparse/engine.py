@@ -357,18 +357,19 @@ class VirtualSparseAllReduce:
         assert len(inputs) == self.plan.nranks
         self.epoch += 1
         e = self.epoch
-        flats = [t.reshape(-1) for t in inputs]
-        outs = [torch.empty_like(f) for f in flats]
+        # a small call is bound by this function: buckets are flat already, and sixteen reshapes of nothing took 16 us of 54 (eight ranks)
+        flats = [t if t.dim() == 1 else t.reshape(-1) for t in inputs]
         n, dtype = self.plan.numel, flats[0].dtype
-        for f, o in zip(flats, outs):
+        for f in flats:
             assert f.is_cuda and f.is_contiguous() and f.numel() == n and f.dtype == dtype
-            assert o.data_ptr() % 16 == 0
+        outs = [torch.empty_like(f) for f in flats]
         io = array("Q", [t.data_ptr() for t in flats + outs])
+        assert not any(p % 16 for p in io[len(flats):])
         rc = self.ranks[0].lib.zen_sparse_allreduce_local(
             self._ctx_addr, len(flats), io.buffer_info()[0], _native.ptr(threshold), e, _fmt_for(method),
             _native.DTYPE_CODE[dtype], int(method == 1), int(self.deterministic), _native.stream_ptr())
         _native.check(rc, "zen_sparse_allreduce_local")
-        return [o.reshape(t.shape) for o, t in zip(outs, inputs)]
+        return [o if t.dim() == 1 else o.reshape(t.shape) for o, t in zip(outs, inputs)]
 
     def status(self) -> list[int]:
         return [r.read_status() for r in self.ranks]
