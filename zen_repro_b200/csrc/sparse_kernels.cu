@@ -118,7 +118,9 @@ __device__ __forceinline__ ZenMail* zen_rec_mail(const ZenSparseCtx& c, int at_r
 
 #define K1_THREADS 288                                  // eight consumer warps and the producer warp
 #define K1_WARPS 8
-#define K1_QCAP 256
+// Records of a queue: a longer queue is drained less often (every drain stops the consumer warps twice), as long as three CTAs still fit
+// an SM.  us with 256 / 512: four ranks of 4 M bf16 at 10 % 30.8 / 25.9, two of 13 M fp32 at 2 % 32.8 / 29.6, eight of 64 M at 1 % 207 / 228.
+__host__ __device__ __forceinline__ uint32_t k1_qcap(int queues) { return queues <= 4 ? 512u : 256u; }
 #define K1_FLUSH_MIN 128
 #define K1_STAGE_BYTES 16384
 #define K1_NS 2
@@ -228,8 +230,9 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
   constexpr int VPL = K1_STAGE_BYTES / VB / K1_CONSUMERS;             // vectors per lane per stage
   static_assert(VPL >= 1, "stage too small");
   const int nq = kBroadcast ? 1 : c.nranks;
+  const uint32_t qcap = k1_qcap(nq);
   unsigned char* ring = smem_raw;                                     // [K1_NS][K1_STAGE_BYTES] (kRing)
-  uint2* q = reinterpret_cast<uint2*>(smem_raw + (kRing ? K1_NS * K1_STAGE_BYTES : 0));   // [nq][K1_QCAP]
+  uint2* q = reinterpret_cast<uint2*>(smem_raw + (kRing ? K1_NS * K1_STAGE_BYTES : 0));   // [nq][qcap]
   __shared__ uint64_t full[K1_NS], empty[K1_NS];
   __shared__ uint32_t qn[ZEN_MAX_RANKS];
   __shared__ uint32_t qvalid[ZEN_MAX_RANKS];
@@ -326,8 +329,8 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
       const uint32_t cnt = __popc(m);
       uint32_t k = atomicAdd(&qn[owner], cnt);
       bool direct = false;
-      if (k + cnt > K1_QCAP) {
-        if (k <= K1_QCAP) qvalid[owner] = k;                          // exactly one lane per overflow sees this
+      if (k + cnt > qcap) {
+        if (k <= qcap) qvalid[owner] = k;                          // exactly one lane per overflow sees this
         direct = true;
         k = atomicAdd(&c.cursors[owner], cnt);                        // reserve directly in the destination
       }
@@ -336,7 +339,7 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
         m &= m - 1;
         const uint2 rec = make_uint2(slot0 + i, sizeof(T) == 4 ? en.w[i] : (uint32_t)reinterpret_cast<const unsigned short*>(en.w)[i]);
         if (!direct) {
-          q[owner * K1_QCAP + k] = rec;
+          q[owner * qcap + k] = rec;
         } else if (k < c.cap_rec) {
           if (kBroadcast) {
             for (int p = 0; p < c.nranks; ++p)
@@ -354,7 +357,7 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
     auto flush = [&](bool final_flush) {
       if (warp < nq) {
         uint32_t n = qn[warp];
-        const bool overflowed = n > K1_QCAP;
+        const bool overflowed = n > qcap;
         if (overflowed) n = qvalid[warp];
         if (n > 0 && (n >= K1_FLUSH_MIN || final_flush || overflowed)) {
           uint32_t gbase = 0;
@@ -362,7 +365,7 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
           gbase = __shfl_sync(0xffffffffu, gbase, 0);
           const uint32_t fit = (gbase >= c.cap_rec) ? 0u : min(n, c.cap_rec - gbase);
           if (fit < n) local_status |= ZEN_REC_OVERFLOW;
-          const uint2* src = q + warp * K1_QCAP;
+          const uint2* src = q + warp * qcap;
           if (kBroadcast) {
             for (int p = 0; p < c.nranks; ++p) {
               uint2* dst = reinterpret_cast<uint2*>(c.sym[p] + c.off_rec) + rec_base + gbase;
@@ -878,7 +881,10 @@ zen_gather_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int ppw) {
 // 10 us with 24 warps to an SM, of which the stores to eight peers are a quarter.  us, K2 + K3 / K2b + K3b: 8 ranks of 2^26 bf16
 // elements at 1 % 170 + 121 / 34 + 100, 4 of 13 M 20 + 20 / 7 + 19, 2 of 50 000 (fp32) 4 + 11 / 0 + 8.
 // (Tried: one CTA per bucket, not persistent, 120 us for the first; the next bucket's runs fetched ahead 195, in spills and waits.)
-// K2 and K3 remain for owners of more than 2^25 slots, whose tiles would leave less than four records to a run.
+// K2 and K3 remain for owners of more than 2^25 slots, whose tiles would leave less than four records to a run, and for calls of
+// less than one bucket over all owners, which the host's side bounds (3 x 10 000: 26 us as four
+// kernels, 25 to 28 in buckets).
+#define SB_MIN_SLOTS (1u << 14)
 #define SB_TILE 4096
 #define SB_MAX_BUCKETS 1024
 #define SB_SORT_THREADS 512
@@ -892,7 +898,7 @@ __host__ __device__ __forceinline__ SbShape sb_shape(uint32_t nslots, uint32_t c
   s.nbuckets = (nslots + (1u << s.lg) - 1) >> s.lg;
   s.tiles = (cap_rec + SB_TILE - 1) / SB_TILE;
   s.lg_lanes = s.nbuckets > 384 ? 3u : s.nbuckets > 160 ? 4u : 5u;      // a full tile's runs: 4096 / buckets records
-  s.on = s.nbuckets <= SB_MAX_BUCKETS;
+  s.on = s.nbuckets <= SB_MAX_BUCKETS && (uint64_t)nslots * nranks >= SB_MIN_SLOTS;
   s.sorted = s.nbuckets > 1 && (uint64_t)cap_rec * nranks > SB_FILTER_RECORDS;
   return s;
 }
@@ -1509,7 +1515,7 @@ zen_scatter_source_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int src
 
 // Method 1 in buckets: the elements of the output are cut up as the slots of an owner are for K2b and K3b.  One CTA adds up a bucket's
 // elements in shared memory, source after source, rounding to T after each as the scatter above does, and writes them out, zeros
-// included: one or two launches instead of a clearing pass a rank and a launch a source.  That is what bounds small calls; from
+// included: one or two launches instead of a clearing pass a rank and a launch a source (from a bucket's size on).  That is what bounds small calls; from
 // IB_MAX elements on the scatter's traffic costs less than the sort's.  us, scatter / buckets: 2 x 20 000 bf16 at 2 % 47 / 34, 8 x
 // 200 000 fp32 at 10 % 140 / 80, 8 x 500 000 bf16 at 10 % 133 / 112; 8 x 1 M at 10 % 152 / 178, 2 x 2 M at 1 % 34 / 41.
 #define IB_MAX (1u << 19)
@@ -1671,10 +1677,10 @@ static int launch_partition_as(const ZenSparseBatch<NB>& b, int n, const float* 
   const ZenSparseCtx& c = b.c[0];
   const uint64_t nst = (c.numel + EPS - 1) / EPS;
   const int nq = kBroadcast ? 1 : c.nranks;
-  constexpr size_t kRingBytes = kRing ? (size_t)K1_NS * K1_STAGE_BYTES : 0, kQueue = K1_QCAP * sizeof(uint2);
-  const size_t smem = nq * kQueue + kRingBytes;
+  constexpr size_t kRingBytes = kRing ? (size_t)K1_NS * K1_STAGE_BYTES : 0, kQueue = sizeof(uint2);
+  const size_t smem = nq * k1_qcap(nq) * kQueue + kRingBytes;
   static int known[16][ZEN_MAX_RANKS + 1];
-  const int per_sm = resident(zen_partition_push_kernel<T, kBroadcast, kRing, NB>, K1_THREADS, smem, (kBroadcast ? 1 : ZEN_MAX_RANKS) * kQueue + kRingBytes, known, nq);
+  const int per_sm = resident(zen_partition_push_kernel<T, kBroadcast, kRing, NB>, K1_THREADS, smem, 2048 * kQueue + kRingBytes, known, nq);
   if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
   // every CTA takes a fixed share of the stages, so the grid is exactly what is resident at once
   const int grid = grid_for(nst, 1, share_of(sm_count() * per_sm, n));
@@ -1683,7 +1689,7 @@ static int launch_partition_as(const ZenSparseBatch<NB>& b, int n, const float* 
   int batch = 2;
   if (c.k1_density_ppm) {
     const double per_stage = (double)EPS * c.k1_density_ppm * 1e-6 / nq;
-    batch = per_stage > 0 ? (int)((K1_QCAP / 2) / per_stage) : 16;
+    batch = per_stage > 0 ? (int)((k1_qcap(nq) / 2) / per_stage) : 16;
     if (batch < 1) batch = 1;
     if (batch > 16) batch = 16;
   }
@@ -1769,7 +1775,7 @@ static int launch_sort(const ZenSparseBatch<NB>& b, int n, int deterministic, in
 template <typename T, int NB>
 static int launch_scatter(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   const ZenSparseCtx& c = b.c[0];
-  if (c.numel <= IB_MAX) {
+  if (c.numel <= IB_MAX && c.numel >= SB_MIN_SLOTS) {
     const SbShape sh = sb_shape((uint32_t)c.numel, c.cap_rec, c.nranks);
     int rc = 0;
     if (sh.sorted && (rc = launch_sort<NB>(b, n, 0, 1, st))) return rc;
@@ -1840,7 +1846,7 @@ int zen_partition_push(const ZenSparseCtx* c, const void* g, const float* thr, i
 int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, uint32_t method1_numel, int64_t* out) {
   const SbShape sh = sb_shape(nslots, cap_rec, nranks), s1 = sb_shape(method1_numel, cap_rec, nranks);
   out[0] = sh.on && sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 1;
-  const int64_t m1 = method1_numel <= IB_MAX && s1.sorted ? (int64_t)s1.nbuckets * s1.tiles * nranks : 1;
+  const int64_t m1 = method1_numel <= IB_MAX && method1_numel >= SB_MIN_SLOTS && s1.sorted ? (int64_t)s1.nbuckets * s1.tiles * nranks : 1;
   if (m1 > out[0]) out[0] = m1;
   out[1] = sh.on ? 0 : 1;
   return 0;
