@@ -101,3 +101,17 @@ def test_loss_function_equals_the_separate_passes(rows, softcap, monkeypatch):
     assert abs(one[0] - two[0]) <= 1e-5 * two[0] and abs(one[1] - one[0]) <= 1e-6 * one[0]
     for x, y in zip(one[2:], two[2:]):
         assert (x.double() - y.double()).norm() <= 4e-3 * y.double().norm()       # bf16 gradients of the same fp32 softmax
+
+
+@pytest.mark.parametrize("labels", [lambda: torch.zeros(299, dtype=torch.int64, device="cuda"), lambda: torch.zeros(600, dtype=torch.int64, device="cuda"),
+                                    lambda: torch.zeros(300, dtype=torch.int32, device="cuda"), lambda: torch.zeros(300, dtype=torch.int64),
+                                    lambda: torch.zeros(600, dtype=torch.int64, device="cuda")[::2]])
+def test_labels_that_the_kernel_would_misread_are_refused(labels):
+    from zen_repro_b200 import _native
+    from zen_repro_b200.ops import gemm as G
+
+    a, b = torch.randn(300, 64, device="cuda").bfloat16(), torch.randn(1000, 64, device="cuda").bfloat16()
+    before = _native.launch_count()
+    with pytest.raises(ValueError):
+        G.gemm_nt_loss(a, b, labels())
+    assert _native.launch_count() == before

@@ -263,6 +263,8 @@ def gemm_nt_loss(a, b, labels, out=None, softcap: float = 0.0):
     nowhere) and what a cross-entropy against ``labels`` (int64) needs of them: ``(part, target)`` for ``elementwise.xent_finish``.
     Operands as :func:`makes_loss_statistics` asks."""
     (M, K), N = a.shape, b.shape[0]
+    if labels.numel() != M or labels.dtype is not torch.int64 or not labels.is_contiguous() or labels.device != a.device:
+        raise ValueError(f"{labels.numel()} labels of {labels.dtype} on {labels.device} for {M} rows of logits on {a.device}")
     part = torch.empty(2 * ((N + 255) // 256), (M + 31) // 32 * 32, 2, dtype=torch.float32, device=a.device)
     target = torch.empty(M, dtype=torch.float32, device=a.device)
     c, ldc = (0, 0) if out is None else (out.data_ptr(), out.stride(0))
