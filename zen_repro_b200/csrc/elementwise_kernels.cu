@@ -659,11 +659,11 @@ norm_bwd_fused_kernel(const T* dy, const T* h, const T* wgt, const float* rstd_i
 // row per warp or CTA, read, summed and written in turn, and (a CTA per row) h read back from where it had just been stored.
 // us, before / now, with a residual: 8192 x 768 10.5 / 8.8, 20 000 x 768 28.8 / 20.5, 4096 x 3072 18.2 / 13.9, 8192 x 2048 25.2 / 21.0,
 // 777 x 3072 6.2 / 4.5, 64 x 768 5.0 / 4.8.
-template <typename T, bool kLayer, int RS>
+template <typename T, bool kLayer, int RS, int NIT>
 __global__ void __launch_bounds__(256, 2)
 norm_fwd_staged_kernel(const T* x, const T* res, const T* wgt, const T* bias, T* __restrict__ y, T* __restrict__ hout, float* __restrict__ rstd_out,
                        float* __restrict__ mean_out, int rows, int cols, int chunk, float eps, int unit_offset) {
-  constexpr int WPR = 8 / RS, NIT = 3;
+  constexpr int WPR = 8 / RS;
   extern __shared__ __align__(128) unsigned char nf_smem[];
   __shared__ __align__(8) uint64_t full[NF_STAGES];
   __shared__ float red[2][8];
@@ -699,16 +699,16 @@ norm_fwd_staged_kernel(const T* x, const T* res, const T* wgt, const T* bias, T*
       if (kLayer && bias) rb[k] = Pack<T>::load(bias + (size_t)v * 8);
     }
   }
-  // sum over a row's warps; `slot` alternates so that one barrier a sum is enough
+  // Sum over a row's warps, in the order of norm_fwd_warp_kernel up to 1024 columns and of norm_fwd_kernel above: a
+  // last bit of one row's statistics flips one rounding in 400 000, which four layers of a Llama amplify to 0.9 % of the
+  // logits, and the kernel that a call takes should not decide that.  `slot` alternates so that one barrier a sum is enough
   auto row_sum = [&](float v, int slot) {
     v = warp_sum(v);
-    if (WPR == 1) return v;
+    if constexpr (WPR == 1) return v;
     if (lane == 0) red[slot][warp] = v;
     __syncthreads();
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < WPR; ++k) t += red[slot][row * WPR + k];
-    return t;
+    const float* r = &red[slot][row * WPR];
+    return (r[0] + r[2]) + (r[1] + r[3]);                // as block_sum adds four warps
   };
   for (int sb = 0; sb < nsb; ++sb) {
     const int s = sb % NF_STAGES, n = min(RS, nrows - sb * RS);
@@ -1809,20 +1809,20 @@ int zen_norm_fwd(const void* x, const void* res, const void* w, const void* b, v
                          reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(hout);
   if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && rows > 0 && ptrs % 16 == 0) {
     const int chunk = (rows + 2 * sm_count_e() - 1) / (2 * sm_count_e()), grid = (rows + chunk - 1) / chunk;
-#define NORM_STAGED(L_, RS_)                                                                                                            \
+#define NORM_STAGED(L_, RS_, NIT_)                                                                                                      \
   do {                                                                                                                                  \
     const size_t smem = (size_t)NF_STAGES * (res ? 2 : 1) * RS_ * cols * 2;                                                             \
-    static const int rc = (int)cudaFuncSetAttribute(norm_fwd_staged_kernel<T, L_, RS_>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                                    NF_STAGES * 2 * 2 * NF_COLS * 2);                                                   \
+    static const int rc = (int)cudaFuncSetAttribute(norm_fwd_staged_kernel<T, L_, RS_, NIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                    NF_STAGES * 2 * 8 * 1024 * 2);                                                      \
     if (rc) return rc;                                                                                                                  \
-    zen_pdl::launch_small(norm_fwd_staged_kernel<T, L_, RS_>, grid, 256, smem, st, (const T*)x, (const T*)res, (const T*)w, (const T*)b,  \
+    zen_pdl::launch_small(norm_fwd_staged_kernel<T, L_, RS_, NIT_>, grid, 256, smem, st, (const T*)x, (const T*)res, (const T*)w, (const T*)b,  \
                           (T*)y, (T*)hout, rstd, mean, rows, cols, chunk, eps, unit_offset);                                            \
   } while (0)
 #define NORM_STAGED_RS(L_)                                   \
   do {                                                       \
-    if (cols <= 768) NORM_STAGED(L_, 8);                     \
-    else if (cols <= 1536) NORM_STAGED(L_, 4);               \
-    else NORM_STAGED(L_, 2);                                 \
+    if (cols <= 768) NORM_STAGED(L_, 8, 3);                  \
+    else if (cols <= 1024) NORM_STAGED(L_, 8, 4);            \
+    else NORM_STAGED(L_, 2, 3);                              \
   } while (0)
     const auto run = [&](auto zero) -> int {
       typedef decltype(zero) T;
