@@ -10,6 +10,7 @@ oracle for tests.  The library attention is reached only for other dtypes or whe
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -66,6 +67,7 @@ def attention_fwd_kernel(qkv, bsz, seq, hq, hkv, hd, scale, softcap: float = 0.0
     return out, lse2
 
 
+@functools.lru_cache(maxsize=4096)
 def _flash_ds_bytes(bsz, seq, hq, hkv, hd) -> int:
     """Bytes of scratch for which the backward keeps dS between its kernels, or 0."""
     out = ctypes.c_int64()
@@ -77,15 +79,17 @@ def attention_bwd_kernel(dout, qkv, out, lse2, bsz, seq, hq, hkv, hd, scale, sof
     """tcgen05 backward: gradient of the fused qkv buffer (no atomics)."""
     dout = dout if (dout.is_contiguous() and dout.data_ptr() % 16 == 0) else dout.contiguous()
     dqkv = torch.empty_like(qkv)
-    stat = torch.empty(2, *lse2.shape, dtype=torch.float32, device=qkv.device)
     if hd <= 128 and softcap <= 0:
-        need = _flash_ds_bytes(bsz, seq, hq, hkv, hd)
-        ds = torch.empty(need, dtype=torch.uint8, device=qkv.device) if need else None
-        rc = _native.lib().zen_flash_bwd(_native.ptr(qkv), _native.ptr(out), _native.ptr(dout), _native.ptr(lse2), _native.ptr(stat),
-                                         _native.ptr(dqkv), bsz, seq, hq, hkv, hd, qkv.stride(0), out.stride(0), dqkv.stride(0),
-                                         float(scale), _native.ptr(ds), _native.stream_ptr())
-        _native.check(rc, "zen_flash_bwd")
+        need, nstat = _flash_ds_bytes(bsz, seq, hq, hkv, hd), 2 * lse2.numel()
+        scratch = torch.empty(nstat + need // 4, dtype=torch.float32, device=qkv.device)       # row statistics (a multiple of 1 KB), dS
+        stat = scratch.data_ptr()
+        rc = _native.lib().zen_flash_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse2.data_ptr(), stat, dqkv.data_ptr(), bsz, seq, hq,
+                                         hkv, hd, qkv.stride(0), out.stride(0), dqkv.stride(0), float(scale), stat + 4 * nstat if need else 0,
+                                         _native.stream_ptr())
+        if rc:
+            _native.check(rc, "zen_flash_bwd")
         return dqkv
+    stat = torch.empty(2, *lse2.shape, dtype=torch.float32, device=qkv.device)
     # few KV heads (MQA / GQA): the query heads of a group are shared out over several CTA pairs
     hsplit, part = _native.lib().zen_attn_hsplit(bsz, seq, hq, hkv, hd), None
     if hsplit > 1:
