@@ -742,15 +742,17 @@ int g_tail_min_kb = 1;             // fewest 64-wide K blocks for which the tile
 // The tiles of the last, partly filled wave of clusters run as two units each when both units of all of them fit in that wave.
 // Halves of 128 columns need nothing from each other and sum every element in the order of a whole tile, but each reads its
 // rows of A again, and what bounds a tile is what its SMs draw from L2: three quarters of a tile's time.  K halves take half
-// of it, and about 4 us to exchange half an accumulator each through memory; they pay from K = 4096 on (and need the TMA store and
-// a workspace).  us, K halves / column halves: the 108 tiles of a GPT-2 layer's weight gradients, K = 8192, 75 / 80;
-// 8192 x 768 x 3072 40.9 / 40.9; 8192 x 768 x 2304 34.7 / 32.7; 8192 x 3072 x 768 38.8 (whole) / 36.8; 700 x 2304 x 9216 without
-// a workspace 55.1 (whole) / 47.0.
-constexpr int TAIL_K_MIN_KB = 64;
+// of it, and about 4 us to exchange half an accumulator each through memory (and need the TMA store and a workspace).  us, K halves /
+// column halves: the 108 tiles of a GPT-2 layer's weight gradients, K = 8192, 75 / 80; 8192 x 768 x 3072 40.9 / 40.9;
+// 8192 x 768 x 2304 34.7 / 32.7; 8192 x 3072 x 768 38.8 (whole) / 36.8; 700 x 2304 x 9216 without a workspace 55.1 (whole) / 47.0.
+// By time the line would lie near K = 4096.  It lies at 1024, where the sum of a tile's two halves has been taken since K was
+// first cut, and not for outputs of one round, which split_k_choice cuts where that pays: another order of summation in one tile of ten moves the logits of a four-layer Llama by up to 1.2 % (2 x 600 and 1 x
+// 2048 tokens), as much as any rounding there, and scores should not change by that for 2 us.
+constexpr int TAIL_K_MIN_KB = 16;
 static void cut_tail(GemmGroup& g, int min_kb) {
   const int clusters = zen_tmap::sm_count() / 2, rem = g.num_tiles % clusters;
   g.tail = g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && 2 * rem <= clusters ? rem : 0;
-  g.tail_k = g.tail > 0 && min_kb >= TAIL_K_MIN_KB && g.ws && g.counters;
+  g.tail_k = g.tail > 0 && g.num_tiles > clusters && min_kb >= TAIL_K_MIN_KB && g.ws && g.counters;
   for (int i = 0; i < g.n && g.tail_k; ++i) {
     const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
     if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
