@@ -83,8 +83,44 @@ struct GemmGroup {
   float* target;
   int part_ld;
   float cap;
+  // Rows beyond the last whole 256 (one product, K-major A, whole tiles): see narrow_rows.  `narrow` columns of the transposed tiles, a
+  // multiple of 32; ta_narrow: these rows of A in boxes of half as many
+  CUtensorMap ta_narrow;
+  int narrow, narrow_first;
 };
-enum Epilogue { EPI_STORE, EPI_ACT, EPI_LOSS, EPI_LOSS_CAP };
+enum Epilogue { EPI_STORE, EPI_ACT, EPI_LOSS, EPI_LOSS_CAP, EPI_STORE_NARROW };
+
+// The units of one cluster, in order.  With narrow tiles (one per tile column, index num_tiles + column): whole tiles go round;
+// narrow ones go to the clusters that have one whole tile less, narrow_first times, then round from the first of these.  Both
+// lists are merged by column, so that the weights of a column are read at about the same time.
+template <bool NARROW>
+struct Units {
+  int at, step, end;
+  __device__ Units(const GemmGroup&, int cluster, int clusters, int num_units) : at(cluster), step(clusters), end(num_units) {}
+  __device__ __forceinline__ bool more() const { return at < end; }
+  __device__ __forceinline__ int unit() const { return at; }
+  __device__ __forceinline__ void advance() { at += step; }
+};
+template <>
+struct Units<true> {
+  int whole, nar, step, tiles, cols, per_col, idle, first, turn;
+  __device__ Units(const GemmGroup& g, int cluster, int clusters, int)
+      : whole(cluster), step(clusters), tiles(g.num_tiles), cols(g.pr[0].num_n_tiles), per_col(g.pr[0].num_m_pairs) {
+    const int rem = tiles % clusters;
+    idle = clusters - rem;
+    first = idle * (rem ? g.narrow_first : 0);
+    turn = cluster >= rem ? cluster - rem : cluster - rem + clusters;       // place in the order of the narrow tiles
+    nar = turn < idle && first > 0 ? turn : first + turn;
+  }
+  __device__ __forceinline__ bool take_narrow() const { return nar < cols && (whole >= tiles || nar <= whole / per_col); }
+  __device__ __forceinline__ bool more() const { return whole < tiles || nar < cols; }
+  __device__ __forceinline__ int unit() const { return take_narrow() ? tiles + nar : whole; }
+  __device__ __forceinline__ void advance() {
+    if (!take_narrow()) whole += step;
+    else if (nar < first) nar = nar + idle < first ? nar + idle : first + turn;
+    else nar += step;
+  }
+};
 
 // One unit of work of a cluster: an output tile, one K slice of it, or half of its columns.
 struct Unit {
@@ -282,6 +318,23 @@ __device__ __forceinline__ void epilogue_loss(const GemmGroup& gg, const GemmPro
   if (row < p.M) gg.part[(size_t)((n0 + cb_lo * 64) / 128) * gg.part_ld + row] = make_float2(m, s);
 }
 
+// A transposed tile: the lane's column of the output, `narrow` rows of it in the columns of tensor memory.
+template <int HALVES>
+__device__ __forceinline__ void store_narrow(const GemmGroup& gg, uint32_t taddr, int col, int half) {
+  const GemmProblem& p = gg.pr[0];
+  const float bias = p.bias && col < p.N ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col]) : 0.f;
+#pragma unroll 1
+  for (int ch = half; ch < gg.narrow / 32; ch += HALVES) {
+    uint32_t r[32];
+    tmem_ld32(taddr + ch * 32, r);
+    const int row = p.num_m_pairs * 256 + ch * 32;
+    __nv_bfloat16* c = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row * p.ldc + col;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (row + i < p.M && col < p.N) c[(size_t)i * p.ldc] = __float2bfloat16_rn(__uint_as_float(r[i]) + bias);
+  }
+}
+
 template <bool A_MN, bool B_MN, int BN2, int EW, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + EW * 32, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
@@ -296,6 +349,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
   uint64_t* tempty = bars + 2 * STAGES2 + 2;   // [2]         used on the leader, one arrival per epilogue warp of the pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES2 + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  constexpr bool NARROW = EPI == EPI_STORE_NARROW;
   constexpr uint32_t IDESC = make_idesc(256, BN2, A_MN, B_MN), IDESC_HALF = make_idesc(256, BN2 / 2, A_MN, B_MN);
   constexpr int A_BYTES = BM2 * BK2 * 2;
 
@@ -324,8 +378,28 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       // ---------------------------------------------------------------- TMA producer (both CTAs)
       uint32_t it = 0;
       bool ok = true;
-      for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters) {
-        const Unit u = decode_unit(gg, unit);
+      for (Units<NARROW> w(gg, cluster_id, num_clusters, num_units); w.more() && ok; w.advance()) {
+        if (NARROW && w.unit() >= num_tiles) {
+          const GemmProblem& p = gg.pr[0];
+          const int n0 = (w.unit() - num_tiles) * 256 + (int)cta * BM2, m0 = p.num_m_pairs * 256 + (int)cta * (gg.narrow / 2);
+          const uint32_t bytes = 2 * (A_BYTES + gg.narrow / 2 * (BK2 * 2));
+          for (int kb = 0; kb < gg.kb_per_split; ++kb, ++it) {
+            const int s = it % STAGES2;
+            if (!mbar_wait(&empty[s], ((it / STAGES2) & 1) ^ 1, abort_flag, 1, &g_gemm2_error)) { ok = false; break; }
+            unsigned char* sa = smem + s * STAGE_BYTES2;
+            if (cta == 0) mbar_expect_tx(&full[s], bytes);
+            const int k0 = kb * BK2;
+            if (!B_MN) {
+              tma_load_2d_pair(sa, &p.tb, &full[s], k0, n0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BM2 / 64; ++j) tma_load_2d_pair(sa + j * 8192, &p.tb, &full[s], n0 + 64 * j, k0);
+            }
+            tma_load_2d_pair(sa + A_BYTES, &gg.ta_narrow, &full[s], k0, m0);
+          }
+          continue;
+        }
+        const Unit u = decode_unit(gg, w.unit());
         const GemmProblem& p = gg.pr[u.pi];
         int tm, tn;
         tile_coords(p, u.lt, tm, tn);
@@ -363,14 +437,15 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       const uint32_t tmem_u = uniform(tmem_base);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
-      for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++tcount) {
+      for (Units<NARROW> w(gg, cluster_id, num_clusters, num_units); w.more() && ok; w.advance(), ++tcount) {
         const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
         if (!mbar_wait(&tempty[acc], aph ^ 1, abort_flag, 2, &g_gemm2_error)) { ok = false; break; }
         fence_after();
         const uint32_t d_tmem = tmem_u + acc * BN2;
-        const Unit u = decode_unit(gg, unit);
+        const bool narrow = NARROW && w.unit() >= num_tiles;
+        const Unit u = decode_unit(gg, narrow ? 0 : w.unit());           // (whole tiles share their blocks of K)
         const int kb0 = u.kb0, kb1 = u.kb1;
-        const uint32_t idesc = u.part ? IDESC_HALF : IDESC;
+        const uint32_t idesc = narrow ? make_idesc(256, gg.narrow, B_MN, A_MN) : u.part ? IDESC_HALF : IDESC;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES2;
           const uint32_t ph = (it / STAGES2) & 1;
@@ -378,13 +453,14 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
           fence_after();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES2);
           const uint32_t sb = sa + A_BYTES;
-          const uint64_t adesc = A_MN ? make_desc(sa, 8192, 1024) : make_desc(sa, 16, 1024);
-          const uint64_t bdesc = B_MN ? make_desc(sb, 8192, 1024) : make_desc(sb, 16, 1024);
+          const bool a_mn = NARROW && narrow ? B_MN : A_MN, b_mn = NARROW && narrow ? A_MN : B_MN;
+          const uint64_t adesc = a_mn ? make_desc(sa, 8192, 1024) : make_desc(sa, 16, 1024);
+          const uint64_t bdesc = b_mn ? make_desc(sb, 8192, 1024) : make_desc(sb, 16, 1024);
           if (leader) {
 #pragma unroll
             for (int j = 0; j < BK2 / 16; ++j) {
-              const uint64_t astep = (uint64_t)((A_MN ? j * 2048 : j * 32) >> 4);
-              const uint64_t bstep = (uint64_t)((B_MN ? j * 2048 : j * 32) >> 4);
+              const uint64_t astep = (uint64_t)((a_mn ? j * 2048 : j * 32) >> 4);
+              const uint64_t bstep = (uint64_t)((b_mn ? j * 2048 : j * 32) >> 4);
               umma_bf16_pair(d_tmem, adesc + astep, bdesc + bstep, idesc, (kb != kb0 || j != 0) ? 1u : 0u);
             }
             umma_commit_pair(&empty[s]);
@@ -402,8 +478,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
     uint32_t buf = 0;
     uint32_t tcount = 0;
     bool ok = true;
-    for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++tcount) {
-      const Unit u = decode_unit(gg, unit);
+    for (Units<NARROW> w(gg, cluster_id, num_clusters, num_units); w.more() && ok; w.advance(), ++tcount) {
+      if (NARROW && w.unit() >= num_tiles) {
+        if (!mbar_wait(&tfull[tcount & 1], (tcount >> 1) & 1, abort_flag, 4, &g_gemm2_error)) { ok = false; break; }
+        fence_after();
+        store_narrow<HALVES>(gg, tmem_base + ((uint32_t)(grp * 32) << 16) + (tcount & 1) * BN2,
+                             (w.unit() - num_tiles) * 256 + (int)cta * BM2 + grp * 32 + lane, half);
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_leader(&tempty[tcount & 1]);
+        continue;
+      }
+      const Unit u = decode_unit(gg, w.unit());
       const GemmProblem& p = gg.pr[u.pi];
       const int tile = u.tile, ks = u.ks;
       int tm, tn;
@@ -420,7 +506,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ GemmGroup gg) {
       fence_after();
       const int row = m0 + grp * 32 + lane;
       const uint32_t taddr0 = tmem_base + ((uint32_t)(grp * 32) << 16) + acc * BN2;
-      if constexpr (EPI != EPI_STORE) {
+      if constexpr (EPI != EPI_STORE && EPI != EPI_STORE_NARROW) {
         if constexpr (EPI == EPI_ACT) epilogue_act<EW>(gg, p, stg, buf, taddr0, n0, m0 + grp * 32, cb_lo, cb_hi, bias, lane);
         else epilogue_loss<EW, EPI == EPI_LOSS_CAP>(gg, p, stg, buf, taddr0, n0, m0 + grp * 32, cb_lo, cb_hi, lane);
         fence_before();
@@ -658,7 +744,7 @@ int launch2_as(const GemmGroup& g, cudaStream_t st) {
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  const int units = g.tail ? g.num_tiles + g.tail : g.num_tiles * g.splits;
+  const int units = EPI == EPI_STORE_NARROW ? g.num_tiles + g.pr[0].num_n_tiles : g.tail ? g.num_tiles + g.tail : g.num_tiles * g.splits;
   int clusters = zen_tmap::sm_count() / 2;
   if (units < clusters) clusters = units;
   zen_pdl::launch(gemm_bf16_2cta_kernel<A_MN, B_MN, BN2, EW, EPI>, clusters * 2, 64 + EW * 32, pair_smem_bytes<BN2>(), st, g);
@@ -758,6 +844,41 @@ static void cut_tail(GemmGroup& g, int min_kb) {
     if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
   }
 }
+// Rows beyond the last whole 256: up to 128 of them as transposed tiles, 256 columns of the output (rows of B) as the
+// rows of the MMA and these rows of A, rounded up to 32, as its columns.  Such a tile draws half as much from L2 and takes about
+// 0.78 of a whole one's time (its stages are as many, and half as full).  Taken where the rounds, so weighed, come out shorter by
+// 3 %; the clusters that would be idle in the last round take up to three.  In practice that is an output many rounds long: us, whole tiles /
+// with transposed ones, 777 x 128256 x 3072 494 / 454, 1300 x 16384 x 2048 71.7 / 68.6, 300 x 50257 x 768 41.0 / 40.0; but
+// 777 x 16384 x 3072 70.6 / 73.3, 2100 x 2304 x 768 19.0 / 20.0 and 3100 x 7680 x 2560 86 / 89, which the weights leave whole.
+static bool narrow_rows(GemmGroup& g, const void* A, int lda, int min_kb) {
+  GemmProblem& p = g.pr[0];
+  const int clusters = zen_tmap::sm_count() / 2, rows = p.M % 256;
+  if (g_tail_min_kb <= 0 || min_kb < g_tail_min_kb || p.M < 256 || rows == 0 || rows > 128 || !p.tma_store) return false;
+  if (g.tail_k && p.N <= 32768) return false;           // the order of summation, see cut_tail; wider ones are logits, and no product follows
+  const int width = (rows + 31) / 32 * 32, cols = p.num_n_tiles, tiles = (p.num_m_pairs - 1) * cols;
+  const double cost = 0.75 + width / 1024.0;
+  const int now_rem = g.num_tiles % clusters;
+  const double now = g.num_tiles / clusters + (now_rem == 0 ? 0.0 : g.tail ? (g.tail_k ? 0.6 : 0.75) : 1.0);
+  const int rounds = tiles / clusters, rem = tiles % clusters, idle = clusters - rem;
+  double best = now * 0.97;
+  int first = -1;
+  for (int k = 0; k <= (rem ? 3 : 0); ++k) {
+    const int head = k * idle < cols ? k * idle : cols, rest = cols - head, after = rest > idle ? rest - idle : 0;
+    const double early = rounds + ((head + idle - 1) / idle + (rest + clusters - 1) / clusters) * cost;
+    const double late = rounds + (rem ? 1 : 0) + (after + clusters - 1) / clusters * cost;
+    const double t = early > late ? early : late;
+    if (t < best) { best = t; first = k; }
+  }
+  if (first < 0) return false;
+  if (zen_tmap::get(A, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda, 64, (uint32_t)(width / 2), &g.ta_narrow)) return false;
+  g.narrow = width;
+  g.narrow_first = first;
+  --p.num_m_pairs;
+  p.group_m = pick_group_m(p.M, p.N, p.K, p.num_m_pairs);
+  g.num_tiles = tiles;
+  g.tail = g.tail_k = 0;
+  return true;
+}
 // Whether a caller's workspace holds the halves of the tiles that a last wave may have: half of the clusters.
 static bool tail_workspace(const float* ws, uint64_t ws_floats, const int* counters, int n_counters) {
   const int most = zen_tmap::sm_count() / 4;
@@ -833,6 +954,10 @@ int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void*
   if (splits == 1 && bn == 256) {
     if (!tail_workspace(ws, ws_floats, counters, n_counters)) g.ws = nullptr;
     cut_tail(g, nkb);
+    if (!a_mn && narrow_rows(g, A, lda, nkb)) {
+      if (bias) return b_mn ? launch2_as<false, true, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
+      return b_mn ? launch2_as<false, true, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
+    }
   }
   return launch2_layout(g, a_mn, b_mn, bn, (cudaStream_t)stream);
 }

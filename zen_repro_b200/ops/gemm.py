@@ -178,9 +178,9 @@ def _plan(M: int, N: int, K: int, bn: int):
 
 @functools.lru_cache(maxsize=4096)
 def plan_forward_only(M: int, N: int, K: int):
-    """The plan for the products of a block that no backward will follow (scoring, validation).  K is cut into two at most, from
-    4096 on and in two places: by ``split_k_choice`` (from 256 rows, tiles for at most half of the CTA pairs), and in the last
-    round of an output of at least 512 rows whose tiles fill 60 % of the pairs' rounds.  Never among the clusters of
+    """The plan for the products of a block that no backward will follow (scoring, validation).  K is cut into two at most, in two
+    places: by ``split_k_choice`` (from 256 rows, K from 4096, tiles for at most half of the CTA pairs), and, K from 1024, in the
+    last round of an output of at least 512 rows whose tiles fill 60 % of the pairs' rounds.  Never among the clusters of
     csrc/gemm_splitk.cu, nor in the last round of smaller outputs, which a third element 1 marks.
 
     So the order of summation is that of the products as they were before clusters shared K, but it is not the same at every
