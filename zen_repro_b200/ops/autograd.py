@@ -325,7 +325,10 @@ class LMHeadLossFn(torch.autograd.Function):
         for s in range(0, T, chunk_tokens):
             e = min(T, s + chunk_tokens)
             hs, ls = h2[s:e], lab[s:e]
-            fused = in_kernel and G.makes_loss_statistics(hs, weight)
+            # Statistics from the product's epilogue: one launch and two scratch tensors more, 16 us of host time, against a pass over
+            # the logits (in training; in validation the writing of them too).  476 rows of 50 257: 26 -> 19 us of kernels, a step that
+            # the host bounds; 8192 rows: 397 -> 294.
+            fused = in_kernel and (not train or e - s >= 1024) and G.makes_loss_statistics(hs, weight)
             logits = torch.empty(e - s, vpad, dtype=h2.dtype, device=h2.device)[:, :V] if train or not fused else None
             if fused:
                 ls = E._index(ls, hs)
