@@ -85,17 +85,17 @@ def test_loss_function_equals_the_separate_passes(rows, softcap, monkeypatch):
     labels[::5] = -100
 
     def run():
-        loss = lm_head_loss(h, w, labels, chunk_tokens=512, unit_grad=False, softcap=softcap)
+        loss = lm_head_loss(h, w, labels, chunk_tokens=1024, unit_grad=False, softcap=softcap)
         gh, gw = torch.autograd.grad(loss, (h, w))
         with torch.no_grad():
-            quiet = lm_head_loss(h, w, labels, chunk_tokens=512, softcap=softcap)
+            quiet = lm_head_loss(h, w, labels, chunk_tokens=1024, softcap=softcap)
         return loss.detach(), quiet, gh, gw
 
     ran = []
     real = G.gemm_nt_loss
     monkeypatch.setattr(G, "gemm_nt_loss", lambda *a, **k: ran.append(1) or real(*a, **k))
     one = run()
-    assert bool(ran) == G.makes_loss_statistics(h.detach()[:512], w.detach())
+    assert bool(ran) == G.makes_loss_statistics(h.detach()[:1024], w.detach())
     monkeypatch.setattr(G, "makes_loss_statistics", lambda a, b: False)
     two = run()
     assert abs(one[0] - two[0]) <= 1e-5 * two[0] and abs(one[1] - one[0]) <= 1e-6 * one[0]
