@@ -58,7 +58,7 @@ struct ZenSparseCtx {
   const uint32_t* epoch_dev;  // optional: call counter on the device (zen_sparse_epoch_bump); overrides `epoch`
   char* mc;                   // optional: multicast alias of the symmetric region (stores reach every rank)
   uint32_t k1_density_ppm;    // nonzeros per million elements that the plan was sized for (0 = unknown)
-  uint32_t pad0;
+  uint32_t seg_words;         // what `seg` holds
 };
 
 // Contexts, inputs and outputs of the ranks that one launch works for: one, or all ranks of a call that runs on one device
@@ -1772,10 +1772,24 @@ static int launch_sort(const ZenSparseBatch<NB>& b, int n, int deterministic, in
   start<NB>(small_call(c, n), zen_record_sort_kernel<NB>, batch_grid<NB>(grid, n), SB_SORT_THREADS, 0, st, b, deterministic, by_index);
   return (int)cudaGetLastError();
 }
+
+// Words of `seg` for outputs of `numel` elements by method 1 in buckets; -1 where they are not taken.
+static int64_t index_bucket_words(uint64_t numel, uint32_t cap_rec, int nranks) {
+  if (numel > IB_MAX || numel < SB_MIN_SLOTS) return -1;
+  const SbShape sh = sb_shape((uint32_t)numel, cap_rec, nranks);
+  return sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 0;
+}
+// Method 1 in buckets: only where the plan's `seg` holds the runs (a plan that was not made for method 1 may hold fewer).
+static bool by_buckets(const ZenSparseCtx& c) {
+  const int64_t words = index_bucket_words(c.numel, c.cap_rec, c.nranks);
+  return words >= 0 && words <= (int64_t)c.seg_words;
+}
 template <typename T, int NB>
 static int launch_scatter(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   const ZenSparseCtx& c = b.c[0];
-  if (c.numel <= IB_MAX && c.numel >= SB_MIN_SLOTS) {
+  bool buckets = true;
+  for (int i = 0; i < n; ++i) buckets = buckets && by_buckets(b.c[i]);
+  if (buckets) {
     const SbShape sh = sb_shape((uint32_t)c.numel, c.cap_rec, c.nranks);
     int rc = 0;
     if (sh.sorted && (rc = launch_sort<NB>(b, n, 0, 1, st))) return rc;
@@ -1844,9 +1858,9 @@ int zen_partition_push(const ZenSparseCtx* c, const void* g, const float* thr, i
 // whether `acc` and `bitmap` are used.
 // method1_numel: the elements of the output where method 1 is to be served, else 0.
 int zen_sparse_scratch(uint32_t nslots, uint32_t cap_rec, int nranks, uint32_t method1_numel, int64_t* out) {
-  const SbShape sh = sb_shape(nslots, cap_rec, nranks), s1 = sb_shape(method1_numel, cap_rec, nranks);
+  const SbShape sh = sb_shape(nslots, cap_rec, nranks);
   out[0] = sh.on && sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 1;
-  const int64_t m1 = method1_numel <= IB_MAX && method1_numel >= SB_MIN_SLOTS && s1.sorted ? (int64_t)s1.nbuckets * s1.tiles * nranks : 1;
+  const int64_t m1 = index_bucket_words(method1_numel, cap_rec, nranks);
   if (m1 > out[0]) out[0] = m1;
   out[1] = sh.on ? 0 : 1;
   return 0;
@@ -1878,7 +1892,10 @@ int zen_densify(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
   return rc;
 }
 
-// Method 1 consumer: every source added in rank order, in buckets or (above IB_MAX elements) into the cleared `out`.
+// Whether method 1 takes its buckets for this context; else it clears the output and scatters.
+int zen_sparse_method1_buckets(const ZenSparseCtx* c) { return by_buckets(*c) ? 1 : 0; }
+
+// Method 1 consumer: every source added in rank order, in buckets or into the cleared `out`.
 int zen_scatter_sources(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
   int rc = 0;
   DISPATCH_DTYPE(dtype, rc = (launch_scatter<T, 1>(one_rank(c, nullptr, out), 1, (cudaStream_t)stream)));

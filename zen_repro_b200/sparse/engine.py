@@ -52,7 +52,7 @@ class _Ctx(ctypes.Structure):
         ("numel", ctypes.c_uint64), ("nslots", ctypes.c_uint32), ("nwords", ctypes.c_uint32),
         ("perm", _Perm),
         ("epoch_dev", ctypes.c_void_p), ("mc", ctypes.c_void_p),
-        ("k1_density_ppm", ctypes.c_uint32), ("pad0", ctypes.c_uint32),
+        ("k1_density_ppm", ctypes.c_uint32), ("seg_words", ctypes.c_uint32),
     ]
 
 
@@ -148,7 +148,8 @@ class SparseRank:
                      "cap_rec", "cap_g", "g_idx_words", "nchunks", "nwords"):
             setattr(c, name, getattr(plan, name))
         c.acc, c.bitmap = self.acc.data_ptr(), self.bitmap.data_ptr()
-        c.seg, c.cursors, c.status = self.seg.data_ptr(), self.cursors.data_ptr(), self.status_t.data_ptr()
+        c.seg, c.seg_words = self.seg.data_ptr(), self.seg.numel()
+        c.cursors, c.status = self.cursors.data_ptr(), self.status_t.data_ptr()
         c.numel, c.nslots = plan.numel, plan.nslots
         c.perm = perm_struct(plan.perm)
         c.k1_density_ppm = max(1, min(1_000_000, int(plan.max_density * 1e6)))
