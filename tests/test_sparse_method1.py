@@ -1,4 +1,5 @@
-"""Method 1 by plans that were not made for it: its buckets are taken only where the plan's scratch holds the runs of its records."""
+"""Method 1 takes its buckets only where the plan's scratch holds the runs of its records (plans that were not made for it) and where
+the output takes 16-byte stores."""
 import ctypes
 
 import pytest
@@ -31,7 +32,8 @@ def test_buckets_only_where_the_scratch_holds_them(numel, P, density, methods):
     used = tiles * P * buckets if buckets > 1 and plan.cap_rec * P > 65_536 else 0
     for words in (_words(plan, 1 in methods), used, max(used - 1, 0), 0):
         c.seg_words = words
-        assert _native.lib().zen_sparse_method1_buckets(ctypes.byref(c)) == (16_384 <= numel <= 524_288 and used <= words)
+        for addr in (0x7f0000000000, 0x7f0000000002, 0x7f0000000004, 0x7f0000000008):
+            assert _native.lib().zen_sparse_method1_buckets(ctypes.byref(c), addr) == (16_384 <= numel <= 524_288 and used <= words and addr % 16 == 0)
     if 1 in methods and 16_384 <= numel <= 524_288:
         assert _words(plan, True) >= used
 
@@ -59,3 +61,28 @@ def test_sums_and_the_words_behind_the_scratch(numel, P, density, methods, dtype
         assert eng.status() == [0] * P
         assert all(torch.equal(o, want) for o in outs)
         assert all(bool((w == 0x5AFEC0DE).all()) for w in guarded)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("numel,P", [(20_000, 2), (524_288, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_stage_by_stage_into_any_element(numel, P, dtype, shift):
+    """The stages launched one by one write to outputs that start at any element; what lies around them stays."""
+    from zen_repro_b200.sparse.engine import VirtualSparseAllReduce
+
+    eng = VirtualSparseAllReduce(numel, P, max_density=0.1, methods=(1,))
+    g = torch.Generator("cuda").manual_seed(shift)
+    xs = [(torch.randn(numel, device="cuda", generator=g) * (torch.rand(numel, device="cuda", generator=g) < 0.05)).to(dtype) for _ in range(P)]
+    want = torch.zeros(numel, device="cuda", dtype=dtype)
+    for x in xs:
+        want = (want.float() + x.float()).to(dtype)
+    eng.epoch += 1
+    for r, x in zip(eng.ranks, xs):
+        r.partition_push(x, eng.epoch, broadcast=True)
+    for r in eng.ranks:
+        buf = torch.full((numel + 16,), 7.0, device="cuda", dtype=dtype)
+        r.scatter_sources(buf[shift:shift + numel], eng.epoch)
+        assert torch.equal(buf[shift:shift + numel], want)
+        assert bool((buf[:shift] == 7).all()) and bool((buf[shift + numel:] == 7).all())
+    assert eng.status() == [0] * P

@@ -1779,16 +1779,17 @@ static int64_t index_bucket_words(uint64_t numel, uint32_t cap_rec, int nranks) 
   const SbShape sh = sb_shape((uint32_t)numel, cap_rec, nranks);
   return sh.sorted ? (int64_t)sh.nbuckets * sh.tiles * nranks : 0;
 }
-// Method 1 in buckets: only where the plan's `seg` holds the runs (a plan that was not made for method 1 may hold fewer).
-static bool by_buckets(const ZenSparseCtx& c) {
+// Method 1 in buckets: only where the plan's `seg` holds the runs (a plan that was not made for method 1 may hold fewer) and the
+// output takes 16-byte stores.
+static bool by_buckets(const ZenSparseCtx& c, const void* out) {
   const int64_t words = index_bucket_words(c.numel, c.cap_rec, c.nranks);
-  return words >= 0 && words <= (int64_t)c.seg_words;
+  return words >= 0 && words <= (int64_t)c.seg_words && reinterpret_cast<uintptr_t>(out) % 16 == 0;
 }
 template <typename T, int NB>
 static int launch_scatter(const ZenSparseBatch<NB>& b, int n, cudaStream_t st) {
   const ZenSparseCtx& c = b.c[0];
   bool buckets = true;
-  for (int i = 0; i < n; ++i) buckets = buckets && by_buckets(b.c[i]);
+  for (int i = 0; i < n; ++i) buckets = buckets && by_buckets(b.c[i], b.out[i]);
   if (buckets) {
     const SbShape sh = sb_shape((uint32_t)c.numel, c.cap_rec, c.nranks);
     int rc = 0;
@@ -1892,8 +1893,8 @@ int zen_densify(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
   return rc;
 }
 
-// Whether method 1 takes its buckets for this context; else it clears the output and scatters.
-int zen_sparse_method1_buckets(const ZenSparseCtx* c) { return by_buckets(*c) ? 1 : 0; }
+// Whether method 1 takes its buckets for this context and output; else it clears the output and scatters.
+int zen_sparse_method1_buckets(const ZenSparseCtx* c, const void* out) { return by_buckets(*c, out) ? 1 : 0; }
 
 // Method 1 consumer: every source added in rank order, in buckets or into the cleared `out`.
 int zen_scatter_sources(const ZenSparseCtx* c, void* out, int dtype, void* stream) {
