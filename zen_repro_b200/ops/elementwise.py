@@ -587,3 +587,8 @@ def xent_apply_(logits, labels, lse, valid_cols: int, vocab_start: int, grad_sca
                                       _native.stream_ptr())
     _native.check(rc, "zen_xent_apply")
     return logits
+
+
+def norm_error() -> int:
+    """Code of the staged norm kernel that gave up waiting for its rows, since the last call (0 = none)."""
+    return int(_native.lib().zen_norm_error())

@@ -249,17 +249,20 @@ class Trainer:
     def check_health(self, raise_on_error: bool = True) -> dict:
         """Read (and clear) the status words that the kernels set instead of faulting: capacity overflow or an expired
         wait in the sparse engines (element and row granule) and in the fused tensor-parallel GEMMs, and the error
-        codes of the tcgen05 GEMM / attention kernels.  Synchronises the device; meant for every N-th step and the end
-        of a run, not for the hot loop.  Non-zero entries mean that a step used incomplete data."""
+        codes of the tcgen05 GEMM / attention kernels and of the staged norms.  Synchronises the device; meant for
+        every N-th step and the end of a run, not for the hot loop.  Non-zero entries mean that a step used incomplete
+        data."""
         out = {}
         if self.device.type != "cuda":
             return out
         from .ops import attention as A
+        from .ops import elementwise as E
         from .ops import gemm as G
 
         torch.cuda.synchronize()
         out["gemm"] = int(G.gemm_error())
         out["attention"] = int(A.attention_error())
+        out["norm"] = E.norm_error()
         emb = getattr(self.model.module, "embedding_sync", None)
         if emb is not None:
             out["embedding_rows"] = int(emb.check())
