@@ -500,6 +500,27 @@ zen_partition_push_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, const f
   }
 }
 
+// Records received from sources [src_begin, src_end), s_n[source - src_begin], after a bounded wait for each one's mail; one thread per
+// source.  Returns the calling thread's part of the status.  Every CTA waits for itself and one may give up on a mail that another
+// still saw, so every CTA has to report what it got: its records are missing from the result.
+__device__ __forceinline__ uint32_t records_wait(const ZenSparseCtx& c, uint32_t epoch, int src_begin, int src_end, uint32_t* s_n) {
+  uint32_t status = 0;
+  if ((int)threadIdx.x < src_end - src_begin) {
+    const ZenMail* mail = zen_rec_mail(c, c.rank, src_begin + threadIdx.x, epoch);
+    uint32_t n = 0;
+    if (zen_wait_epoch(&mail->epoch, epoch, c.wait_ns)) {
+      // count and info were written before the epoch's release store: plain loads after the acquire above see them
+      n = min(*reinterpret_cast<const volatile uint32_t*>(&mail->count), c.cap_rec);
+      if (*reinterpret_cast<const volatile uint32_t*>(&mail->info) & 1u) status = ZEN_PEER_OVERFLOW;
+    } else {
+      status = ZEN_TIMEOUT;
+    }
+    s_n[threadIdx.x] = n;
+  }
+  __syncthreads();
+  return status;
+}
+
 // ---------------------------------------------------------------------------------------------
 // K2: owner-side reduce of sources [src_begin, src_end).  One launch over all sources is the fast
 // mode; one launch per source gives a fixed accumulation order.  The waits on the sources' mailboxes
@@ -513,27 +534,9 @@ zen_owner_reduce_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int src_b
   __shared__ ZenSparseCtx s_ctx;
   const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
   __shared__ uint32_t s_n[ZEN_MAX_RANKS];
-  __shared__ uint32_t s_flag[ZEN_MAX_RANKS];
   const uint32_t epoch = zen_epoch(c);
   const int ns = src_end - src_begin;
-  if ((int)threadIdx.x < ns) {
-    const int s = src_begin + threadIdx.x;
-    const ZenMail* mail = zen_rec_mail(c, c.rank, s, epoch);
-    uint32_t n = 0, fl = 0;
-    if (zen_wait_epoch(&mail->epoch, epoch, c.wait_ns)) {
-      // count and info were written before the epoch's release store: plain loads after the acquire above see them
-      const uint32_t cnt = *reinterpret_cast<const volatile uint32_t*>(&mail->count);
-      const uint32_t info = *reinterpret_cast<const volatile uint32_t*>(&mail->info);
-      n = min(cnt, c.cap_rec);
-      if (info & 1u) fl = ZEN_PEER_OVERFLOW;
-    } else {
-      fl = ZEN_TIMEOUT;
-    }
-    s_n[threadIdx.x] = n;
-    s_flag[threadIdx.x] = fl;
-  }
-  __syncthreads();
-  uint32_t local_status = 0;
+  uint32_t local_status = records_wait(c, epoch, src_begin, src_end, s_n);
   // With many records the occupancy bitmap is not kept: the gather then reads every slot anyway and takes "touched" to mean
   // "sum is not zero" (a slot whose sum is exactly zero need not travel), which halves the number of atomics here.  At 24 % of
   // the slots reduce + gather take the same time both ways (16 M x 8 bf16: 126 us), at 20 % the scan costs 6 us of 33 more (4 M x 2
@@ -541,10 +544,7 @@ zen_owner_reduce_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int src_b
   uint64_t total = 0;
   for (int k = 0; k < ns; ++k) total += s_n[k];
   const bool dense_mode = allow_dense && total * (uint64_t)allow_dense > (uint64_t)c.nslots;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    c.cursors[ZEN_MAX_RANKS + 3] = dense_mode ? 1u : 0u;
-    for (int k = 0; k < ns; ++k) local_status |= s_flag[k];
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) c.cursors[ZEN_MAX_RANKS + 3] = dense_mode ? 1u : 0u;
   const uint32_t nslots = c.nslots;
   float* acc = c.acc;
   uint32_t* bitmap = c.bitmap;
@@ -903,41 +903,19 @@ __host__ __device__ __forceinline__ SbShape sb_shape(uint32_t nslots, uint32_t c
   return s;
 }
 
-// Records received from each source, after a bounded wait for its mail; one thread per source.
-__device__ __forceinline__ void sb_wait(const ZenSparseCtx& c, uint32_t epoch, uint32_t* s_n, uint32_t* s_flag) {
-  if ((int)threadIdx.x < c.nranks) {
-    const ZenMail* mail = zen_rec_mail(c, c.rank, threadIdx.x, epoch);
-    uint32_t n = 0, fl = 0;
-    if (zen_wait_epoch(&mail->epoch, epoch, c.wait_ns)) {
-      // count and info were written before the epoch's release store: plain loads after the acquire above see them
-      n = min(*reinterpret_cast<const volatile uint32_t*>(&mail->count), c.cap_rec);
-      if (*reinterpret_cast<const volatile uint32_t*>(&mail->info) & 1u) fl = ZEN_PEER_OVERFLOW;
-    } else {
-      fl = ZEN_TIMEOUT;
-    }
-    s_n[threadIdx.x] = n;
-    s_flag[threadIdx.x] = fl;
-  }
-  __syncthreads();
-}
-
 template <int NB>
 __global__ void __launch_bounds__(SB_SORT_THREADS, 2)
 zen_record_sort_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int deterministic, int by_index) {
   zen_pdl::enter();
   __shared__ ZenSparseCtx s_ctx;
   const ZenSparseCtx& c = zen_ctx(bt, s_ctx);
-  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS];
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS];
   __shared__ uint32_t hist[SB_MAX_BUCKETS + 1], s_warp[SB_SORT_THREADS / 32];
   __shared__ __align__(16) uint2 sorted[SB_TILE];
   const uint32_t epoch = zen_epoch(c);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  sb_wait(c, epoch, s_n, s_flag);
-  uint32_t local_status = 0;
-  if (blockIdx.x == 0 && tid == 0) {
-    c.cursors[ZEN_MAX_RANKS + 3] = deterministic ? 2u : 0u;              // for a K3b that is launched without being told
-    for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
-  }
+  uint32_t local_status = records_wait(c, epoch, 0, c.nranks, s_n);
+  if (blockIdx.x == 0 && tid == 0) c.cursors[ZEN_MAX_RANKS + 3] = deterministic ? 2u : 0u;     // for a K3b that is launched without being told
   const uint32_t nslots = by_index ? (uint32_t)c.numel : c.nslots;       // method 1: records carry element indices
   const SbShape sh = sb_shape(nslots, c.cap_rec, c.nranks);
   if (sh.on && sh.sorted) {
@@ -1096,20 +1074,17 @@ zen_reduce_gather_kernel(const __grid_constant__ ZenSparseBatch<NB> bt, int det)
   uint32_t* bm = reinterpret_cast<uint32_t*>(acc + BS);                  // [BS / 32]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hl = lane & 15, hf = lane >> 4;
   unsigned short* list = reinterpret_cast<unsigned short*>(bm + BS / 32) + warp * SB_WINDOW;    // pair-local slots
-  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS], s_last, s_fmt, s_base, s_tot[W];
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_last, s_fmt, s_base, s_tot[W];
   const uint32_t epoch = zen_epoch(c);
   const SbShape sh = sb_shape(c.nslots, c.cap_rec, c.nranks);
   for (uint32_t i = tid; i < (BS + BS / 32) / 4; i += W * 32) reinterpret_cast<uint4*>(smem_raw)[i] = make_uint4(0u, 0u, 0u, 0u);
-  sb_wait(c, epoch, s_n, s_flag);
-  uint32_t local_status = 0;
+  uint32_t local_status = records_wait(c, epoch, 0, c.nranks, s_n);
   uint64_t recs = 0;
   for (int k = 0; k < c.nranks; ++k) recs += s_n[k];
   // With many records the occupancy bitmap is not kept while they are added up: "touched" then means "sum is not zero" (a slot
   // whose sum is exactly zero need not travel).
   const bool dense_mode = recs * K2_DENSE > (uint64_t)c.nslots;
   if (tid == 0) {
-    if (blockIdx.x == 0)
-      for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
     // index format: bitmap when more than one slot in 32 is expected to be touched; the estimate is the number of records
     // received (an upper bound of the union), which every CTA reads from the same mails
     uint32_t fmt = c.fmt_mode;
@@ -1530,13 +1505,10 @@ zen_index_buckets_kernel(const __grid_constant__ ZenSparseBatch<NB> bt) {
   constexpr int W = 8;
   constexpr uint32_t BS = W * 2048, EPV = 16 / sizeof(T);
   float* acc = reinterpret_cast<float*>(smem_raw);                       // [BS]
-  __shared__ uint32_t s_n[ZEN_MAX_RANKS], s_flag[ZEN_MAX_RANKS];
+  __shared__ uint32_t s_n[ZEN_MAX_RANKS];
   const uint32_t epoch = zen_epoch(c), tid = threadIdx.x;
   for (uint32_t i = tid; i < BS / 4; i += W * 32) reinterpret_cast<float4*>(acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  sb_wait(c, epoch, s_n, s_flag);
-  uint32_t local_status = 0;
-  if (blockIdx.x == 0 && tid == 0)
-    for (int k = 0; k < c.nranks; ++k) local_status |= s_flag[k];
+  uint32_t local_status = records_wait(c, epoch, 0, c.nranks, s_n);
   const uint32_t N = (uint32_t)c.numel;
   const SbShape sh = sb_shape(N, c.cap_rec, c.nranks);
   // an element occurs once in a source
