@@ -48,3 +48,64 @@ def test_both_backwards_agree_with_fp32(B, S, hq, hkv, hd, monkeypatch):
     assert torch.equal(kept[:, v:], twice[:, v:])                    # dV is the same kernel's; dQ and dK hang on D, summed in another order
     for sl in (slice(0, q), slice(q, v)):
         assert (kept[:, sl].float() - twice[:, sl].float()).norm() <= 2e-3 * want[:, sl].norm()
+
+
+# ------------------------------------------------------------------------------------------- where the scratch does not fit
+class _Room:
+    """torch.empty as on a device with room for ``left`` bytes a tensor."""
+
+    def __init__(self, left):
+        self.left, self.real, self.refused = left, torch.empty, 0
+
+    def __call__(self, *size, **kw):
+        t = self.real(*size, **dict(kw, device="meta"))
+        if t.numel() * t.element_size() > self.left:
+            self.refused += 1
+            raise torch.OutOfMemoryError("no room")
+        return self.real(*size, **kw)
+
+
+def test_attention_runs_where_the_scratch_does_not_fit(monkeypatch):
+    from zen_repro_b200.ops import attention as A
+
+    B, S, hq, hkv, hd = 1, 1152, 16, 4, 128
+    need = _bytes(B, S, hq, hkv, hd)
+    assert need > 16 << 20
+    qkv = torch.randn(B * S, (hq + 2 * hkv) * hd, device="cuda").bfloat16()
+    dout = torch.randn(B * S, hq * hd, device="cuda").bfloat16()
+    out, lse2 = A.attention_fwd_kernel(qkv, B, S, hq, hkv, hd, hd ** -0.5)
+    room = _Room(need - 1)
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", room)
+        got = A.attention_bwd_kernel(dout, qkv, out, lse2, B, S, hq, hkv, hd, hd ** -0.5)
+    assert room.refused == 1
+    monkeypatch.setattr(A, "_flash_ds_bytes", lambda *a: 0)
+    assert torch.equal(got, A.attention_bwd_kernel(dout, qkv, out, lse2, B, S, hq, hkv, hd, hd ** -0.5))
+    assert A.attention_error() == 0
+
+
+def test_block_runs_where_the_scratch_does_not_fit(monkeypatch):
+    from zen_repro_b200.models import build_model
+    from zen_repro_b200.ops import attention as A
+
+    model = build_model("gpt2", device="cuda", num_layers=1)
+    model.reset_parameters(seed=0)
+    B, S = 4, 512
+    cfg = model.cfg
+    need = _bytes(B, S, cfg.num_heads, cfg.num_heads, cfg.head_dim)
+    assert need > 0
+    ids = torch.randint(0, cfg.vocab_size, (B, S), device="cuda")
+
+    def grads():
+        model.zero_grad()
+        model(ids, ids).backward()
+        return [p.grad.clone() for p in model.parameters() if p.grad is not None]
+
+    kept = grads()
+    asked = []
+    real = A.scratch
+    monkeypatch.setattr(A, "scratch", lambda most, least, dev: (asked.append(most - least), real(least, least, dev))[1])
+    twice = grads()
+    assert asked and asked[0] >= need
+    for a, b in zip(kept, twice):                                    # as the two backwards of the attention alone
+        assert (a.double() - b.double()).norm() <= 1e-2 * b.double().norm() + 1e-12

@@ -199,7 +199,8 @@ struct BwdTemp {
 };
 size_t lse_floats(const ZenBlock& z, const Shape& s) { return (size_t)s.B * z.hq * s.Sp; }
 
-BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base) {
+// keep_ds: with room for dS between the kernels of the attention backward, where they would keep it.
+BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base, bool keep_ds) {
   Layout l{(char*)base};
   typedef uint16_t bf;
   BwdTemp t{};
@@ -214,7 +215,7 @@ BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base) {
   t.stat = l.take<float>(2 * lse_floats(z, s));
   if (!wide_attention(z)) {
     int64_t need = 0;
-    zen_flash_ds_bytes(s.B, s.S, z.hq, z.hkv, z.hd, &need);
+    if (keep_ds) zen_flash_ds_bytes(s.B, s.S, z.hq, z.hkv, z.hd, &need);
     if (need) t.ds = l.take<char>((size_t)need);
   } else {
     const int hs = zen_attn_hsplit(s.B, s.S, z.hq, z.hkv, z.hd);
@@ -240,14 +241,16 @@ BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base) {
 
 extern "C" {
 
-// Bytes of the saved buffer (with and without a residual input), of the forward temporaries and of the backward ones.
+// Bytes of the saved buffer (with and without a residual input), of the forward temporaries and of the backward ones (with dS kept
+// and without).
 int zen_block_bytes(const ZenBlock* z, int B, int S, int64_t* out) {
   const Shape s = shape_of(*z, B, S);
   const size_t lse = up(lse_floats(*z, s) * 4);
   out[0] = (int64_t)(saved_of(s, nullptr, false).bytes + lse);
   out[1] = (int64_t)(saved_of(s, nullptr, true).bytes + lse);
   out[2] = (int64_t)(2 * up((size_t)s.T * s.d * 2));
-  out[3] = (int64_t)bwd_temp_of(*z, s, nullptr).bytes;
+  out[3] = (int64_t)bwd_temp_of(*z, s, nullptr, true).bytes;
+  out[4] = (int64_t)bwd_temp_of(*z, s, nullptr, false).bytes;
   return 0;
 }
 
@@ -281,14 +284,14 @@ int zen_block_fwd(const ZenBlock* zb, int B, int S, const void* x, const void* r
 }
 
 // Gradient of x (which is also the gradient of res) into dx and of the parameters into gr, from the gradients of dn and of h2
-// (null: none).  x, res, h2, saved: as in the forward.
-int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* res, const void* h2, void* saved, void* temp,
+// (null: none).  x, res, h2, saved: as in the forward.  keep_ds: which of the two sizes temp has.
+int zen_block_bwd(const ZenBlock* zb, int B, int S, const void* x, const void* res, const void* h2, void* saved, void* temp, int keep_ds,
                   const void* d_dn, const void* d_h2, void* dx, const ZenBlockGrads* gr, const ZenWorkspace* ws, void* stream) {
   const ZenBlock& z = *zb;
   const Shape s = shape_of(z, B, S);
   Saved v = saved_of(s, saved, res != nullptr);
   v.lse = reinterpret_cast<float*>((char*)saved + v.bytes);
-  BwdTemp t = bwd_temp_of(z, s, temp);
+  BwdTemp t = bwd_temp_of(z, s, temp, keep_ds != 0);
   Call c{z, *ws, stream};
   const int T = s.T, d = s.d, L = z.layer_norm;
   ReduceJob jobs[8];

@@ -75,16 +75,27 @@ def _flash_ds_bytes(bsz, seq, hq, hkv, hd) -> int:
     return out.value
 
 
+def scratch(most: int, least: int, device) -> tuple:
+    """(bytes, 1) of size ``most``, or (bytes, 0) of size ``least`` where the device has no room for as much: what dS takes between the
+    kernels of the backward is up to 3 GB, and a step that fits without it has to run."""
+    if most > least:
+        try:
+            return torch.empty(most, dtype=torch.uint8, device=device), 1
+        except torch.OutOfMemoryError:
+            pass
+    return torch.empty(least, dtype=torch.uint8, device=device), 0
+
+
 def attention_bwd_kernel(dout, qkv, out, lse2, bsz, seq, hq, hkv, hd, scale, softcap: float = 0.0):
     """tcgen05 backward: gradient of the fused qkv buffer (no atomics)."""
     dout = dout if (dout.is_contiguous() and dout.data_ptr() % 16 == 0) else dout.contiguous()
     dqkv = torch.empty_like(qkv)
     if hd <= 128 and softcap <= 0:
-        need, nstat = _flash_ds_bytes(bsz, seq, hq, hkv, hd), 2 * lse2.numel()
-        scratch = torch.empty(nstat + need // 4, dtype=torch.float32, device=qkv.device)       # row statistics (a multiple of 1 KB), dS
-        stat = scratch.data_ptr()
+        need, nstat = _flash_ds_bytes(bsz, seq, hq, hkv, hd), 8 * lse2.numel()
+        temp, keep_ds = scratch(nstat + need, nstat, qkv.device)                                 # row statistics (a multiple of 1 KB), dS
+        stat = temp.data_ptr()
         rc = _native.lib().zen_flash_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse2.data_ptr(), stat, dqkv.data_ptr(), bsz, seq, hq,
-                                         hkv, hd, qkv.stride(0), out.stride(0), dqkv.stride(0), float(scale), stat + 4 * nstat if need else 0,
+                                         hkv, hd, qkv.stride(0), out.stride(0), dqkv.stride(0), float(scale), stat + nstat if keep_ds else 0,
                                          _native.stream_ptr())
         if rc:
             _native.check(rc, "zen_flash_bwd")

@@ -87,9 +87,9 @@ class _Plan:
             z.fwd_only[i] = _pick(G.plan_forward_only(T, fout, fin))
             z.dw[i] = _pick_weight(fin, fout, T) if z.w_in_out else _pick_weight(fout, fin, T)
         self.z, self.addr = z, ctypes.addressof(z)
-        sizes = (ctypes.c_int64 * 4)()
+        sizes = (ctypes.c_int64 * 5)()
         lib.zen_block_bytes(self.addr, bsz, seq, sizes)
-        self.saved, self.saved_res, self.fwd_temp, self.bwd_temp = (int(v) for v in sizes)
+        self.saved, self.saved_res, self.fwd_temp, self.bwd_temp, self.bwd_temp_least = (int(v) for v in sizes)
 
 
 def usable(blk, x: torch.Tensor, bsz: int, seq: int) -> bool:
@@ -180,9 +180,9 @@ class BlockFn(torch.autograd.Function):
                 if g is not None:
                     gr.g[i] = g.data_ptr()
         dx = torch.empty_like(x)
-        temp = torch.empty(plan.bwd_temp, dtype=torch.uint8, device=dev)
+        temp, keep_ds = A.scratch(plan.bwd_temp, plan.bwd_temp_least, dev)
         rc = _native.lib().zen_block_bwd(plan.addr, bsz, seq, x.data_ptr(), _native.ptr(res), h2.data_ptr(), saved.data_ptr(), temp.data_ptr(),
-                                         d_dn.data_ptr(), _native.ptr(d_h2), dx.data_ptr(), ctypes.addressof(gr), _workspace(dev),
+                                         keep_ds, d_dn.data_ptr(), _native.ptr(d_h2), dx.data_ptr(), ctypes.addressof(gr), _workspace(dev),
                                          _native.stream_ptr())
         if rc:
             _native.check(rc, "zen_block_bwd")
