@@ -1,0 +1,61 @@
+"""The tiles of a partly filled last round as two halves of K: where the workspace holds what they exchange, and nothing beyond it is
+written."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+HALVES = 2 * 2 * 128 * 256                  # floats that the two halves of a tile exchange; 16 counters beside them
+
+
+def _clusters():
+    return torch.cuda.get_device_properties(0).multi_processor_count // 2
+
+
+def _group(pairs, ws_floats, n_counters):
+    """a' b of each pair in one launch, with a workspace of that size between guard words."""
+    from zen_repro_b200 import _native
+    from zen_repro_b200.ops import gemm as G
+
+    ws = torch.full((ws_floats + 4096,), 3.0, device="cuda")
+    cnt = torch.zeros(n_counters + 64, dtype=torch.int32, device="cuda")
+    outs = [torch.empty(a.shape[1], b.shape[1], dtype=torch.bfloat16, device="cuda") for a, b in pairs]
+    descs = (G._GemmDesc * len(pairs))()
+    for i, ((a, b), c) in enumerate(zip(pairs, outs)):
+        descs[i] = G._GemmDesc(a.data_ptr(), b.data_ptr(), c.data_ptr(), a.shape[1], b.shape[1], a.shape[0], a.stride(0), b.stride(0), c.stride(0), 0, 0)
+    rc = _native.lib().zen_gemm_bf16_2cta_group(descs, len(pairs), 1, 1, ws.data_ptr() if ws_floats else 0, ws_floats, cnt.data_ptr(), n_counters,
+                                                _native.stream_ptr())
+    assert rc == 0 and G.gemm_error() == 0
+    assert bool((ws[ws_floats:] == 3.0).all()) and not bool(cnt.any())
+    return outs
+
+
+def _pair(k, m, n):
+    return torch.randn(k, m, device="cuda").bfloat16(), torch.randn(k, n, device="cuda").bfloat16()
+
+
+def _sum_of_halves(a, b):
+    """a' b as the two halves of K, each summed in fp32 by a launch of its own, then added and rounded."""
+    from zen_repro_b200.ops import gemm as G
+
+    half = (a.shape[0] // 64 + 1) // 2 * 64
+    parts = [G.gemm_tn(a[s], b[s], out_dtype=torch.float32, bn=512) for s in (slice(0, half), slice(half, None))]
+    return (parts[0] + parts[1]).bfloat16()
+
+
+@pytest.mark.parametrize("k", [1024, 2112])
+@pytest.mark.parametrize("missing", [0, 1])
+def test_a_workspace_for_the_tiles_at_hand_is_enough(k, missing):
+    torch.manual_seed(k)
+    rem = 5
+    pairs = [_pair(k, (_clusters() + rem) * 256, 256)]
+    (whole,) = _group(pairs, 0, 0)
+    for floats, counters in ((rem * HALVES - missing, rem * 16), (rem * HALVES, rem * 16 - missing)):
+        (got,) = _group(pairs, floats, counters)
+        cut = (got != whole).any(1).view(-1, 256).any(1)            # per tile
+        # fp32 sums in another order differ somewhere in every tile of 65 536 elements
+        assert int(cut.sum()) == (0 if missing else rem)
+        if not missing:
+            assert torch.equal(got.view(-1, 256, 256)[cut], _sum_of_halves(*pairs[0]).view(-1, 256, 256)[cut])

@@ -835,10 +835,13 @@ int g_tail_min_kb = 1;             // fewest 64-wide K blocks for which the tile
 // first cut, and not for outputs of one round, which split_k_choice cuts where that pays: another order of summation in one tile of ten moves the logits of a four-layer Llama by up to 1.2 % (2 x 600 and 1 x
 // 2048 tokens), as much as any rounding there, and scores should not change by that for 2 us.
 constexpr int TAIL_K_MIN_KB = 16;
-static void cut_tail(GemmGroup& g, int min_kb) {
+// ws_floats, n_counters: what the caller's workspace holds.
+static void cut_tail(GemmGroup& g, int min_kb, uint64_t ws_floats = 0, int n_counters = 0) {
   const int clusters = zen_tmap::sm_count() / 2, rem = g.num_tiles % clusters;
   g.tail = g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && 2 * rem <= clusters ? rem : 0;
-  g.tail_k = g.tail > 0 && g.num_tiles > clusters && min_kb >= TAIL_K_MIN_KB && g.ws && g.counters;
+  const bool room = g.ws && g.counters && reinterpret_cast<uintptr_t>(g.ws) % 16 == 0 && ws_floats >= (uint64_t)g.tail * 2 * 2 * BM2 * 256 &&
+                    n_counters >= g.tail * 16;
+  g.tail_k = g.tail > 0 && g.num_tiles > clusters && min_kb >= TAIL_K_MIN_KB && room;
   for (int i = 0; i < g.n && g.tail_k; ++i) {
     const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
     if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
@@ -879,11 +882,6 @@ static bool narrow_rows(GemmGroup& g, const void* A, int lda, int min_kb) {
   g.tail = g.tail_k = 0;
   return true;
 }
-// Whether a caller's workspace holds the halves of the tiles that a last wave may have: half of the clusters.
-static bool tail_workspace(const float* ws, uint64_t ws_floats, const int* counters, int n_counters) {
-  const int most = zen_tmap::sm_count() / 4;
-  return ws && counters && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && ws_floats >= (uint64_t)most * 2 * 2 * BM2 * 256 && n_counters >= most * 16;
-}
 
 // 256-wide pair tiles.  The narrower ones exist for outputs whose 256-wide tiles fill the 74 CTA pairs unevenly: 8192 x 768 is
 // 96 tiles of 256, 1.3 rounds, or 128 tiles of 192 (K-major B only: its half of 96 rows is one TMA box; an MN-major half would
@@ -905,8 +903,8 @@ extern "C" {
 // long K, the weight-gradient shape): `ws` must hold splits * tiles * 2 * 128 * 256 floats and `counters`
 // tiles * 16 ints that are zero on entry (the kernel leaves them zero); both are caller-owned and used in stream
 // order.  The slices are summed in slice order, so the result does not depend on timing.
-// With splits == 1 a caller may still pass `ws` and `counters` (sizes as for two slices of one wave of clusters): the tiles of a
-// partly filled last wave may then be cut along K (cut_tail).
+// With splits == 1 a caller may still pass `ws` and `counters` (as for two slices of the tiles of a partly filled last wave): these may
+// then be cut along K (cut_tail).
 // n_store: 0, or a width in [N, ldc] that the kernel may write (columns N.. receive zeros).
 int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                               int ldb, int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int splits, float* ws,
@@ -952,8 +950,7 @@ int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void*
   g.counters = counters;
   g.tail = g.tail_k = 0;
   if (splits == 1 && bn == 256) {
-    if (!tail_workspace(ws, ws_floats, counters, n_counters)) g.ws = nullptr;
-    cut_tail(g, nkb);
+    cut_tail(g, nkb, ws_floats, n_counters);
     if (!a_mn && narrow_rows(g, A, lda, nkb)) {
       if (bias) return b_mn ? launch2_as<false, true, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
       return b_mn ? launch2_as<false, true, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
@@ -1041,8 +1038,7 @@ int zen_gemm_bf16_2cta_group(const ZenGemmDesc* descs, int n, int a_mn, int b_mn
   g.kb_per_split = 1 << 30;
   g.ws = ws;
   g.counters = counters;
-  if (!tail_workspace(ws, ws_floats, counters, n_counters)) g.ws = nullptr;
-  cut_tail(g, min_kb);
+  cut_tail(g, min_kb, ws_floats, n_counters);
   return launch2_layout(g, a_mn, b_mn, 256, (cudaStream_t)stream);
 }
 
