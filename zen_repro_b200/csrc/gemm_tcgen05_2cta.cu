@@ -832,16 +832,17 @@ int g_tail_min_kb = 1;             // fewest 64-wide K blocks for which the tile
 // column halves: the 108 tiles of a GPT-2 layer's weight gradients, K = 8192, 75 / 80; 8192 x 768 x 3072 40.9 / 40.9;
 // 8192 x 768 x 2304 34.7 / 32.7; 8192 x 3072 x 768 38.8 (whole) / 36.8; 700 x 2304 x 9216 without a workspace 55.1 (whole) / 47.0.
 // By time the line would lie near K = 4096.  It lies at 1024, where the sum of a tile's two halves has been taken since K was
-// first cut, and not for outputs of one round, which split_k_choice cuts where that pays: another order of summation in one tile of ten moves the logits of a four-layer Llama by up to 1.2 % (2 x 600 and 1 x
-// 2048 tokens), as much as any rounding there, and scores should not change by that for 2 us.
+// first cut, and for single products not in outputs of one round, which split_k_choice cuts where that pays (no plan sees the tiles of
+// a group): another order of summation in one tile of ten moves the logits of a four-layer Llama by up to 1.2 % (2 x 600 and 1 x 2048
+// tokens), as much as any rounding there, and scores should not change by that for 2 us.
 constexpr int TAIL_K_MIN_KB = 16;
-// ws_floats, n_counters: what the caller's workspace holds.
-static void cut_tail(GemmGroup& g, int min_kb, uint64_t ws_floats = 0, int n_counters = 0) {
+// ws_floats, n_counters: what the caller's workspace holds; one_round: K also where all tiles fit one round.
+static void cut_tail(GemmGroup& g, int min_kb, uint64_t ws_floats = 0, int n_counters = 0, bool one_round = false) {
   const int clusters = zen_tmap::sm_count() / 2, rem = g.num_tiles % clusters;
   g.tail = g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && 2 * rem <= clusters ? rem : 0;
   const bool room = g.ws && g.counters && reinterpret_cast<uintptr_t>(g.ws) % 16 == 0 && ws_floats >= (uint64_t)g.tail * 2 * 2 * BM2 * 256 &&
                     n_counters >= g.tail * 16;
-  g.tail_k = g.tail > 0 && g.num_tiles > clusters && min_kb >= TAIL_K_MIN_KB && room;
+  g.tail_k = g.tail > 0 && (one_round || g.num_tiles > clusters) && min_kb >= TAIL_K_MIN_KB && room;
   for (int i = 0; i < g.n && g.tail_k; ++i) {
     const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
     if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
@@ -1038,7 +1039,7 @@ int zen_gemm_bf16_2cta_group(const ZenGemmDesc* descs, int n, int a_mn, int b_mn
   g.kb_per_split = 1 << 30;
   g.ws = ws;
   g.counters = counters;
-  cut_tail(g, min_kb, ws_floats, n_counters);
+  cut_tail(g, min_kb, ws_floats, n_counters, true);
   return launch2_layout(g, a_mn, b_mn, 256, (cudaStream_t)stream);
 }
 
