@@ -115,3 +115,25 @@ def test_labels_that_the_kernel_would_misread_are_refused(labels):
     with pytest.raises(ValueError):
         G.gemm_nt_loss(a, b, labels())
     assert _native.launch_count() == before
+
+
+@pytest.mark.parametrize("dead", [64, 128, 700, 1000])
+def test_infinite_logits_are_capped_too(dead):
+    """Soft-capped logits of -inf are -cap: boxes, pieces and whole rows of nothing else still count."""
+    from zen_repro_b200.ops import elementwise as E
+    from zen_repro_b200.ops import gemm as G
+
+    torch.manual_seed(dead)
+    M, N, K, cap = 256, 1000, 64, 5.0
+    a = (torch.rand(M, K, device="cuda") + 0.1).bfloat16()
+    b = (torch.randn(N, K, device="cuda") * 0.1 - 0.6).bfloat16()           # the others lie near -cap as well
+    b[:dead] = float("-inf")
+    labels = torch.randint(0, N, (M,), device="cuda")
+    loss = torch.empty(M, device="cuda")
+    part, target = G.gemm_nt_loss(a, b, labels, softcap=cap)
+    lse = E.xent_finish(part, target, labels, N, loss, softcap=cap)
+    z = cap * torch.tanh(G.gemm_nt(a, b, bn=512).double() / cap)
+    assert (z[:, :dead] == -cap).all()
+    bound = 16 * 2.0 ** -24 * (cap + 16)                                    # as in test_against_64_bits
+    assert (lse - torch.logsumexp(z, -1)).abs().max() <= bound
+    assert (loss - F.cross_entropy(z, labels, reduction="none")).abs().max() <= bound

@@ -303,7 +303,7 @@ __device__ __forceinline__ void epilogue_loss(const GemmGroup& gg, const GemmPro
 #pragma unroll
     for (int i = 0; i < 64; ++i) mx[i & 3] = fmaxf(mx[i & 3], at(i));
     float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-    if (CAP && top != -INFINITY) top = zen_xe::xent_cap<T, CAP>(top, gg.cap, k2);   // monotonic
+    if (CAP) top = zen_xe::xent_cap<T, CAP>(top, gg.cap, k2);                      // monotonic; -inf becomes -cap (a box has columns inside)
     const float nm = fmaxf(m, top), ref = nm == -INFINITY ? 0.f : nm;
     float add[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
