@@ -33,6 +33,7 @@ def test_rows_beyond_the_last_whole_tile(m, n, k, b_mn, bias):
         else:
             G.gemm_nt(a, b, bias=v, out=out, bn=512, pad_ok=True)
         assert (buf[m:] == 7.0).all() and (buf[:, ld:] == 7.0).all()     # nothing beyond the matrix and its padding
+        assert b_mn or (buf[:m, n:ld] == 0.0).all()                      # which is written with zeros
         return out.float()
 
     got = run()

@@ -54,6 +54,7 @@ struct GemmProblem {
   const void* bias;
   int M, N, K, ldc;
   int out_fp32, accumulate;
+  int n_store;                      // columns that a bf16 output may be written in: N, or more (zeros)
   int tma_store;                    // bf16 output written through shared memory and TMA stores (full lines, async)
   int num_m_pairs, num_n_tiles;
   int group_m;                      // tile order: blocks of group_m tile rows, all their columns, rows fastest (see pick_group_m)
@@ -318,7 +319,8 @@ __device__ __forceinline__ void epilogue_loss(const GemmGroup& gg, const GemmPro
   if (row < p.M) gg.part[(size_t)((n0 + cb_lo * 64) / 128) * gg.part_ld + row] = make_float2(m, s);
 }
 
-// A transposed tile: the lane's column of the output, `narrow` rows of it in the columns of tensor memory.
+// A transposed tile: the lane's column of the output, `narrow` rows of it in the columns of tensor memory.  Columns from N on are zero
+// there, as B is filled up with zeros.
 template <int HALVES>
 __device__ __forceinline__ void store_narrow(const GemmGroup& gg, uint32_t taddr, int col, int half) {
   const GemmProblem& p = gg.pr[0];
@@ -331,7 +333,7 @@ __device__ __forceinline__ void store_narrow(const GemmGroup& gg, uint32_t taddr
     __nv_bfloat16* c = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row * p.ldc + col;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (row + i < p.M && col < p.N) c[(size_t)i * p.ldc] = __float2bfloat16_rn(__uint_as_float(r[i]) + bias);
+      if (row + i < p.M && col < p.n_store) c[(size_t)i * p.ldc] = __float2bfloat16_rn(__uint_as_float(r[i]) + bias);
   }
 }
 
@@ -812,6 +814,7 @@ int fill_problem(GemmProblem& q, const void* A, const void* B, void* C, const vo
     rc = zen_tmap::get(C, (uint64_t)n_store, (uint64_t)M, (uint64_t)ldc, 64, 32, &q.tc);
     if (rc) return rc;
   }
+  q.n_store = n_store;
   q.C = C; q.bias = bias; q.M = M; q.N = N; q.K = K; q.ldc = ldc; q.out_fp32 = out_fp32; q.accumulate = accumulate;
   q.num_m_pairs = (M + 255) / 256;
   q.num_n_tiles = (N + bn - 1) / bn;
