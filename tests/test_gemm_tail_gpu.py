@@ -70,3 +70,41 @@ def test_groups_of_less_than_a_round_are_cut(shapes):
     assert 2 * tiles <= _clusters()
     for got, (a, b) in zip(_group(pairs, tiles * HALVES, tiles * 16), pairs):
         assert torch.equal(got, _sum_of_halves(a, b))
+
+
+@pytest.mark.parametrize("n", [28672, 40960])
+def test_the_caller_says_what_no_product_reads(n):
+    """Rows beyond the last whole 256 in an output whose last round is cut along K: transposed tiles, and with them another order of
+    summation, only where the caller allows it, whatever the width."""
+    from zen_repro_b200 import _native
+    from zen_repro_b200.ops import gemm as G
+
+    torch.manual_seed(n)
+    # 44 rows over; narrow tiles shorten the rounds of both widths
+    a, b = torch.randn(300, 1024, device="cuda").bfloat16(), torch.randn(n, 1024, device="cuda").bfloat16()
+    tiles, per = 2 * (n // 256), _clusters()
+    assert tiles > per and 0 < 2 * (tiles % per) <= per
+    inner, last = (G.gemm_nt(a, b, bn=512, last=flag) for flag in (False, True))
+    old = _native.lib().zen_gemm2_tail_split(0)
+    try:
+        whole = G.gemm_nt(a, b, bn=512)
+    finally:
+        _native.lib().zen_gemm2_tail_split(old)
+    changed = (inner != whole).view(300, n // 256, 256).any(2)
+    assert 0 < int(changed.any(0).sum()) < n // 256                  # the tiles of the last round alone
+    assert torch.equal(last, whole)
+
+
+def test_logits_say_so(monkeypatch):
+    from zen_repro_b200.models import build_model
+    from zen_repro_b200.ops import gemm as G
+
+    model = build_model("gpt2", device="cuda", num_layers=1)
+    model.reset_parameters(seed=0)
+    ids = torch.randint(0, model.cfg.vocab_size, (1, 300), device="cuda")
+    seen = []
+    real = G.gemm_nt
+    monkeypatch.setattr(G, "gemm_nt", lambda a, b, *r, **k: (seen.append((b.shape[0], bool(k.get("last")))), real(a, b, *r, **k))[1])
+    model(ids)
+    model(ids, ids)
+    assert {w for w, flag in seen if flag} == {model.cfg.vocab_size} == {w for w, _ in seen if w > 10_000}

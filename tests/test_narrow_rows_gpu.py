@@ -29,9 +29,9 @@ def test_rows_beyond_the_last_whole_tile(m, n, k, b_mn, bias):
         out = buf[:m, :n]
         if b_mn:
             bt = b.t().contiguous()
-            G._launch(a, bt, m, n, k, False, True, v, out, False, None, 512)
+            G._launch(a, bt, m, n, k, False, True, v, out, False, None, 512, last=True)
         else:
-            G.gemm_nt(a, b, bias=v, out=out, bn=512, pad_ok=True)
+            G.gemm_nt(a, b, bias=v, out=out, bn=512, pad_ok=True, last=True)
         assert (buf[m:] == 7.0).all() and (buf[:, ld:] == 7.0).all()     # nothing beyond the matrix and its padding
         assert b_mn or (buf[:m, n:ld] == 0.0).all()                      # which is written with zeros
         return out.float()

@@ -34,7 +34,7 @@ int zen_attn_hsplit(int B, int S, int Hq, int Hkv, int hd);
 int zen_gemm_bf16_2cta_act(const void*, const void*, void*, const void*, void*, int, int, int, int, int, int, int, int, int, int, void*);
 int zen_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, void*);
 int zen_gemm_bf16_2cta_splitk(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, float*,
-                              uint64_t, int*, int, int, void*);
+                              uint64_t, int*, int, int, int, void*);
 int zen_gemm_bf16_cluster_splitk(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, int,
                                  void*);
 struct ZenGemmDesc {
@@ -147,7 +147,7 @@ struct Call {
     if (rc) return;
     if (k.kind == 1)                                       // p1: no workspace to cut the last round's K with
       rc = zen_gemm_bf16_2cta_splitk(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, 0, acc, k.p0, k.p1 ? nullptr : w.ws, k.p1 ? 0 : w.n_ws,
-                                     k.p1 ? nullptr : w.cnt, k.p1 ? 0 : w.n_cnt, 0, st);
+                                     k.p1 ? nullptr : w.cnt, k.p1 ? 0 : w.n_cnt, 0, 0, st);
     else if (k.kind == 2 && reinterpret_cast<uintptr_t>(C) % 16 == 0)
       rc = zen_gemm_bf16_cluster_splitk(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, 0, acc, k.p0, k.p1, st);
     else

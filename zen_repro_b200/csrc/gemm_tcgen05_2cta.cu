@@ -857,11 +857,12 @@ static void cut_tail(GemmGroup& g, int min_kb, uint64_t ws_floats = 0, int n_cou
 // 3 %; the clusters that would be idle in the last round take up to three.  In practice that is an output many rounds long: us, whole tiles /
 // with transposed ones, 777 x 128256 x 3072 494 / 454, 1300 x 16384 x 2048 71.7 / 68.6, 300 x 50257 x 768 41.0 / 40.0; but
 // 777 x 16384 x 3072 70.6 / 73.3, 2100 x 2304 x 768 19.0 / 20.0 and 3100 x 7680 x 2560 86 / 89, which the weights leave whole.
-static bool narrow_rows(GemmGroup& g, const void* A, int lda, int min_kb) {
+// last: no product reads the output (logits), so the order of summation may change with it, see cut_tail.
+static bool narrow_rows(GemmGroup& g, const void* A, int lda, int min_kb, bool last) {
   GemmProblem& p = g.pr[0];
   const int clusters = zen_tmap::sm_count() / 2, rows = p.M % 256;
   if (g_tail_min_kb <= 0 || min_kb < g_tail_min_kb || p.M < 256 || rows == 0 || rows > 128 || !p.tma_store) return false;
-  if (g.tail_k && p.N <= 32768) return false;           // the order of summation, see cut_tail; wider ones are logits, and no product follows
+  if (g.tail_k && !last) return false;
   const int width = (rows + 31) / 32 * 32, cols = p.num_n_tiles, tiles = (p.num_m_pairs - 1) * cols;
   const double cost = 0.75 + width / 1024.0;
   const int now_rem = g.num_tiles % clusters;
@@ -909,20 +910,20 @@ extern "C" {
 // order.  The slices are summed in slice order, so the result does not depend on timing.
 // With splits == 1 a caller may still pass `ws` and `counters` (as for two slices of the tiles of a partly filled last wave): these may
 // then be cut along K (cut_tail).
-// n_store: 0, or a width in [N, ldc] that the kernel may write (columns N.. receive zeros).
+// n_store: 0, or a width in [N, ldc] that the kernel may write (columns N.. receive zeros).  last: no product reads the output.
 int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                               int ldb, int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int splits, float* ws,
-                              uint64_t ws_floats, int* counters, int n_counters, int n_store, void* stream);
+                              uint64_t ws_floats, int* counters, int n_counters, int n_store, int last, void* stream);
 
 int zen_gemm_bf16_2cta(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
                        int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, void* stream) {
   return zen_gemm_bf16_2cta_splitk(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, 1, nullptr, 0,
-                                   nullptr, 0, 0, stream);
+                                   nullptr, 0, 0, 0, stream);
 }
 
 int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                               int ldb, int ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int splits, float* ws,
-                              uint64_t ws_floats, int* counters, int n_counters, int n_store, void* stream) {
+                              uint64_t ws_floats, int* counters, int n_counters, int n_store, int last, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   const int nkb = (K + BK2 - 1) / BK2;
   if (splits < 1) splits = 1;
@@ -955,7 +956,7 @@ int zen_gemm_bf16_2cta_splitk(const void* A, const void* B, void* C, const void*
   g.tail = g.tail_k = 0;
   if (splits == 1 && bn == 256) {
     cut_tail(g, nkb, ws_floats, n_counters);
-    if (!a_mn && narrow_rows(g, A, lda, nkb)) {
+    if (!a_mn && narrow_rows(g, A, lda, nkb, last != 0)) {
       if (bias) return b_mn ? launch2_as<false, true, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 8, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
       return b_mn ? launch2_as<false, true, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream) : launch2_as<false, false, 256, 4, EPI_STORE_NARROW>(g, (cudaStream_t)stream);
     }

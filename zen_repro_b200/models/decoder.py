@@ -287,7 +287,7 @@ class DecoderLM(nn.Module):
 
     def _logits(self, y):
         w = self.head_weight()
-        logits = O.linear(y, w, None, "out_in")
+        logits = O.linear(y, w, None, "out_in", last=True)
         _, tp = _tp(self.tp_group)
         if tp > 1:
             parts = [torch.empty_like(logits) for _ in range(tp)]

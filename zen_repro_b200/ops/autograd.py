@@ -55,7 +55,7 @@ class LinearFn(torch.autograd.Function):
     after the sum), "col" = the input gradient is summed over the TP group (column-parallel layer)."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, layout, tp_mode=None, tp_ws=None):
+    def forward(ctx, x, weight, bias, layout, tp_mode=None, tp_ws=None, last=False):
         ctx.layout = layout
         ctx.has_bias = bias is not None
         ctx.tp = (tp_mode, tp_ws)
@@ -64,7 +64,7 @@ class LinearFn(torch.autograd.Function):
         if tp_mode == "row":
             y = tp_ws.gemm_ar_nt(x2, weight, bias) if layout == "out_in" else tp_ws.gemm_ar_nn(x2, weight, bias)
         elif layout == "out_in":
-            y = G.gemm_nt(x2, weight, bias=bias)
+            y = G.gemm_nt(x2, weight, bias=bias, last=last)
         else:
             y = G.gemm_nn(x2, weight, bias=bias)
         ctx.save_for_backward(x2, weight)
@@ -110,11 +110,12 @@ class LinearFn(torch.autograd.Function):
                 db = E.colsum_from_parts(part, torch.empty(dy2.shape[1], dtype=dy2.dtype, device=dy2.device), accumulate=False)
             else:
                 db = E.colsum(dy2)
-        return dx, dw, db, None, None, None
+        return dx, dw, db, None, None, None, None
 
 
-def linear(x, weight, bias=None, layout="out_in", tp_mode=None, tp_ws=None):
-    return LinearFn.apply(x, weight, bias, layout, tp_mode, tp_ws)
+def linear(x, weight, bias=None, layout="out_in", tp_mode=None, tp_ws=None, last=False):
+    """``last``: no product reads the result (logits)."""
+    return LinearFn.apply(x, weight, bias, layout, tp_mode, tp_ws, last)
 
 
 class NormFn(torch.autograd.Function):
@@ -336,7 +337,7 @@ class LMHeadLossFn(torch.autograd.Function):
                 lse = E.xent_finish(part, target, ls, V, losses[s:e], ignore_index, softcap)
                 dl = E.xent_grad_(logits, ls, lse, inv, ignore_index=ignore_index, softcap=softcap) if train else None
             else:
-                G.gemm_nt(hs, weight, out=logits, pad_ok=True)
+                G.gemm_nt(hs, weight, out=logits, pad_ok=True, last=True)
                 th = None if in_kernel else _softcap_(logits, softcap)
                 loss, dl = E.cross_entropy(logits, ls, grad_scale=1.0 if train else None, grad_scale_dev=inv, ignore_index=ignore_index,
                                            softcap=softcap if in_kernel else 0.0, loss_out=losses[s:e] if in_kernel else None)
@@ -399,7 +400,7 @@ class VocabParallelLMHeadLossFn(torch.autograd.Function):
             e = min(T, s + chunk_tokens)
             buf = torch.empty(e - s, vpad, dtype=h2.dtype, device=h2.device)
             logits = buf[:, :Vl]
-            G.gemm_nt(h2[s:e], weight, out=logits, pad_ok=True)
+            G.gemm_nt(h2[s:e], weight, out=logits, pad_ok=True, last=True)
             th = _softcap_(logits, softcap)
             m, se, tgt = E.xent_partial(logits, lab[s:e], valid_cols, vocab_start, ignore_index)
             gm = m.clone()

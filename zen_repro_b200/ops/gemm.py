@@ -203,7 +203,7 @@ def plan_forward_only(M: int, N: int, K: int):
     return ("one", 256 if _t_one(M, N, nkb, _T_ONE256) < _t_one(M, N, nkb, _T_ONE128) else 128)
 
 
-def _launch(a, b, M, N, K, a_mn, b_mn, bias, out, accumulate, out_dtype, bn, pad_ok=False):
+def _launch(a, b, M, N, K, a_mn, b_mn, bias, out, accumulate, out_dtype, bn, pad_ok=False, last=False):
     a2, b2 = _rowmajor(a), _rowmajor(b)
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype or torch.bfloat16, device=a.device)
@@ -227,7 +227,7 @@ def _launch(a, b, M, N, K, a_mn, b_mn, bias, out, accumulate, out_dtype, bn, pad
             lib.zen_gemm2_tail_split(0)
         ws, n_ws, cnt, n_cnt = _workspace_args(a.device) if _TAIL_SPLIT or how[0] > 1 else (0, 0, 0, 0)       # where K slices meet
         rc = lib.zen_gemm_bf16_2cta_splitk(a2.data_ptr(), b2.data_ptr(), c, pbias, M, N, K, a2.stride(0), b2.stride(0), ldc, a_mn,
-                                           b_mn, fp32, bool(accumulate), how[0], ws, n_ws, cnt, n_cnt, n_store, stream)
+                                           b_mn, fp32, bool(accumulate), how[0], ws, n_ws, cnt, n_cnt, n_store, bool(last), stream)
     elif kind == "cluster":
         rc = lib.zen_gemm_bf16_cluster_splitk(a2.data_ptr(), b2.data_ptr(), c, pbias, M, N, K, a2.stride(0), b2.stride(0), ldc, a_mn,
                                               b_mn, fp32, bool(accumulate), how[0], how[1], stream)
@@ -239,15 +239,16 @@ def _launch(a, b, M, N, K, a_mn, b_mn, bias, out, accumulate, out_dtype, bn, pad
     return out
 
 
-def gemm_nt(a, b, bias=None, out=None, accumulate=False, out_dtype=None, bn=0, pad_ok=False):
+def gemm_nt(a, b, bias=None, out=None, accumulate=False, out_dtype=None, bn=0, pad_ok=False, last=False):
     """a[M,K] @ b[N,K]^T (+ bias[N]).  ``pad_ok``: ``out`` is the first N columns of a wider buffer whose columns up to
-    the next multiple of 8 may be overwritten (with zeros); lets an odd N use the full-line store path."""
+    the next multiple of 8 may be overwritten (with zeros); lets an odd N use the full-line store path.
+    ``last``: no product reads the result (logits), so that it may be summed in whichever order is fastest."""
     M, K = a.shape[-2] if a.dim() == 2 else a.numel() // a.shape[-1], a.shape[-1]
     N = b.shape[0]
     if not _use_kernel(a, b):
         r = a.reshape(-1, K).float() @ b.float().t()
         return _finish(r, bias, out, accumulate, out_dtype or a.dtype)
-    return _launch(a, b, M, N, K, False, False, bias, out, accumulate, out_dtype, bn, pad_ok)
+    return _launch(a, b, M, N, K, False, False, bias, out, accumulate, out_dtype, bn, pad_ok, last)
 
 
 def makes_loss_statistics(a, b) -> bool:
