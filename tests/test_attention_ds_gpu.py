@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 def _bytes(B, S, hq, hkv, hd):
     from zen_repro_b200.ops import attention as A
-    return A._flash_ds_bytes(B, S, hq, hkv, hd)
+    return A._flash_ds_bytes(B, S, hq, hd)
 
 
 def test_when_it_is_kept():

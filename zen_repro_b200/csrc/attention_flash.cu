@@ -901,9 +901,8 @@ int zen_flash_fwd(const void* qkv, void* out, float* lse2, int B, int S, int Hq,
 //  * Head sizes up to 96 leave a tile in half the time that one of 128 takes, so that dS has to stay in L2 to pay: 8 x 1024, 12 heads of
 //    64 (113 MB) 116 / 110, 1 x 4096 (208 MB) 132 / 138; 3 x 1000, 32 heads of 80 (113 MB) 140 / 127, 1 x 8192 1444 / 1478.
 //  * Above that up to DS_MOST (1 x 4096, 24 heads of 128, 415 MB: 324 / 294; 1 x 8192, 32 heads, 2.2 GB: 1680 / 1575).
-int zen_flash_ds_bytes(int B, int S, int Hq, int Hkv, int hd, int64_t* bytes) {
+int zen_flash_ds_bytes(int B, int S, int Hq, int hd, int64_t* bytes) {
   constexpr int64_t DS_MIN_TILES = 256, DS_IN_L2 = (int64_t)128 << 20, DS_MOST = (int64_t)3 << 30;
-  (void)Hkv;
   const int64_t nq = (S + 127) / 128, tiles = (int64_t)B * Hq * nq * (nq + 1) / 2;
   *bytes = nq < 2 || tiles < DS_MIN_TILES || tiles * DS_TILE > (hd > 96 ? DS_MOST : DS_IN_L2) ? 0 : tiles * DS_TILE;
   return 0;

@@ -26,7 +26,7 @@ int zen_rope(void*, int, int, int, int, int, int, float, int, int, void*);
 int zen_colreduce_multi(const void*, int, int, void*);
 int zen_flash_fwd(const void*, void*, float*, int, int, int, int, int, int, int, float, void*);
 int zen_flash_bwd(const void*, const void*, const void*, const float*, float*, void*, int, int, int, int, int, int, int, int, float, void*, void*);
-int zen_flash_ds_bytes(int, int, int, int, int, int64_t*);
+int zen_flash_ds_bytes(int, int, int, int, int64_t*);
 int zen_attn_fwd(const void*, void*, float*, int, int, int, int, int, int, int, float, float, void*);
 int zen_attn_bwd(const void*, const void*, const void*, const float*, float*, void*, int, int, int, int, int, int, int, int, float, float,
                  float*, int, void*);
@@ -215,7 +215,7 @@ BwdTemp bwd_temp_of(const ZenBlock& z, const Shape& s, void* base, bool keep_ds)
   t.stat = l.take<float>(2 * lse_floats(z, s));
   if (!wide_attention(z)) {
     int64_t need = 0;
-    if (keep_ds) zen_flash_ds_bytes(s.B, s.S, z.hq, z.hkv, z.hd, &need);
+    if (keep_ds) zen_flash_ds_bytes(s.B, s.S, z.hq, z.hd, &need);
     if (need) t.ds = l.take<char>((size_t)need);
   } else {
     const int hs = zen_attn_hsplit(s.B, s.S, z.hq, z.hkv, z.hd);

@@ -1897,10 +1897,9 @@ int zen_sparse_allreduce(const ZenSparseCtx* c, const void* x, const float* thr,
 }
 
 // All `n` ranks of a call that runs on one device, phase by phase: no kernel starts before everything it would wait for
-// has been written.  `io` = n input pointers, then n output pointers.  Partition and densify stream their data once and take
-// all ranks in one launch; reduce and gather of a rank both go over its slot sums at random, so they are launched for as
-// many ranks at a time as keep those sums in two thirds of the L2 (8 x 2^26 elements, 33.5 MB a rank: rank by rank reduce and
-// gather take 403 us, two at a time 381, four 398, all eight 420, which fetches every sum from memory in both).
+// has been written.  `io` = n input pointers, then n output pointers.  All ranks go in one launch a phase.  Only the sums of owners of
+// more than 2^25 slots, which are not cut into buckets, take more than the L2 holds (134 MB): K2 and K3 of such a rank go over
+// them at random, one rank after the other.
 int zen_sparse_allreduce_local(const ZenSparseCtx* c, int n, void* const* io, const float* thr, uint32_t epoch, uint32_t fmt,
                                int dtype, int method1, int deterministic, void* stream) {
   if (n < 1 || n > ZEN_MAX_RANKS) return -1;
@@ -1919,19 +1918,12 @@ int zen_sparse_allreduce_local(const ZenSparseCtx* c, int n, void* const* io, co
       if ((rc = launch_reduce_gather<T, ZEN_MAX_RANKS>(b, n, deterministic ? 1 : 0, st))) return rc;
       return launch_densify<T, ZEN_MAX_RANKS>(b, n, st);
     }
-    int group = (int)((80u << 20) / ((uint64_t)c->nslots * 4 + 1));
-    if (group < 1) group = 1;
-    if (group >= n) {
-      if ((rc = launch_reduce<T, ZEN_MAX_RANKS>(b, n, deterministic, st))) return rc;
-      if ((rc = launch_gather<T, ZEN_MAX_RANKS>(b, n, st))) return rc;
-    } else {
-      for (int i = 0; i < n; i += group) {
-        const int m = n - i < group ? n - i : group;
-        ZenSparseBatch<ZEN_MAX_RANKS> part;
-        for (int k = 0; k < m; ++k) { part.c[k] = b.c[i + k]; part.in[k] = b.in[i + k]; part.out[k] = b.out[i + k]; }
-        if ((rc = launch_reduce<T, ZEN_MAX_RANKS>(part, m, deterministic, st))) return rc;
-        if ((rc = launch_gather<T, ZEN_MAX_RANKS>(part, m, st))) return rc;
-      }
+    const int group = c->nslots < SB_MIN_SLOTS ? n : 1;      // (in between, in_buckets)
+    for (int i = 0; i < n; i += group) {
+      ZenSparseBatch<ZEN_MAX_RANKS> part = b;
+      if (group == 1) { part.c[0] = b.c[i]; part.in[0] = b.in[i]; part.out[0] = b.out[i]; }
+      if ((rc = launch_reduce<T, ZEN_MAX_RANKS>(part, group, deterministic, st))) return rc;
+      if ((rc = launch_gather<T, ZEN_MAX_RANKS>(part, group, st))) return rc;
     }
     rc = launch_densify<T, ZEN_MAX_RANKS>(b, n, st);
   });

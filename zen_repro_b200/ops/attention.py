@@ -68,10 +68,10 @@ def attention_fwd_kernel(qkv, bsz, seq, hq, hkv, hd, scale, softcap: float = 0.0
 
 
 @functools.lru_cache(maxsize=4096)
-def _flash_ds_bytes(bsz, seq, hq, hkv, hd) -> int:
+def _flash_ds_bytes(bsz, seq, hq, hd) -> int:
     """Bytes of scratch for which the backward keeps dS between its kernels, or 0."""
     out = ctypes.c_int64()
-    _native.lib().zen_flash_ds_bytes(bsz, seq, hq, hkv, hd, ctypes.addressof(out))
+    _native.lib().zen_flash_ds_bytes(bsz, seq, hq, hd, ctypes.addressof(out))
     return out.value
 
 
@@ -91,7 +91,7 @@ def attention_bwd_kernel(dout, qkv, out, lse2, bsz, seq, hq, hkv, hd, scale, sof
     dout = dout if (dout.is_contiguous() and dout.data_ptr() % 16 == 0) else dout.contiguous()
     dqkv = torch.empty_like(qkv)
     if hd <= 128 and softcap <= 0:
-        need, nstat = _flash_ds_bytes(bsz, seq, hq, hkv, hd), 8 * lse2.numel()
+        need, nstat = _flash_ds_bytes(bsz, seq, hq, hd), 8 * lse2.numel()
         temp, keep_ds = scratch(nstat + need, nstat, qkv.device)                                 # row statistics (a multiple of 1 KB), dS
         stat = temp.data_ptr()
         rc = _native.lib().zen_flash_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse2.data_ptr(), stat, dqkv.data_ptr(), bsz, seq, hq,

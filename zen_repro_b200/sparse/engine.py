@@ -251,8 +251,9 @@ def status_message(st: int) -> str:
 class SparseAllReduce:
     """Sparse all-reduce (SUM) of a flat bucket across a process group, one process per GPU.
 
-    ``__call__`` enqueues four to six kernels on the current stream and returns
-    the dense result without synchronising.  ``check()`` reads the status word;
+    ``__call__`` enqueues three or four kernels on the current stream (method 1: two
+    or three, or one per source above 2^19 elements) and returns the dense result
+    without synchronising.  ``check()`` reads the status word;
     on overflow every rank sees the same status (overflow bits travel in the
     mails), so the caller can fall back to a dense all-reduce collectively.
     """
