@@ -1807,7 +1807,8 @@ int zen_norm_fwd(const void* x, const void* res, const void* w, const void* b, v
   cudaStream_t st = (cudaStream_t)stream;
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(w) |
                          reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(hout);
-  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && rows > 0 && ptrs % 16 == 0) {
+  if (ptrs % 16) return -3;                             // every kernel below reads and writes 16 bytes at a time
+  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && rows > 0) {
     const int chunk = (rows + 2 * sm_count_e() - 1) / (2 * sm_count_e()), grid = (rows + chunk - 1) / chunk;
 #define NORM_STAGED(L_, RS_, NIT_)                                                                                                      \
   do {                                                                                                                                  \
@@ -1898,9 +1899,10 @@ int zen_norm_bwd_sums(const void* dy, const void* h, const void* w, const float*
   cudaStream_t st = (cudaStream_t)stream;
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(dres) |
                          reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(dh);
+  if (ptrs % 16) return -3;                             // as in the forward
   // One pass up to NF_COLS columns of a 16-bit type (wider rows leave the sums of a thread's columns no registers: 4096 x 5120 90 us as
-  // two kernels, 102 as one), where bulk copies and 16-byte accesses can reach.
-  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS && ptrs % 16 == 0) {
+  // two kernels, 102 as one).
+  if (dtype != ZEN_DTYPE_F32 && cols <= NF_COLS) {
     const int chunk = colsum_rpc(rows), parts = (rows + chunk - 1) / chunk;
     // rows to a stage: three stages in 108 KB, so that two CTAs fit an SM (8 x 1024 rows of 2048 columns take 56 us with one CTA to an SM,
     // 46 with two), and three vectors of a row to a lane
