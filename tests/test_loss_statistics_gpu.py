@@ -72,7 +72,7 @@ def test_a_loss_that_is_not_finite_stays_so():
 
 
 @pytest.mark.parametrize("softcap", [0.0, 30.0])
-@pytest.mark.parametrize("rows", [64, 300, 1000, 1100])
+@pytest.mark.parametrize("rows", [64, 300, 1000, 1023, 1024, 1100, 2047, 2048])
 def test_loss_function_equals_the_separate_passes(rows, softcap, monkeypatch):
     from zen_repro_b200.ops import gemm as G
     from zen_repro_b200.ops.autograd import lm_head_loss
@@ -87,15 +87,20 @@ def test_loss_function_equals_the_separate_passes(rows, softcap, monkeypatch):
     def run():
         loss = lm_head_loss(h, w, labels, chunk_tokens=1024, unit_grad=False, softcap=softcap)
         gh, gw = torch.autograd.grad(loss, (h, w))
+        training.append(len(ran))
         with torch.no_grad():
             quiet = lm_head_loss(h, w, labels, chunk_tokens=1024, softcap=softcap)
         return loss.detach(), quiet, gh, gw
 
-    ran = []
+    ran, training = [], []
     real = G.gemm_nt_loss
     monkeypatch.setattr(G, "gemm_nt_loss", lambda *a, **k: ran.append(1) or real(*a, **k))
     one = run()
-    assert bool(ran) == G.makes_loss_statistics(h.detach()[:1024], w.detach())
+    # in training the chunks of 1024 rows, and those alone; without a gradient every chunk whose product is of that kind
+    sizes = [min(1024, rows - s) for s in range(0, rows, 1024)]
+    kind = [G.makes_loss_statistics(h.detach()[:n], w.detach()) for n in sizes]
+    assert rows < 1024 or kind[0]
+    assert training == [sum(n == 1024 for n in sizes)] and len(ran) == training[0] + sum(kind)
     monkeypatch.setattr(G, "makes_loss_statistics", lambda a, b: False)
     two = run()
     assert abs(one[0] - two[0]) <= 1e-5 * two[0] and abs(one[1] - one[0]) <= 1e-6 * one[0]

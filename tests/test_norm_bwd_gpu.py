@@ -55,6 +55,7 @@ def test_forward_against_64_bits(rows, cols, layer):
     b = torch.randn(cols, device="cuda").bfloat16() if layer else None
     for r in (res, None):
         y, h, rstd, mean = E.norm_fwd(x, w, b, r, eps=1e-5, layer=layer)
+        assert E.norm_error() == 0
         want_h = (x.float() + r.float()).bfloat16() if r is not None else x
         assert torch.equal(h, want_h)
         hd = want_h.double()

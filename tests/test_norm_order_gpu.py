@@ -17,6 +17,7 @@ def test_statistics_equal_those_of_fp32(cols, layer, rows):
     w, b = torch.randn(cols, device="cuda").bfloat16(), torch.randn(cols, device="cuda").bfloat16() if layer else None
     y, _, *stats = E.norm_fwd(x, w, b, eps=1e-5, layer=layer)
     y32, _, *stats32 = E.norm_fwd(x.float(), w.float(), b.float() if layer else None, eps=1e-5, layer=layer)
+    assert E.norm_error() == 0
     for one, two in zip(stats, stats32):
         assert (one is None) == (two is None) and (one is None or torch.equal(one, two))
     assert torch.equal(y, y32.bfloat16())
