@@ -605,8 +605,9 @@ norm_bwd_fused_kernel(const T* dy, const T* h, const T* wgt, const float* rstd_i
         }
       }
     }
-    // The stage of the step before this one is filled again: what was read from it has been added to sums that this step's sums
-    // continue, so none of those loads is still on its way (this step's may be).
+    // The stage of the step before this one is filled again.  A barrier does not wait for loads that have only been issued, so the
+    // step's own stage would be too early.  The loads of the step before have all arrived: every warp has added what it read to its
+    // sums, in program order before it came to the barrier in the middle of this step.
     const int next = sb - 1 + NF_STAGES;
     if (sb >= 1 && next < nsb) {
       if (tid == 0) issue(next);
