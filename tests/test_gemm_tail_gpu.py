@@ -61,15 +61,17 @@ def test_a_workspace_for_the_tiles_at_hand_is_enough(k, missing):
             assert torch.equal(got.view(-1, 256, 256)[cut], _sum_of_halves(*pairs[0]).view(-1, 256, 256)[cut])
 
 
+@pytest.mark.parametrize("k", [1024, 2240, 2248, 4096])
 @pytest.mark.parametrize("shapes", [[(512, 512), (512, 256)], [(256, 256)], [(768, 768), (768, 1024), (1000, 776)]])
-def test_groups_of_less_than_a_round_are_cut(shapes):
+def test_groups_of_less_than_a_round_are_cut(shapes, k):
     """Weight gradients of a narrow layer: no split-K plan sees a group, so the launch itself shares the idle clusters out."""
     torch.manual_seed(len(shapes))
-    pairs = [_pair(4096, m, n) for m, n in shapes]
+    pairs = [_pair(k, m, n) for m, n in shapes]
     tiles = sum(-(-m // 256) * -(-n // 256) for m, n in shapes)
     assert 2 * tiles <= _clusters()
-    for got, (a, b) in zip(_group(pairs, tiles * HALVES, tiles * 16), pairs):
-        assert torch.equal(got, _sum_of_halves(a, b))
+    whole = _group(pairs, 0, 0)
+    for got, one, (a, b) in zip(_group(pairs, tiles * HALVES, tiles * 16), whole, pairs):
+        assert torch.equal(got, _sum_of_halves(a, b) if k > 35 * 64 else one)
 
 
 @pytest.mark.parametrize("n", [28672, 40960])

@@ -838,14 +838,17 @@ int g_tail_min_kb = 1;             // fewest 64-wide K blocks for which the tile
 // first cut, and for single products not in outputs of one round, which split_k_choice cuts where that pays (no plan sees the tiles of
 // a group): another order of summation in one tile of ten moves the logits of a four-layer Llama by up to 1.2 % (2 x 600 and 1 x 2048
 // tokens), as much as any rounding there, and scores should not change by that for 2 us.
-constexpr int TAIL_K_MIN_KB = 16;
+// Groups of less than a round have no last round to balance, so time alone decides: from K = 2304 on.  us, K halves / column halves: 12
+// tiles (a layer 256 wide) of K = 1024 11.8 / 9.5, 2048 14.3 / 13.9, 4096 19.2 / 22.6, 8192 29.2 / 39.9; 36 tiles 12.4 / 9.7, 14.9 / 14.4,
+// 20.1 / 23.5, 32.4 / 41.4.
+constexpr int TAIL_K_MIN_KB = 16, ONE_ROUND_K_MIN_KB = 36;
 // ws_floats, n_counters: what the caller's workspace holds; one_round: K also where all tiles fit one round.
 static void cut_tail(GemmGroup& g, int min_kb, uint64_t ws_floats = 0, int n_counters = 0, bool one_round = false) {
   const int clusters = zen_tmap::sm_count() / 2, rem = g.num_tiles % clusters;
   g.tail = g_tail_min_kb > 0 && min_kb >= g_tail_min_kb && 2 * rem <= clusters ? rem : 0;
   const bool room = g.ws && g.counters && reinterpret_cast<uintptr_t>(g.ws) % 16 == 0 && ws_floats >= (uint64_t)g.tail * 2 * 2 * BM2 * 256 &&
                     n_counters >= g.tail * 16;
-  g.tail_k = g.tail > 0 && (one_round || g.num_tiles > clusters) && min_kb >= TAIL_K_MIN_KB && room;
+  g.tail_k = g.tail > 0 && room && (g.num_tiles > clusters ? min_kb >= TAIL_K_MIN_KB : one_round && min_kb >= ONE_ROUND_K_MIN_KB);
   for (int i = 0; i < g.n && g.tail_k; ++i) {
     const int end = g.pr[i].tile_start + g.pr[i].num_m_pairs * g.pr[i].num_n_tiles;
     if (end > g.num_tiles - g.tail && !g.pr[i].tma_store) g.tail_k = 0;
