@@ -33,7 +33,7 @@ constexpr int MAX_SPLITS = 3;      // K slices per output tile at most
 // Epilogue warps: one per 32 rows, or two of them (one for each half of the columns) where the epilogue has arithmetic to do
 // (bias, activation): a warp alone on its scheduler waits out the latency of everything it does, and with a K of 768 the
 // epilogue of a tile then takes longer than the products of the next one.  Without arithmetic the second warp costs more than it
-// hides.  us, one / two warps, passes of 64 MB between the launches:
+// hides.  us, one / two warps, with a pass over 64 MB before each launch (so that operands come from memory):
 //   8192 x 3072 x 768   plain 37.8 / 39.9   with bias 46.0 / 41.9   with bias and activation 60.3 / 50.2
 //   8192 x 2304 x 768   plain 29.7 / 31.7   with bias 35.7 / 31.8   1024 x 768 x 3072 with bias 27.4 / 25.5
 // (with bias and activation 67.5 with the bias read as described at bias_pair).
@@ -187,7 +187,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 
 // Bias of a warp's boxes (64 columns each): lane l holds columns 2 l and 2 l + 1 of a box, fetched before the wait for the
 // products, and hands them round by shuffles.  (Every lane reading every column, 256 two-byte loads a tile, cost 3.3 us per
-// tile: 8192 x 2304 x 768 38 us with a bias against 25 without.)
+// tile: 8192 x 2304 x 768 launched back to back 38 us with a bias against 25 without; now 24.3 against 23.1.)
 __device__ __forceinline__ uint32_t bias_pair(const GemmProblem& p, int col, int lane) {
   const unsigned short* bp = reinterpret_cast<const unsigned short*>(p.bias);
   const int c = col + 2 * lane;
@@ -1011,9 +1011,9 @@ int zen_gemm_bf16_2cta_loss(const void* A, const void* B, void* C, int M, int N,
 }
 
 // Several products with the same operand layouts in ONE launch (see GemmProblem): the tiles of all of them form one
-// list that the persistent clusters walk, and the tiles of the last, partly filled wave are cut in two (cut_tail).  `descs`: n records of ZenGemmDesc; every product follows the contract of
-// zen_gemm_bf16_2cta (no bias).  ws / counters as for zen_gemm_bf16_2cta_splitk (may be null: K is
-// not cut).
+// list that the persistent clusters walk, and the tiles of the last, partly filled wave are cut in two (cut_tail).  `descs`: n
+// records of ZenGemmDesc; every product follows the contract of zen_gemm_bf16_2cta (no bias).  ws / counters as for
+// zen_gemm_bf16_2cta_splitk (may be null: K is not cut).
 struct ZenGemmDesc {
   const void* A;
   const void* B;
